@@ -175,6 +175,10 @@ void launch_to_fixed2(const double4_32a* pos, uint4* a, uint4* b, uint32_t N, co
 void make_list_cuts(const double* r_cut, uint32_t ntypes, double r_buff, const azp_box& box, ListCut* out,
                     double* rlist_max, double* rlist_min = nullptr);
 
+// host: relative margin on r_cut^2 that covers the error of an FP32 r^2 formed from
+// the fixed-point shadow, for the smallest positive of n cutoffs
+float screen_margin(const double* r_cut, uint32_t n, const azp_box& box);
+
 // The cells of one warp, 32 consecutive cells from (global warp index) * 32: a
 // lane sorts its own cell when it holds at most kSerialCell members, then the
 // warp sorts the larger ones together, one after another (warp_sort_cell).

@@ -108,7 +108,7 @@ AZP_D double rsq_exact(double x, double y, double z)
 AZP_D uint32_t to_fixed(double x, double Linv)
 {
     // x / L in [-1/2, 1/2); scale to [-2^31, 2^31)
-    const double s = x * Linv * 4294967296.0;
+    const double s = x * (Linv * 4294967296.0);  // the power of two is exact either way
     return (uint32_t)(int32_t)__double2ll_rn(s);
 }
 

@@ -801,6 +801,7 @@ struct azp_md {
     uint32_t* nbrs = nullptr;
     ListCut* cuts = nullptr;
     double rlist_max = 0.0, rlist_min = 0.0;
+    float screen = 0.0f;  // relative margin of the FP64 step's FP32 scan
     // bonds
     uint32_t bt_width = 0;
     uint32_t *bt_n_tag = nullptr, *bt_partner_tag = nullptr, *bt_type_tag = nullptr;
@@ -973,6 +974,9 @@ MDArgs base_args(azp_md* m)
     a.flow = m->flow;
     a.max_disp = m->max_disp;
     a.fcap = m->fcap;
+    a.xplor = m->shift_mode == AZP_MODE_XPLOR ? 1 : 0;
+    a.capped = m->fcap > 0.0 ? 1 : 0;
+    a.screen = m->screen;
     const double half = 0.5 * m->r_buff;
     a.disp_thresh2 = (float)(half * half * (1.0 - 1e-5));
     a.flags = m->flags;
@@ -1418,6 +1422,33 @@ int size_list(azp_md* m, cudaStream_t s)
     return AZP_ERR_NLIST_OVERFLOW;
 }
 
+// Threads per particle of the fused step, from N and the list row a particle of mean
+// density has inside the largest list radius.
+// FP64 steps: the lanes of a particle share its candidate queue, which evens out the
+// pairs a warp evaluates, so a row of 13 or more entries per thread is split; beyond
+// that a row is split (down to 3 entries a thread) while the launch has fewer threads
+// than the chip holds (2 blocks of 256 per SM at ~110 registers, 78k threads).
+// Measured per step (microseconds; threads per particle 1 / 2 / 4 / 8 / 16):
+//   LJ fluid (row 132)    N = 4,096: 343 / 185 / 110 / 75 / 73
+//                         N = 54,872: 617 / 556 / 412 / 405 / 443
+//   melt (row 12)         N = 10,000: 56 / 44 / 44 / 58 / 75
+//                         N = 131,300: 136 / 147 / 169 / 268 / 672
+//   DPD fluid (row 28)    N = 60,000: 258 / 222 / 225 / 226 / 260
+int threads_per_particle(const azp_md_config& c)
+{
+    if (c.pair_kind < 0 || !c.r_cut || c.N == 0) return 1;
+    double rmax = 0.0;
+    for (uint32_t t = 0; t < c.ntypes * c.ntypes; ++t)
+        if (c.r_cut[t] > 0.0) rmax = std::max(rmax, c.r_cut[t] + c.r_buff);
+    const double row = c.N / (c.box.L[0] * c.box.L[1] * c.box.L[2]) * 4.18879 * rmax * rmax * rmax;
+    int tpp = 1;
+    if (c.precision == AZP_FP64) {
+        while (tpp < 16 && 2 * tpp <= row / 13.0) tpp *= 2;
+        while (tpp < 32 && 2 * tpp <= row / 3.0 && (double)c.N * tpp < 60000.0) tpp *= 2;
+    }
+    return tpp;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1491,8 +1522,9 @@ azp_md* azp_md_create(const azp_md_config* c, int* status)
     }
     if (!c->use_lambda) m->gamma.assign(c->gamma, c->gamma + c->ntypes);
     else m->gamma.assign(c->ntypes, 0.0);
+    m->tpp = threads_per_particle(*c);
     const char* env_tpp = std::getenv("AZP_TPP");
-    m->tpp = env_tpp ? std::atoi(env_tpp) : 1;
+    if (env_tpp) m->tpp = std::atoi(env_tpp);
     if (!(m->tpp == 1 || m->tpp == 2 || m->tpp == 4 || m->tpp == 8 || m->tpp == 16 || m->tpp == 32)) m->tpp = 1;
     const char* env_graph = std::getenv("AZP_GRAPHS");
     m->use_graphs = !(env_graph && env_graph[0] == '0');
@@ -1620,6 +1652,7 @@ azp_md* azp_md_create(const azp_md_config* c, int* status)
         make_list_cuts(m->r_cut.data(), c->ntypes, m->r_buff, m->box, cuts.data(), &m->rlist_max, &m->rlist_min);
         for (int d = 0; d < 3; ++d)
             if (m->rlist_max > 0.0 && m->box.L[d] < 2.0 * m->rlist_max) return fail(AZP_ERR_BOX_TOO_SMALL, m);
+        m->screen = screen_margin(m->r_cut.data(), nt2, m->box);
         ALLOC(m->cuts, nt2);
         CTRY(cudaMemcpy(m->cuts, cuts.data(), sizeof(ListCut) * nt2, cudaMemcpyHostToDevice));
         m->max_nn = 32;

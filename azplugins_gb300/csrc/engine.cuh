@@ -50,6 +50,9 @@ struct MDArgs {
     FlowD flow;
     double max_disp;
     double fcap;                // > 0: per-pair force magnitude cap
+    int xplor;                  // mode xplor: some type pair may be smoothed
+    int capped;                 // fcap > 0
+    float screen;               // FP64 step: relative margin of the FP32 scan's r_cut^2
     float disp_thresh2;         // (r_buff / 2)^2, slightly reduced
     uint32_t* flags;            // [0] rebuild request, [1] error bits, [2] builds, [4] ticket
     unsigned long long* d_timestep_rw;

@@ -46,34 +46,19 @@ struct NoBond {
     }
 };
 
-// accumulator: compensated force / energy in FP32, plain in FP64
+// accumulator with compensated force / energy in FP32
 template<typename R> struct Acc;
-template<> struct Acc<double> {
+// FP64 accumulator of the fused step; OUT: energy and virial too
+template<bool OUT> struct Acc64 {
     double fx = 0, fy = 0, fz = 0, u = 0, w[6] = {0, 0, 0, 0, 0, 0};
-    AZP_D void add(double dx, double dy, double dz, double fdr, double e, bool vir)
-    {
-        fx += dx * fdr;
-        fy += dy * fdr;
-        fz += dz * fdr;
-        u += 0.5 * e;
-        if (vir) {
-            const double h = 0.5 * fdr;
-            w[0] += h * dx * dx;
-            w[1] += h * dx * dy;
-            w[2] += h * dx * dz;
-            w[3] += h * dy * dy;
-            w[4] += h * dy * dz;
-            w[5] += h * dz * dz;
-        }
-    }
     // force from fdr, virial from fvir (DPD: the conservative part only)
-    AZP_D void add_split(double dx, double dy, double dz, double fdr, double fvir, double e, bool vir)
+    AZP_D void add(double dx, double dy, double dz, double fdr, double fvir, double e)
     {
         fx += dx * fdr;
         fy += dy * fdr;
         fz += dz * fdr;
-        u += 0.5 * e;
-        if (vir) {
+        if constexpr (OUT) {
+            u += 0.5 * e;
             const double h = 0.5 * fvir;
             w[0] += h * dx * dx;
             w[1] += h * dx * dy;
@@ -83,21 +68,40 @@ template<> struct Acc<double> {
             w[5] += h * dz * dz;
         }
     }
-    AZP_D void reduce(int tpp, bool vir)
+    AZP_D void reduce(uint32_t tpp)
     {
-        for (int m = tpp >> 1; m > 0; m >>= 1) {
+        for (uint32_t m = tpp >> 1; m > 0; m >>= 1) {
             fx += __shfl_xor_sync(0xffffffffu, fx, m);
             fy += __shfl_xor_sync(0xffffffffu, fy, m);
             fz += __shfl_xor_sync(0xffffffffu, fz, m);
-            u += __shfl_xor_sync(0xffffffffu, u, m);
-            if (vir)
+            if constexpr (OUT) {
+                u += __shfl_xor_sync(0xffffffffu, u, m);
                 for (int c = 0; c < 6; ++c) w[c] += __shfl_xor_sync(0xffffffffu, w[c], m);
+            }
         }
     }
-    AZP_D double Fx() const { return fx; }
-    AZP_D double Fy() const { return fy; }
-    AZP_D double Fz() const { return fz; }
-    AZP_D double U() const { return u; }
+    static constexpr int WORDS = OUT ? 10 : 3;
+    // column p of a [WORDS][n] array of doubles
+    AZP_D void put(double* s, uint32_t p, uint32_t n) const
+    {
+        s[p] = fx;
+        s[n + p] = fy;
+        s[2 * n + p] = fz;
+        if constexpr (OUT) {
+            s[3 * n + p] = u;
+            for (int c = 0; c < 6; ++c) s[(4 + c) * n + p] = w[c];
+        }
+    }
+    AZP_D void get(const double* s, uint32_t p, uint32_t n)
+    {
+        fx = s[p];
+        fy = s[n + p];
+        fz = s[2 * n + p];
+        if constexpr (OUT) {
+            u = s[3 * n + p];
+            for (int c = 0; c < 6; ++c) w[c] = s[(4 + c) * n + p];
+        }
+    }
 };
 template<> struct Acc<float> {
     Comp fx{0.f, 0.f}, fy{0.f, 0.f}, fz{0.f, 0.f}, u{0.f, 0.f};
@@ -310,8 +314,8 @@ AZP_D void dpd_key(const MDArgs& a, unsigned long long ts, uint32_t& k0, uint32_
 
 AZP_D double dpd_weight_engine(double x, double h)
 {
-    if (h == 0.5) return sqrt(x);
-    if (h == 0.25) return sqrt(sqrt(x));
+    if (h == 0.5) return d_sqrt(x);
+    if (h == 0.25) return d_sqrt(d_sqrt(x));
     if (h == 1.0) return x;
     return pow(x, h);
 }
@@ -324,6 +328,24 @@ AZP_D float dpd_weight_engine_f(float x, float h)
     return powf(x, h);
 }
 
+// the last block to finish advances the timestep and arms the next rebuild
+AZP_D void finish_step(const MDArgs& a, bool want_rebuild)
+{
+    if (__any_sync(0xffffffffu, want_rebuild) && (threadIdx.x & 31) == 0) atomicOr(&a.flags[0], 1u);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const uint32_t t = atomicAdd(&a.flags[4], 1u);
+        if (t == gridDim.x - 1) {
+            __threadfence();
+            const uint32_t req = atomicAdd(&a.flags[0], 0u) && !atomicAdd(&a.flags[1], 0u);
+            if (a.set_cond) cudaGraphSetConditional(a.next_cond, req ? 1u : 0u);
+            a.flags[4] = 0u;
+            *a.d_timestep_rw = *a.d_timestep_rw + 1ull;
+        }
+    }
+}
+
 // one pair in FP64: dx = x_i - x_j, dv = v_i - v_j; rec as in DpdEngine.
 // Returns false outside r_cut (rsq >= rcutsq).
 AZP_D bool dpd_term_fp64(const double* rec, double rcutsq, double dx, double dy, double dz, double dvx, double dvy,
@@ -333,11 +355,11 @@ AZP_D bool dpd_term_fp64(const double* rec, double rcutsq, double dx, double dy,
     const double rs = rsq_exact(dx, dy, dz);
     if (!(rs < rcutsq)) return false;
     const double rcinv = rec[0], rc = rec[1], A = rec[2], gamma = rec[3];
-    const double rinv = 1.0 / sqrt(rs);
-    const double r = 1.0 / rinv;
+    double rinv;
+    const double r = d_sqrt(rs, rinv);
     const double dot = dx * dvx + dy * dvy + dz * dvz;
     fc = A * (rinv - rcinv);
-    const double wR = dpd_weight_engine(fmax(1.0 - r * rcinv, 0.0), rec[4]) * rinv;
+    const double wR = dpd_weight_engine(nonneg(1.0 - r * rcinv), rec[4]) * rinv;
     const Philox4 ph = philox4x32_10(0u, min(tgi, tgj), max(tgi, tgj), 0u, k0, k1);
     const double alpha = -1.0 + 2.0 * open01(ph.v[0], ph.v[1]);
     fdr = fc - gamma * wR * wR * dot + rec[5] * wR * alpha;
@@ -345,27 +367,61 @@ AZP_D bool dpd_term_fp64(const double* rec, double rcutsq, double dx, double dy,
     return true;
 }
 
+// a pair's force with the rare modifications: the smoothing of mode xplor (and the
+// energy shift it needs) and the cap of the overlap relaxation. Out of line, with an
+// evaluation of its own, so that the plain step computes no energy for it.
+template<class PE>
+static __device__ __noinline__ double adjusted_fp64(const MDArgs& a, const double* rec, double rsq, double& e)
+{
+    double fdr;
+    PE::eval(rec, rsq, fdr, e);
+    e -= rec[PE::SHIFT_SLOT];
+    xplor(rec + PAIR_REC, rsq, fdr, e);
+    if (a.capped && fdr * fdr * rsq > a.fcap * a.fcap) fdr = copysign(a.fcap / sqrt(rsq), fdr);
+    return fdr;
+}
+
 // FP64 step: FP64 positions, forces and integration, the oracle's rounding for
-// every decision.
-template<class PE, class BE, typename R, int INTEG>
+// every decision. Bound by the FP64 pipe (fp64.cuh), so FP64 instructions are kept
+// to the pairs inside r_cut and run on full warps. The tpp lanes of a particle scan
+// its list on the 16-byte fixed-point shadow in FP32, with a margin above the
+// scan's error (a.screen), and queue the candidates together in shared memory;
+// the queues of the warp are then drained together, the lanes of a particle taking
+// its candidates in turn. A drained pair takes its FP64 displacement (the minimum
+// image where the bits say that it changes anything), the oracle's exact r^2 and the
+// r_cut decision. The particles' sums then move to the block's first threads, so
+// that bonds and integration run on full warps too.
+// Measured (ncu, LJ fluid of N = 54,872, 131 listed and 90 in range a particle):
+// 950 us with one thread per particle evaluating as it walked, 347 us so, the FP64
+// pipe 80 % busy; melt of N = 131,300: 274 -> 118 us.
+constexpr uint32_t MD_QUEUE = 16;  // queued candidates per lane of a particle
+constexpr int MD_SCAN = 4;         // list entries a lane scans per pass
+
+template<class PE, class BE, int INTEG, bool OUT>
 __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
 {
-    static_assert(std::is_same<R, double>::value, "k_md_step is the FP64 step; FP32 forces use k_md_step_fx");
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool PAIR = !std::is_same<PE, NoPair>::value;
+    constexpr bool DPD = std::is_same<PE, DpdEngine>::value;
     const uint32_t nt2 = a.ntypes * a.ntypes;
-    double* s_rc2 = reinterpret_cast<double*>(smem_raw);
-    double* s_gamma = s_rc2 + nt2;
+    double* s_gamma = reinterpret_cast<double*>(smem_raw);
     double* s_noise = s_gamma + a.ntypes;
-    R* s_rec = reinterpret_cast<R*>(s_noise + a.ntypes);
-    R* s_bond = s_rec + nt2 * PAIR_TBL;
-    if (!std::is_same<PE, NoPair>::value)
-        for (uint32_t t = threadIdx.x; t < nt2 * PAIR_TBL; t += blockDim.x) {
-            s_rec[t] = (R)a.pair_table[t];
-            if (t % PAIR_TBL == PAIR_REC) s_rc2[t / PAIR_TBL] = a.pair_table[t];
+    double* s_rec = s_noise + a.ntypes;
+    double* s_bond = s_rec + nt2 * PAIR_TBL;
+    double* s_sum = s_bond + a.nbondtypes * BOND_REC;
+    const uint32_t tpp = (uint32_t)a.tpp;
+    const uint32_t P = MD_BLOCK >> a.tpp_shift;  // particles of the block
+    float* s_screen = reinterpret_cast<float*>(s_sum + (tpp > 1u ? Acc64<OUT>::WORDS * P : 0u));
+    if constexpr (PAIR) {
+        for (uint32_t t = threadIdx.x; t < nt2 * PAIR_TBL; t += blockDim.x) s_rec[t] = a.pair_table[t];
+        for (uint32_t t = threadIdx.x; t < nt2; t += blockDim.x) {
+            const double* rec = a.pair_table + (size_t)t * PAIR_TBL;
+            s_screen[t] = PE::enabled(rec) ? __double2float_ru(rec[PAIR_REC] * (1.0 + (double)a.screen)) : -1.0f;
         }
-    if (!std::is_same<BE, NoBond>::value)
-        for (uint32_t t = threadIdx.x; t < a.nbondtypes * AZP_BOND_PARAM_DOUBLES; t += blockDim.x)
-            s_bond[t] = (R)a.bond_params[t];
+    }
+    if constexpr (!std::is_same<BE, NoBond>::value)
+        for (uint32_t t = threadIdx.x; t < a.nbondtypes; t += blockDim.x)
+            BE::prepare(a.bond_params + (size_t)t * AZP_BOND_PARAM_DOUBLES, s_bond + (size_t)t * BOND_REC);
     if (INTEG != MD_FORCES_ONLY && !a.use_lambda)
         for (uint32_t t = threadIdx.x; t < a.ntypes; t += blockDim.x) {
             s_gamma[t] = a.gamma[t];
@@ -373,62 +429,112 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
         }
     __syncthreads();
 
-    const int tpp = a.tpp;
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t i = gid / tpp;
-    const uint32_t sub = gid % tpp;
-    const bool active = i < a.N;
-    const bool vir = a.out != 0;
-    Acc<R> acc;
-    if (active) {
-        // ---------------------------------------------------------------- pair
-        if constexpr (!std::is_same<PE, NoPair>::value) {
-            const uint32_t n = min(a.counts[i], a.max_nn);
-            {
-                const double4_32a pi = a.pos[i];
-                const uint32_t ti = type_of(pi.w);
-                uint32_t k0 = 0, k1 = 0, tgi = 0;
-                double4_32a vi{};
-                if constexpr (std::is_same<PE, DpdEngine>::value) {
-                    dpd_key(a, force_timestep<INTEG>(a), k0, k1);
-                    tgi = a.tag[i];
-                    vi = reinterpret_cast<const double4_32a*>(a.dvel)[i];
-                }
-                for (uint32_t k = sub; k < n; k += tpp) {
-                    const uint32_t j = a.nbrs[(size_t)k * a.N + i];
-                    const double4_32a pj = a.pos[j];
-                    const double dx = min_image1(pi.x - pj.x, a.L[0], a.Linv[0]);
-                    const double dy = min_image1(pi.y - pj.y, a.L[1], a.Linv[1]);
-                    const double dz = min_image1(pi.z - pj.z, a.L[2], a.Linv[2]);
-                    const double rsq = rsq_exact(dx, dy, dz);
-                    const uint32_t tp = ti * a.ntypes + type_of(pj.w);
-                    const R* rec = s_rec + (size_t)tp * PAIR_TBL;
-                    const R* cut = rec + PAIR_REC;
-                    if constexpr (std::is_same<PE, DpdEngine>::value) {
-                        const double4_32a vj = reinterpret_cast<const double4_32a*>(a.dvel)[j];
-                        double fdr, fc, e;
-                        if (dpd_term_fp64(rec, cut[0], dx, dy, dz, vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, k0, k1, tgi,
-                                          a.tag[j], fdr, fc, e))
-                            acc.add_split(dx, dy, dz, fdr, fc, e, vir);
-                        continue;
-                    }
-                    if (!(rsq < cut[0]) || !PE::enabled(rec)) continue;
-                    R fdr, e;
-                    PE::eval(rec, rsq, fdr, e);
-                    e -= rec[PE::SHIFT_SLOT];
-                    xplor(cut, rsq, fdr, e);
-                    if (a.fcap > 0.0 && (double)fdr * fdr * rsq > a.fcap * a.fcap)
-                        fdr = (R)copysign(a.fcap / sqrt((double)rsq), (double)fdr);
-                    acc.add(dx, dy, dz, fdr, e, vir);
-                }
+    const double half0 = 0.5 * a.L[0], half1 = 0.5 * a.L[1], half2 = 0.5 * a.L[2];
+    Acc64<OUT> acc;
+    uint32_t i = blockIdx.x * P + (threadIdx.x >> a.tpp_shift);
+    bool active = i < a.N;
+    double4_32a pi = make_double4_32a(0.0, 0.0, 0.0, 0.0);
+    if (active) pi = a.pos[i];
+    // ---------------------------------------------------------------- pair
+    if constexpr (PAIR) {
+        const uint32_t sub = threadIdx.x & (tpp - 1u);
+        const uint32_t gshift = (threadIdx.x & 31u) & ~(tpp - 1u);
+        const uint32_t gmask = tpp == 32u ? 0xffffffffu : (1u << tpp) - 1u;
+        const uint32_t below_me = (1u << sub) - 1u;
+        // a row of 16 entries per lane and one of padding, against bank conflicts
+        uint32_t* queue = reinterpret_cast<uint32_t*>(s_screen + nt2) + (threadIdx.x & ~(tpp - 1u)) * (MD_QUEUE + 1u);
+        const uint32_t full = tpp * (MD_QUEUE - MD_SCAN);
+        const uint32_t n = active ? min(__ldg(a.counts + i), a.max_nn) : 0u;
+        const uint32_t nmax = __reduce_max_sync(0xffffffffu, n);
+        const uint32_t row = type_of(pi.w) * a.ntypes;
+        uint4 fi = make_uint4(0u, 0u, 0u, 0u);
+        uint32_t k0 = 0, k1 = 0, tgi = 0;
+        double4_32a vi{};
+        if (active) {
+            fi = __ldg(a.fix + i);
+            if constexpr (DPD) {
+                dpd_key(a, force_timestep<INTEG>(a), k0, k1);
+                tgi = a.tag[i];
+                vi = reinterpret_cast<const double4_32a*>(a.dvel)[i];
             }
         }
+        const uint32_t* col = a.nbrs + i;
+        uint32_t nq = 0;
+        for (uint32_t kb = 0; kb < nmax; kb += MD_SCAN * tpp) {
+            uint32_t jj[MD_SCAN];
+            uint4 fj[MD_SCAN];
+#pragma unroll
+            for (int u = 0; u < MD_SCAN; ++u) {
+                const uint32_t k = kb + sub + u * tpp;
+                jj[u] = k < n ? __ldg(col + (size_t)k * a.N) : 0xffffffffu;
+            }
+#pragma unroll
+            for (int u = 0; u < MD_SCAN; ++u) fj[u] = __ldg(a.fix + (jj[u] != 0xffffffffu ? jj[u] : 0u));
+#pragma unroll
+            for (int u = 0; u < MD_SCAN; ++u) {
+                const float dx = (float)(int32_t)(fi.x - fj[u].x) * a.sfix[0];
+                const float dy = (float)(int32_t)(fi.y - fj[u].y) * a.sfix[1];
+                const float dz = (float)(int32_t)(fi.z - fj[u].z) * a.sfix[2];
+                const float rs = dx * dx + dy * dy + dz * dz;
+                const bool hit = jj[u] != 0xffffffffu && rs < s_screen[row + fj[u].w];
+                const uint32_t hits = (__ballot_sync(0xffffffffu, hit) >> gshift) & gmask;
+                if (hit) queue[nq + __popc(hits & below_me)] = jj[u];
+                nq += __popc(hits);
+            }
+            const bool last = kb + MD_SCAN * tpp >= nmax;
+            if (!last && !__any_sync(0xffffffffu, nq > full)) continue;
+            __syncwarp();
+            for (uint32_t m = sub; m < nq; m += tpp) {
+                const uint32_t j = queue[m];
+                const double4_32a pj = a.pos[j];
+                const double dx = min_image_if(pi.x - pj.x, half0, a.L[0], a.Linv[0]);
+                const double dy = min_image_if(pi.y - pj.y, half1, a.L[1], a.Linv[1]);
+                const double dz = min_image_if(pi.z - pj.z, half2, a.L[2], a.Linv[2]);
+                const double* rec = s_rec + (size_t)(row + type_of(pj.w)) * PAIR_TBL;
+                const double* cut = rec + PAIR_REC;
+                double fdr, e;
+                if constexpr (DPD) {
+                    const double4_32a vj = reinterpret_cast<const double4_32a*>(a.dvel)[j];
+                    double fc;
+                    if (dpd_term_fp64(rec, cut[0], dx, dy, dz, vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, k0, k1, tgi,
+                                      a.tag[j], fdr, fc, e))
+                        acc.add(dx, dy, dz, fdr, fc, e);
+                } else {
+                    const double rsq = rsq_exact(dx, dy, dz);
+                    if (!less_nonneg(rsq, cut[0])) continue;
+                    if (a.xplor | a.capped) {
+                        fdr = adjusted_fp64<PE>(a, rec, rsq, e);
+                    } else {
+                        PE::eval(rec, rsq, fdr, e);
+                        if (OUT) e -= rec[PE::SHIFT_SLOT];
+                    }
+                    acc.add(dx, dy, dz, fdr, fdr, e);
+                }
+            }
+            __syncwarp();
+            nq = 0;
+        }
+        if (tpp > 1u) {
+            acc.reduce(tpp);
+            if (sub == 0u) acc.put(s_sum, threadIdx.x >> a.tpp_shift, P);
+        }
+    }
+    if (tpp > 1u) {
+        // one thread per particle from here on: the block's first P
+        i = blockIdx.x * P + threadIdx.x;
+        active = threadIdx.x < P && i < a.N;
+        if constexpr (PAIR) {
+            __syncthreads();
+            if (active) acc.get(s_sum, threadIdx.x, P);
+        }
+        if (active) pi = a.pos[i];
+    }
+    if (active) {
         // ---------------------------------------------------------------- bonds
         if constexpr (!std::is_same<BE, NoBond>::value) {
-            const uint32_t nb = a.bt_n[i];
-            for (uint32_t k = sub; k < nb; k += tpp) {
-                const uint2 e2 = a.bt[(size_t)k * a.N + i];
-                const double4_32a pi = a.pos[i];
+            const uint32_t nb = __ldg(a.bt_n + i);
+            for (uint32_t k = 0; k < nb; ++k) {
+                const uint2 e2 = __ldg(a.bt + (size_t)k * a.N + i);
                 const double4_32a pj = a.pos[e2.x];
                 double dx, dy, dz;
                 if constexpr (bond_uses_image<BE>::value) {
@@ -439,169 +545,149 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
                     dy = __dadd_rn(pi.y - pj.y, __dmul_rn((double)(gi[1] - gj[1]), a.L[1]));
                     dz = __dadd_rn(pi.z - pj.z, __dmul_rn((double)(gi[2] - gj[2]), a.L[2]));
                 } else {
-                    dx = min_image1(pi.x - pj.x, a.L[0], a.Linv[0]);
-                    dy = min_image1(pi.y - pj.y, a.L[1], a.Linv[1]);
-                    dz = min_image1(pi.z - pj.z, a.L[2], a.Linv[2]);
+                    dx = min_image_if(pi.x - pj.x, half0, a.L[0], a.Linv[0]);
+                    dy = min_image_if(pi.y - pj.y, half1, a.L[1], a.Linv[1]);
+                    dz = min_image_if(pi.z - pj.z, half2, a.L[2], a.Linv[2]);
                 }
                 const double rsq = rsq_exact(dx, dy, dz);
                 double fdr, en;
-                if (!BE::eval(s_bond + e2.y * AZP_BOND_PARAM_DOUBLES, rsq, fdr, en)) {
+                if (!BE::eval_prepared(s_bond + (size_t)e2.y * BOND_REC, rsq, fdr, en)) {
                     atomicOr(&a.flags[1], AZP_EBIT_BOND);
                     continue;
                 }
-                acc.add(dx, dy, dz, fdr, en, vir);
+                acc.add(dx, dy, dz, fdr, fdr, en);
             }
         }
     }
-    if (tpp > 1) acc.reduce(tpp, vir);
 
     bool want_rebuild = false;
-    if (active && sub == 0) {
-        double Fx = acc.Fx(), Fy = acc.Fy(), Fz = acc.Fz();
+    if (active) {
+        double Fx = acc.fx, Fy = acc.fy, Fz = acc.fz;
         double Ub = 0.0;
         if (a.bar_geom >= 0) {
             // the barrier's force joins the net force (src/HarmonicBarrier.h:149-180)
             double fb[3] = {0.0, 0.0, 0.0};
-            barrier_fp64(a, a.pos[i], *a.d_timestep + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), fb, Ub);
+            barrier_fp64(a, pi, *a.d_timestep + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), fb, Ub);
             Fx += fb[0];
             Fy += fb[1];
             Fz += fb[2];
         }
         double fw[4] = {0.0, 0.0, 0.0, 0.0};
-        double4_32a pw;
         if (a.wall_kind >= 0) {
             // the wall potential's force joins the net force (HOOMD adds the
             // external wall compute into net_force)
-            pw = a.pos[i];
-            engine_walls(a.wall_kind, a.walls, a.wall_tab, pw.x, pw.y, pw.z, type_of(pw.w), fw);
+            engine_walls(a.wall_kind, a.walls, a.wall_tab, pi.x, pi.y, pi.z, type_of(pi.w), fw);
             Fx += fw[0];
             Fy += fw[1];
             Fz += fw[2];
             Ub += fw[3];
         }
-        if (a.out) {
-            a.out_force[i] = make_double4_32a(Fx, Fy, Fz, acc.U() + Ub);
-            double wv[6] = {(double)acc.w[0], (double)acc.w[1], (double)acc.w[2],
-                            (double)acc.w[3], (double)acc.w[4], (double)acc.w[5]};
+        if constexpr (OUT) {
+            a.out_force[i] = make_double4_32a(Fx, Fy, Fz, acc.u + Ub);
+            double wv[6] = {acc.w[0], acc.w[1], acc.w[2], acc.w[3], acc.w[4], acc.w[5]};
             if (a.wall_kind >= 0) {
-                wv[0] += fw[0] * pw.x;
-                wv[1] += fw[0] * pw.y;
-                wv[2] += fw[0] * pw.z;
-                wv[3] += fw[1] * pw.y;
-                wv[4] += fw[1] * pw.z;
-                wv[5] += fw[2] * pw.z;
+                wv[0] += fw[0] * pi.x;
+                wv[1] += fw[0] * pi.y;
+                wv[2] += fw[0] * pi.z;
+                wv[3] += fw[1] * pi.y;
+                wv[4] += fw[1] * pi.z;
+                wv[5] += fw[2] * pi.z;
             }
             for (int c = 0; c < 6; ++c) a.out_virial[(size_t)c * a.N + i] = wv[c];
         }
         if constexpr (INTEG != MD_FORCES_ONLY) {
             const unsigned long long ts = *a.d_timestep;
-            double4_32a p = a.pos[i];
+            double4_32a p = pi;
             const uint32_t ti = type_of(p.w);
             const uint32_t tg = a.tag[i];
             bool moved = false;
-            {
-                // FP64 path: the reference arithmetic throughout; the per-type noise
-                // amplitude sqrt(6 gamma kT / dt) comes from a host table built with
-                // the same double operations, so the draws stay bit-exact
-                const double gam = a.use_lambda ? a.lambda * a.diameter[i] : s_gamma[ti];
-                // the method's temperature at this timestep (a table when it varies)
-                double kTv = a.kT, nz = a.use_lambda ? 0.0 : s_noise[ti];
-                if (a.kT_hdr) {
-                    const size_t r = kT_row(a, ts);
-                    kTv = a.kT_tab[r];
-                    nz = a.noise_tab[r * a.ntypes + ti];
+            // The reference arithmetic; the per-type noise amplitude
+            // sqrt(6 gamma kT / dt) comes from a host table built with the same
+            // double operations, so the draws stay bit-exact
+            const double gam = a.use_lambda ? a.lambda * a.diameter[i] : s_gamma[ti];
+            // the method's temperature at this timestep (a table when it varies)
+            double kTv = a.kT, nz = a.use_lambda ? 0.0 : s_noise[ti];
+            if (a.kT_hdr) {
+                const size_t r = kT_row(a, ts);
+                kTv = a.kT_tab[r];
+                nz = a.noise_tab[r * a.ntypes + ti];
+            }
+            const double c = a.noiseless ? 0.0 : (a.use_lambda ? sqrt(6.0 * gam * kTv / a.dt) : nz);
+            const bool mover = in_group(a, ti);
+            double ux, uy, uz;
+            flow_at(a.flow, p.y, ux, uy, uz);
+            double r0 = 0.0, r1 = 0.0, r2 = 0.0;
+            if constexpr (INTEG == MD_INTEG_LANGEVIN) {
+                uniform3(AZP_RNG_LANGEVIN_FLOW, ts, a.seed, tg, -c, c - (-c), r0, r1, r2);
+                double4_32a v = a.vel[i];
+                const double minv = rcp(v.w);
+                const double ax = (Fx + (r0 - gam * (v.x - ux))) * minv;
+                const double ay = (Fy + (r1 - gam * (v.y - uy))) * minv;
+                const double az = (Fz + (r2 - gam * (v.z - uz))) * minv;
+                const double h = 0.5 * a.dt;
+                if (mover) {
+                    v.x += h * ax;
+                    v.y += h * ay;
+                    v.z += h * az;
                 }
-                const double c = a.noiseless ? 0.0 : (a.use_lambda ? sqrt(6.0 * gam * kTv / a.dt) : nz);
-                const bool mover = in_group(a, ti);
-                double ux, uy, uz;
-                flow_at(a.flow, p.y, ux, uy, uz);
-                double r0, r1, r2;
-                if constexpr (INTEG == MD_INTEG_LANGEVIN) {
-                    uniform3(AZP_RNG_LANGEVIN_FLOW, ts, a.seed, tg, -c, c - (-c), r0, r1, r2);
-                    double4_32a v = a.vel[i];
-                    const double minv = 1.0 / v.w;
-                    const double ax = (Fx + (r0 - gam * (v.x - ux))) * minv;
-                    const double ay = (Fy + (r1 - gam * (v.y - uy))) * minv;
-                    const double az = (Fz + (r2 - gam * (v.z - uz))) * minv;
-                    const double h = 0.5 * a.dt;
+                if (a.next) {
+                    // step one of the next timestep with the acceleration just computed
                     if (mover) {
+                        p.x += (v.x + h * ax) * a.dt;
+                        p.y += (v.y + h * ay) * a.dt;
+                        p.z += (v.z + h * az) * a.dt;
                         v.x += h * ax;
                         v.y += h * ay;
                         v.z += h * az;
                     }
-                    if (a.next) {
-                        // step one of the next timestep with the acceleration just computed
-                        if (mover) {
-                            p.x += (v.x + h * ax) * a.dt;
-                            p.y += (v.y + h * ay) * a.dt;
-                            p.z += (v.z + h * az) * a.dt;
-                            v.x += h * ax;
-                            v.y += h * ay;
-                            v.z += h * az;
-                        }
-                        moved = true;
-                    } else if (mover) {
-                        a.accel[3 * i] = ax;
-                        a.accel[3 * i + 1] = ay;
-                        a.accel[3 * i + 2] = az;
-                    }
-                    a.vel[i] = v;
-                } else {
-                    uniform3(AZP_RNG_BROWNIAN_FLOW, ts, a.seed, tg, -c, c - (-c), r0, r1, r2);
-                    double dx = (ux + (Fx + r0) / gam) * a.dt;
-                    double dy = (uy + (Fy + r1) / gam) * a.dt;
-                    double dz = (uz + (Fz + r2) / gam) * a.dt;
-                    if (a.max_disp > 0.0) {
-                        dx = fmin(fmax(dx, -a.max_disp), a.max_disp);
-                        dy = fmin(fmax(dy, -a.max_disp), a.max_disp);
-                        dz = fmin(fmax(dz, -a.max_disp), a.max_disp);
-                    }
-                    if (mover) {
-                        p.x += dx;
-                        p.y += dy;
-                        p.z += dz;
-                    }
                     moved = true;
+                } else if (mover) {
+                    a.accel[3 * i] = ax;
+                    a.accel[3 * i + 1] = ay;
+                    a.accel[3 * i + 2] = az;
                 }
-                if (moved) {
-                    int wx = 0, wy = 0, wz = 0;
-                    wrap1(p.x, wx, a.L[0], a.lo[0], a.hi[0]);
-                    wrap1(p.y, wy, a.L[1], a.lo[1], a.hi[1]);
-                    wrap1(p.z, wz, a.L[2], a.lo[2], a.hi[2]);
-                    if (wx | wy | wz) {
-                        a.image[3 * i] += wx;
-                        a.image[3 * i + 1] += wy;
-                        a.image[3 * i + 2] += wz;
-                    }
-                    a.pos_next[i] = p;
-                    uint4 f;
-                    f.x = to_fixed(p.x, a.Linv[0]);
-                    f.y = to_fixed(p.y, a.Linv[1]);
-                    f.z = to_fixed(p.z, a.Linv[2]);
-                    f.w = ti;
-                    a.fix_next[i] = f;
-                    want_rebuild = displaced(f, a.fix_build[i], a.sfix, a.disp_thresh2);
-                    if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicOr(&a.flags[1], AZP_EBIT_NONFINITE);
+                a.vel[i] = v;
+            } else {
+                uniform3(AZP_RNG_BROWNIAN_FLOW, ts, a.seed, tg, -c, c - (-c), r0, r1, r2);
+                double dx = (ux + (Fx + r0) / gam) * a.dt;
+                double dy = (uy + (Fy + r1) / gam) * a.dt;
+                double dz = (uz + (Fz + r2) / gam) * a.dt;
+                if (a.max_disp > 0.0) {
+                    dx = fmin(fmax(dx, -a.max_disp), a.max_disp);
+                    dy = fmin(fmax(dy, -a.max_disp), a.max_disp);
+                    dz = fmin(fmax(dz, -a.max_disp), a.max_disp);
                 }
+                if (mover) {
+                    p.x += dx;
+                    p.y += dy;
+                    p.z += dz;
+                }
+                moved = true;
+            }
+            if (moved) {
+                int wx = 0, wy = 0, wz = 0;
+                wrap_if(p.x, wx, a.L[0], a.lo[0], a.hi[0]);
+                wrap_if(p.y, wy, a.L[1], a.lo[1], a.hi[1]);
+                wrap_if(p.z, wz, a.L[2], a.lo[2], a.hi[2]);
+                if (wx | wy | wz) {
+                    a.image[3 * i] += wx;
+                    a.image[3 * i + 1] += wy;
+                    a.image[3 * i + 2] += wz;
+                }
+                a.pos_next[i] = p;
+                uint4 f;
+                f.x = to_fixed(p.x, a.Linv[0]);
+                f.y = to_fixed(p.y, a.Linv[1]);
+                f.z = to_fixed(p.z, a.Linv[2]);
+                f.w = ti;
+                a.fix_next[i] = f;
+                want_rebuild = displaced(f, a.fix_build[i], a.sfix, a.disp_thresh2);
+                if (!(finite_bits(p.x) && finite_bits(p.y) && finite_bits(p.z)))
+                    atomicOr(&a.flags[1], AZP_EBIT_NONFINITE);
             }
         }
     }
-    if constexpr (INTEG != MD_FORCES_ONLY) {
-        if (__any_sync(0xffffffffu, want_rebuild) && (threadIdx.x & 31) == 0) atomicOr(&a.flags[0], 1u);
-        // the last block to finish advances the timestep and arms the next rebuild
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            const uint32_t t = atomicAdd(&a.flags[4], 1u);
-            if (t == gridDim.x - 1) {
-                __threadfence();
-                const uint32_t req = atomicAdd(&a.flags[0], 0u) && !atomicAdd(&a.flags[1], 0u);
-                if (a.set_cond) cudaGraphSetConditional(a.next_cond, req ? 1u : 0u);
-                a.flags[4] = 0u;
-                *a.d_timestep_rw = *a.d_timestep_rw + 1ull;
-            }
-        }
-    }
+    if constexpr (INTEG != MD_FORCES_ONLY) finish_step(a, want_rebuild);
 }
 
 // ---------------------------------------------------------------- FP32-force step
@@ -917,23 +1003,6 @@ AZP_D void bond_term_fx_image(const MDArgs& a, const uint4& fi, const uint4& li,
     acc.add(dx, dy, dz, fdr, en, vir);
 }
 
-// the last block to finish advances the timestep and arms the next rebuild
-AZP_D void finish_step(const MDArgs& a, bool want_rebuild)
-{
-    if (__any_sync(0xffffffffu, want_rebuild) && (threadIdx.x & 31) == 0) atomicOr(&a.flags[0], 1u);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const uint32_t t = atomicAdd(&a.flags[4], 1u);
-        if (t == gridDim.x - 1) {
-            __threadfence();
-            const uint32_t req = atomicAdd(&a.flags[0], 0u) && !atomicAdd(&a.flags[1], 0u);
-            if (a.set_cond) cudaGraphSetConditional(a.next_cond, req ? 1u : 0u);
-            a.flags[4] = 0u;
-            *a.d_timestep_rw = *a.d_timestep_rw + 1ull;
-        }
-    }
-}
 
 // neighbours gathered per batch: the list indices of a batch are loaded first,
 // then their positions, so each thread keeps this many gathers in flight
@@ -1402,9 +1471,17 @@ int launch_md_t(const MDArgs& a, cudaStream_t s)
         k<<<blocks, FX_BLOCK, smem_k, s>>>(a);
         AZP_CHECK_LAUNCH("k_md_step_fx");
     } else {
-        const size_t smem = nt2 * sizeof(double) + 2 * a.ntypes * sizeof(double) + nt2 * PAIR_TBL * sizeof(R) +
-                            (size_t)a.nbondtypes * AZP_BOND_PARAM_DOUBLES * sizeof(R);
-        auto k = k_md_step<PE, BE, R, INTEG>;
+        const size_t smem = 2 * a.ntypes * sizeof(double) + nt2 * PAIR_TBL * sizeof(double) +
+                            (size_t)a.nbondtypes * BOND_REC * sizeof(double) + nt2 * sizeof(float) +
+                            (a.tpp > 1 ? (size_t)(MD_BLOCK / a.tpp) * (a.out ? 10 : 3) * sizeof(double) : 0) +
+                            (std::is_same<PE, NoPair>::value ? 0 : MD_BLOCK * (MD_QUEUE + 1) * sizeof(uint32_t));
+        // a Brownian step writes no forces, a forces-only launch nothing else
+        auto k = k_md_step<PE, BE, INTEG, INTEG == MD_FORCES_ONLY>;
+        if constexpr (INTEG == MD_INTEG_LANGEVIN) {
+            if (a.out) k = k_md_step<PE, BE, INTEG, true>;
+        } else if ((a.out != 0) != (INTEG == MD_FORCES_ONLY)) {
+            return record_error(AZP_ERR_UNSUPPORTED, "k_md_step: output mode not built");
+        }
         if (smem > 48 * 1024) AZP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k<<<blocks, MD_BLOCK, smem, s>>>(a);
         AZP_CHECK_LAUNCH("k_md_step");

@@ -13,6 +13,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fp64.cuh"
 #include <math.h>
 #include <type_traits>
 
@@ -21,17 +22,63 @@ namespace azp
 constexpr int PAIR_REC = 8;   // values per pair kernel record
 constexpr int CUT_REC = 4;    // rcutsq, ronsq, 1/(rcutsq-ronsq)^3, xplor flag
 
-// correctly rounded reciprocal; the FP32 form maps to the hardware-assisted
-// rounded reciprocal instead of a full division (an approximate reciprocal's
-// extra ulp, raised to the 12th power by the LJ core, costs too much of the
-// FP32 force budget at overlapped pairs)
-AZP_HD double rcp(double x) { return 1.0 / x; }
+// Reciprocal, root and quotient of the evaluators. FP32: correctly rounded; the
+// reciprocal maps to the hardware-assisted rounded reciprocal instead of a full
+// division (an approximate reciprocal's extra ulp, raised to the 12th power by
+// the LJ core, costs too much of the FP32 force budget at overlapped pairs). FP64
+// on the device: the refined forms of fp64.cuh, within an ulp.
+AZP_HD double rcp(double x)
+{
+#ifdef __CUDA_ARCH__
+    return d_rcp(x);
+#else
+    return 1.0 / x;
+#endif
+}
 AZP_HD float rcp(float x)
 {
 #ifdef __CUDA_ARCH__
     return __frcp_rn(x);
 #else
     return 1.0f / x;
+#endif
+}
+template<typename R> AZP_HD R root(R x) { return sqrt(x); }
+template<> AZP_HD double root<double>(double x)
+{
+#ifdef __CUDA_ARCH__
+    return d_sqrt(x);
+#else
+    return sqrt(x);
+#endif
+}
+// x, or 0 where rounding took a difference that cannot be negative below it
+template<typename R> AZP_HD R nonneg(R x) { return x; }
+template<> AZP_HD double nonneg<double>(double x)
+{
+#ifdef __CUDA_ARCH__
+    return x < 0.0 ? 0.0 : x;
+#else
+    return x;
+#endif
+}
+// a < b for a >= 0: on the bit patterns in FP64
+template<typename R> AZP_HD bool below(R a, R b) { return a < b; }
+template<> AZP_HD bool below<double>(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    return less_nonneg(a, b);
+#else
+    return a < b;
+#endif
+}
+template<typename R> AZP_HD R over(R a, R b) { return a / b; }
+template<> AZP_HD double over<double>(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+    return a * d_rcp(b);
+#else
+    return a / b;
 #endif
 }
 
@@ -63,7 +110,7 @@ struct PerturbedLJ {
         const R r6inv = r2inv * r2inv * r2inv;
         R f = r2inv * r6inv * (rec[5] * r6inv - rec[6]);
         R u = r6inv * (rec[0] * r6inv - rec[1]);
-        if (rsq < rec[3]) {
+        if (below(rsq, rec[3])) {
             u += rec[4];
         } else {
             f *= rec[2];
@@ -88,11 +135,11 @@ struct ExpandedYukawa {
     template<typename R> AZP_HD static bool enabled(const R* rec) { return rec[0] != R(0); }
     template<typename R> AZP_HD static void eval(const R* rec, R rsq, R& fdr, R& e)
     {
-        const R r = sqrt(rsq);
+        const R r = root(rsq);
         const R s = r - rec[2];
         const R sinv = rcp(s);
         const R u = rec[0] * exp(-rec[1] * s) * sinv;
-        fdr = u * (rec[1] + sinv) / r;
+        fdr = over(u * (rec[1] + sinv), r);
         e = u;
     }
 };
@@ -109,11 +156,11 @@ struct Hertz {
     template<typename R> AZP_HD static bool enabled(const R* rec) { return rec[0] != R(0); }
     template<typename R> AZP_HD static void eval(const R* rec, R rsq, R& fdr, R& e)
     {
-        const R r = sqrt(rsq);
+        const R r = root(rsq);
         const R rc = rec[1];
-        const R x = R(1) - r / rc;
-        const R ex32 = rec[0] * x * sqrt(x);
-        fdr = R(2.5) * ex32 / (r * rc);
+        const R x = nonneg(R(1) - over(r, rc));
+        const R ex32 = rec[0] * x * root(x);
+        fdr = over(R(2.5) * ex32, r * rc);
         e = ex32 * x;
     }
 };
@@ -152,11 +199,11 @@ struct Colloid {
         const R d3 = d * d * d;
         const R d6 = d3 * d3;
         const R r4 = rsq * rsq;
-        const R pre = s3 * A * a * a2 / d3;
+        const R pre = over(s3 * A * a * a2, d3);
         const R poly = R(2) * (a2 + rsq) * (a2 * (R(5) * a2 + R(22) * rsq) + R(5) * r4);
-        fdr = R(4.0 / 15.0) * pre * (poly * s6 / d6 - R(5)) / d;
+        fdr = over(R(4.0 / 15.0) * pre * (over(poly * s6, d6) - R(5)), d);
         const R poly_e = a2 * (a2 * (a2 / R(3) + R(3) * rsq) + R(4.2) * r4) + rsq * r4;
-        e = R(2.0 / 9.0) * pre * (R(1) - poly_e * s6 / d6);
+        e = R(2.0 / 9.0) * pre * (R(1) - over(poly_e * s6, d6));
     }
 
     // sphere -- sphere (Everaers & Ejtehadi, PRE 67, 041710), with r = sqrt(rsq)
@@ -174,16 +221,16 @@ struct Colloid {
         const R h1 = ((sm + R(5) * sum) * sm + R(30) * prod) * g1;
         const R h2 = ((dp + R(5) * dif) * dp - R(30) * prod) * g2;
         const R h3 = ((dm + R(5) * dif) * dm - R(30) * prod) * g3;
-        const R pre = A * s6 / r / R(37800);
+        const R pre = over(over(A * s6, r), R(37800));
         R u = pre * (h0 - h1 - h2 + h3);
-        g0 *= R(42) * prod / sp + R(6) * sum + sp;
-        g1 *= R(42) * prod / sm + R(6) * sum + sm;
-        g2 *= R(-42) * prod / dp + R(6) * dif + dp;
-        g3 *= R(-42) * prod / dm + R(6) * dif + dm;
-        const R dur = u / r + R(5) * pre * (g0 + g1 - g2 - g3);
+        g0 *= over(R(42) * prod, sp) + R(6) * sum + sp;
+        g1 *= over(R(42) * prod, sm) + R(6) * sum + sm;
+        g2 *= over(R(-42) * prod, dp) + R(6) * dif + dp;
+        g3 *= over(R(-42) * prod, dm) + R(6) * dif + dm;
+        const R dur = over(u, r) + R(5) * pre * (g0 + g1 - g2 - g3);
         const R dua = -A / R(3) * r * ((R(2) * prod * q7 + R(1)) * q7 + (R(2) * prod * q8 - R(1)) * q8);
-        fdr = (dur + dua) / r;
-        u += A / R(6) * (R(2) * prod * (q7 + q8) - log(q8 / q7));
+        fdr = over(dur + dua, r);
+        u += A / R(6) * (R(2) * prod * (q7 + q8) - log(over(q8, q7)));
         e = u;
     }
 
@@ -202,7 +249,7 @@ struct Colloid {
             const R a = rec[6];
             cs_form(rec, rsq, a * a - rsq, fdr, e);
         } else {
-            const R r = sqrt(rsq);
+            const R r = root(rsq);
             cc_form(rec, r, (rec[1] + rec[2]) - r, fdr, e);
         }
     }
@@ -313,6 +360,8 @@ template<typename R> AZP_HD void xplor(const R* cut, R rsq, R& fdr, R& e)
 // instead, with the per-type constants of eval precomputed (prepare_f), so its
 // eval_f holds no parameter division.
 constexpr int BOND_F = 12;
+// values of a prepared bond record (prepare / eval_prepared) in either arithmetic
+constexpr int BOND_REC = 16;
 
 struct QuarticBond {
     static constexpr int REC_DOUBLES = 8;  // param_type: k, r_0, b_1, b_2, U_0, sigma_6, epsilon_x_4, delta
@@ -349,6 +398,59 @@ struct QuarticBond {
             e += k * (rr - b1) * (rr - b2) * rr * rr + U0;
         } else {
             e += U0;
+        }
+        return true;
+    }
+    // Per-type constants of eval in its own arithmetic, formed by the same
+    // operations, so that a bond costs no parameter arithmetic: k, r_0, b_1, b_2,
+    // U_0, delta, 12 lj1, 6 lj2, lj1, lj2, WCA r^-6 threshold (a value no r^-6
+    // exceeds without a core), WCA energy shift, 3 (b_1 + b_2), 2 b_1 b_2, r_0^2
+    template<typename R> AZP_HD static void prepare(const R* p, R* q)
+    {
+        const R lj1 = p[6] * p[5] * p[5], lj2 = p[6] * p[5];
+        for (int k = 0; k < 5; ++k) q[k] = p[k];
+        q[5] = p[7];
+        q[6] = R(12) * lj1;
+        q[7] = R(6) * lj2;
+        q[8] = lj1;
+        q[9] = lj2;
+        q[10] = lj1 != R(0) ? (lj2 / lj1) / R(2) : R(INFINITY);
+        q[11] = p[7] == R(0) ? (lj1 != R(0) ? lj2 * lj2 / R(4) / lj1 : R(0)) : p[6] / R(4);
+        q[12] = R(3) * (p[2] + p[3]);
+        q[13] = R(2) * p[2] * p[3];
+        q[14] = p[1] * p[1];
+        q[15] = R(0);
+    }
+    template<typename R> AZP_HD static bool eval_prepared(const R* q, R rsq, R& fdr, R& e)
+    {
+        const R r0 = q[1], del = q[5];
+        fdr = R(0);
+        e = R(0);
+        if (r0 == R(0)) return false;
+        R rr = R(1);
+        if (del == R(0)) {
+            const R r2inv = rcp(rsq);
+            const R r6inv = r2inv * r2inv * r2inv;
+            if (r6inv > q[10]) {
+                fdr += r2inv * r6inv * (q[6] * r6inv - q[7]);
+                e += r6inv * (q[8] * r6inv - q[9]) + q[11];
+            }
+            if (below(rsq, q[14])) rr = root(rsq) - r0;
+        } else {
+            const R rs = root(rsq) - del;
+            const R r2inv = over(over(R(1), rs), rs);
+            const R r6inv = r2inv * r2inv * r2inv;
+            if (r6inv > q[10]) {
+                fdr += over(over(r6inv * (q[6] * r6inv - q[7]), rs), rs + del);
+                e += r6inv * (q[8] * r6inv - q[9]) + q[11];
+            }
+            if (rs < r0) rr = rs - r0;
+        }
+        if (rr < R(0)) {
+            fdr += over(-q[0] * rr * (R(4) * rr * rr - q[12] * rr + q[13]), rr + r0 + del);
+            e += q[0] * (rr - q[2]) * (rr - q[3]) * rr * rr + q[4];
+        } else {
+            e += q[4];
         }
         return true;
     }
@@ -409,12 +511,20 @@ struct DoubleWellBond {
         fdr = R(0);
         e = R(0);
         if (rd == R(0)) return false;
-        const R r = sqrt(rsq);
-        const R x = (r1 - r) / rd;
+        const R r = root(rsq);
+        const R x = over(r1 - r, rd);
         const R y = R(1) - x * x;
         e = U1 * y * y + Ut * (R(1) - x - y * y);
-        fdr = (R(4) * x * y * (Ut - U1) - Ut) / (rd * r);
+        fdr = over(R(4) * x * y * (Ut - U1) - Ut, rd * r);
         return true;
+    }
+    template<typename R> AZP_HD static void prepare(const R* p, R* q)
+    {
+        for (int k = 0; k < BOND_REC; ++k) q[k] = k < AZP_BOND_PARAM_DOUBLES ? p[k] : R(0);
+    }
+    template<typename R> AZP_HD static bool eval_prepared(const R* q, R rsq, R& fdr, R& e)
+    {
+        return eval(q, rsq, fdr, e);
     }
     AZP_HD static void prepare_f(const double* p, float* q)
     {
@@ -447,10 +557,18 @@ struct HarmonicBond {
     template<typename R> AZP_HD static bool eval(const R* p, R rsq, R& fdr, R& e)
     {
         const R k = p[0], r0 = p[1];
-        const R r = sqrt(rsq);
-        fdr = r > R(0) ? k * (r0 / r - R(1)) : R(0);
+        const R r = root(rsq);
+        fdr = r > R(0) ? k * (over(r0, r) - R(1)) : R(0);
         e = R(0.5) * k * (r0 - r) * (r0 - r);
         return true;
+    }
+    template<typename R> AZP_HD static void prepare(const R* p, R* q)
+    {
+        for (int k = 0; k < BOND_REC; ++k) q[k] = k < AZP_BOND_PARAM_DOUBLES ? p[k] : R(0);
+    }
+    template<typename R> AZP_HD static bool eval_prepared(const R* q, R rsq, R& fdr, R& e)
+    {
+        return eval(q, rsq, fdr, e);
     }
     // FP32 record of the fused step: q = k, r_0
     AZP_HD static void prepare_f(const double* p, float* q)

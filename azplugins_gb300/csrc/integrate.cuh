@@ -9,6 +9,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fp64.cuh"
 #include "philox.cuh"
 
 namespace azp
@@ -19,16 +20,19 @@ constexpr uint32_t MAX_GAMMA_TYPES = 64;
 struct FlowD {
     int kind;
     double a, b, c;  // CONSTANT: U; PARABOLIC: a = Umax = 1.5 mean_velocity, b = L = separation / 2
+    double binv;     // 1 / b
 };
 
 inline FlowD make_flow(const azp_flow& f)
 {
     FlowD r;
     r.kind = f.kind;
+    r.binv = 0.0;
     if (f.kind == AZP_FLOW_PARABOLIC) {
         r.a = 1.5 * f.p[0];
         r.b = 0.5 * f.p[1];
         r.c = 0.0;
+        r.binv = 1.0 / r.b;
     } else {
         r.a = f.p[0];
         r.b = f.p[1];
@@ -40,7 +44,9 @@ inline FlowD make_flow(const azp_flow& f)
 AZP_D void flow_at(const FlowD& f, double y, double& ux, double& uy, double& uz)
 {
     if (f.kind == AZP_FLOW_PARABOLIC) {
-        const double yr = y / f.b;
+        // y / b: the product with 1 / b corrected by its residual
+        double yr = y * f.binv;
+        yr = fma(fma(-yr, f.b, y), f.binv, yr);
         ux = f.a * (1.0 - yr * yr);
         uy = 0.0;
         uz = 0.0;
@@ -55,7 +61,7 @@ AZP_D void flow_at(const FlowD& f, double y, double& ux, double& uy, double& uz)
 AZP_D void flow_at_f(const FlowD& f, float y, float& ux, float& uy, float& uz)
 {
     if (f.kind == AZP_FLOW_PARABOLIC) {
-        const float yr = y * (float)(1.0 / f.b);
+        const float yr = y * (float)f.binv;
         ux = (float)f.a * (1.0f - yr * yr);
         uy = 0.0f;
         uz = 0.0f;
@@ -75,6 +81,12 @@ AZP_D void wrap1(double& x, int& img, double L, double lo, double hi)
         x += L;
         img -= 1;
     }
+}
+
+// wrap1 that runs only where it can change x: |x| >= hi (the box is centred, lo = -hi)
+AZP_D void wrap_if(double& x, int& img, double L, double lo, double hi)
+{
+    if (!less_nonneg(fabs(x), hi)) wrap1(x, img, L, lo, hi);
 }
 
 struct StepArgs {

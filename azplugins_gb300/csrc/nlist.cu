@@ -66,6 +66,17 @@ int grid_subdivision(double rlist_max, double rlist_min)
     return std::max(1, std::min(3, (int)(rlist_max / rlist_min)));
 }
 
+float screen_margin(const double* r_cut, uint32_t n, const azp_box& box)
+{
+    double rmin = 0.0;
+    for (uint32_t t = 0; t < n; ++t)
+        if (r_cut[t] > 0.0 && (rmin == 0.0 || r_cut[t] < rmin)) rmin = r_cut[t];
+    // as in make_list_cuts: float rounding of the components and their squares,
+    // and the fixed-point rounding of both positions
+    const double Lmax = std::max(box.L[0], std::max(box.L[1], box.L[2]));
+    return (float)(rmin > 0.0 ? std::max(4e-6, 16.0 * Lmax * 2.3283064365386963e-10 / rmin) : 4e-6);
+}
+
 void make_list_cuts(const double* r_cut, uint32_t ntypes, double r_buff, const azp_box& box, ListCut* out,
                     double* rlist_max, double* rlist_min)
 {

@@ -63,12 +63,15 @@ AZP_HD void stream_key(uint32_t id, uint64_t timestep, uint32_t seed, uint32_t& 
     k1 = (uint32_t)(timestep & 0xffffffffu);
 }
 
-AZP_HD double open01(uint32_t hi, uint32_t lo)
+// the draw in units of 2^-53: (w >> 11) + 0.5
+AZP_HD double steps53(uint32_t hi, uint32_t lo)
 {
     const uint64_t w = ((uint64_t)hi << 32) | lo;
-    // (w >> 11) + 0.5 and the power-of-two scale are exact
-    return ((double)(w >> 11) + 0.5) * (1.0 / 9007199254740992.0);
+    return (double)(w >> 11) + 0.5;
 }
+
+// scaled by the (exact) power of two
+AZP_HD double open01(uint32_t hi, uint32_t lo) { return steps53(hi, lo) * (1.0 / 9007199254740992.0); }
 
 // three uniform doubles in (lo, lo + width): two Philox calls
 AZP_HD void uniform3(uint32_t id, uint64_t timestep, uint32_t seed, uint32_t tag, double lo, double width,
@@ -79,10 +82,12 @@ AZP_HD void uniform3(uint32_t id, uint64_t timestep, uint32_t seed, uint32_t tag
     const Philox4 a = philox4x32_10(0u, tag, 0u, 0u, k0, k1);
     const Philox4 b = philox4x32_10(1u, tag, 0u, 0u, k0, k1);
 #ifdef __CUDA_ARCH__
-    // two roundings, no FMA: the same doubles as the oracle
-    r0 = __dadd_rn(lo, __dmul_rn(width, open01(a.v[0], a.v[1])));
-    r1 = __dadd_rn(lo, __dmul_rn(width, open01(a.v[2], a.v[3])));
-    r2 = __dadd_rn(lo, __dmul_rn(width, open01(b.v[0], b.v[1])));
+    // two roundings, no FMA: the same doubles as the oracle (the power of two of
+    // open01 moved into the width, where it is as exact)
+    const double ws = width * (1.0 / 9007199254740992.0);
+    r0 = __dadd_rn(lo, __dmul_rn(ws, steps53(a.v[0], a.v[1])));
+    r1 = __dadd_rn(lo, __dmul_rn(ws, steps53(a.v[2], a.v[3])));
+    r2 = __dadd_rn(lo, __dmul_rn(ws, steps53(b.v[0], b.v[1])));
 #else
     r0 = lo + width * open01(a.v[0], a.v[1]);
     r1 = lo + width * open01(a.v[2], a.v[3]);
