@@ -285,17 +285,18 @@ __global__ void k_walls_fx(MDArgs a)
 
 // What a step reads of its neighbours while their owners update it in the same
 // step, copied right before the step: DPD the velocities (FP64: (v, mass);
-// FP32-force: the leading floats (v, 1/m)), ImageHarmonic bonds the image counts.
+// FP32-force: the leading floats and the tag), ImageHarmonic bonds the image counts.
 // Either output may be null.
-__global__ void k_step_snapshot(const double4_32a* __restrict__ vel, const int* __restrict__ image, uint32_t N,
-                                int fx, void* __restrict__ vel_out, int* __restrict__ img_out)
+__global__ void k_step_snapshot(const double4_32a* __restrict__ vel, const int* __restrict__ image,
+                                const uint32_t* __restrict__ tag, uint32_t N, int fx, void* __restrict__ vel_out, int* __restrict__ img_out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     if (vel_out) {
-        if (fx)
-            reinterpret_cast<float4*>(vel_out)[i] = reinterpret_cast<const VelFF*>(vel)[i].h;
-        else
+        if (fx) {
+            const float4 v = reinterpret_cast<const VelFF*>(vel)[i].h;
+            reinterpret_cast<float4*>(vel_out)[i] = make_float4(v.x, v.y, v.z, __uint_as_float(tag[i]));
+        } else
             reinterpret_cast<double4_32a*>(vel_out)[i] = vel[i];
     }
     if (img_out)
@@ -1132,7 +1133,7 @@ int md_launch(azp_md* m, int integ, const MDArgs& a, cudaStream_t s)
         m->launches += 1;
     }
     if (m->d_dvel || m->d_img0) {
-        k_step_snapshot<<<blocks_for(m->N, 256), 256, 0, s>>>(m->vel, m->image, m->N, m->precision == AZP_FP32 ? 1 : 0,
+        k_step_snapshot<<<blocks_for(m->N, 256), 256, 0, s>>>(m->vel, m->image, m->tag, m->N, m->precision == AZP_FP32 ? 1 : 0,
                                                               m->d_dvel, m->d_img0);
         AZP_CHECK_LAUNCH("k_step_snapshot");
         m->launches += 1;
@@ -1434,17 +1435,32 @@ int size_list(azp_md* m, cudaStream_t s)
 //   melt (row 12)         N = 10,000: 56 / 44 / 44 / 58 / 75
 //                         N = 131,300: 136 / 147 / 169 / 268 / 672
 //   DPD fluid (row 28)    N = 60,000: 258 / 222 / 225 / 226 / 260
+// FP32-force steps: latency bound, so a row is split (down to 3 entries a thread)
+// only while the launch has fewer threads than half of what the chip holds. Cutoffs
+// far apart make rows uneven (a colloid lists many times what a solvent bead does,
+// and its warp waits for it): those are split from 28 entries a thread on.
+//   LJ fluid              N = 4,096: 85 / 64 / 51 / 47 / 47
+//                         N = 54,872: 108 / 90 / 92 / 102 / 121
+//                         N = 110,592: 127 / 130 / 132 / 151 / 196
+//   melt                  N = 40,000: 35 / 34 / 36 / 43 / 55
+//   colloid mixture       N = 65,537: 441 / 311 / 240 / 220 / 207
 int threads_per_particle(const azp_md_config& c)
 {
     if (c.pair_kind < 0 || !c.r_cut || c.N == 0) return 1;
-    double rmax = 0.0;
+    double rmax = 0.0, rmin = 1e300;
     for (uint32_t t = 0; t < c.ntypes * c.ntypes; ++t)
-        if (c.r_cut[t] > 0.0) rmax = std::max(rmax, c.r_cut[t] + c.r_buff);
+        if (c.r_cut[t] > 0.0) {
+            rmax = std::max(rmax, c.r_cut[t] + c.r_buff);
+            rmin = std::min(rmin, c.r_cut[t] + c.r_buff);
+        }
     const double row = c.N / (c.box.L[0] * c.box.L[1] * c.box.L[2]) * 4.18879 * rmax * rmax * rmax;
     int tpp = 1;
     if (c.precision == AZP_FP64) {
         while (tpp < 16 && 2 * tpp <= row / 13.0) tpp *= 2;
         while (tpp < 32 && 2 * tpp <= row / 3.0 && (double)c.N * tpp < 60000.0) tpp *= 2;
+    } else {
+        while (rmax > 1.5 * rmin && tpp < 16 && 2 * tpp <= row / 28.0) tpp *= 2;
+        while (tpp < 16 && 2 * tpp <= row / 3.0 && (double)c.N * tpp < 80000.0) tpp *= 2;
     }
     return tpp;
 }

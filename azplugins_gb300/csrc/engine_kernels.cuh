@@ -883,10 +883,38 @@ AZP_D void pair_term_fx_masked(const MDArgs& a, const uint4& fi, const uint4& fj
     acc.add(dx, dy, dz, in ? fdr : 0.0f, in ? e : 0.0f, vir);
 }
 
+// A DPD pair near r_cut in a box that is not cubic, in FP64 from the 64-bit
+// positions. Out of line: its registers do not count against the pair loop.
+static __device__ __noinline__ bool dpd_near_cutoff_fp64(const MDArgs& a, const uint4& fi, const uint4& fj, uint32_t i,
+                                                         uint32_t j, uint32_t tp, double rc2, const float4& vi,
+                                                         const float4& vj, uint32_t tgi, uint32_t tgj, uint32_t k0,
+                                                         uint32_t k1, float& dx, float& dy, float& dz, float& fdr,
+                                                         float& fc, float& e)
+{
+    const uint4 li = a.flo[i], lj = a.flo[j];
+    const double ddx = min_image1(fx_to_double(fx_join(fi.x, li.x), a.l64[0]) - fx_to_double(fx_join(fj.x, lj.x), a.l64[0]),
+                                  a.L[0], a.Linv[0]);
+    const double ddy = min_image1(fx_to_double(fx_join(fi.y, li.y), a.l64[1]) - fx_to_double(fx_join(fj.y, lj.y), a.l64[1]),
+                                  a.L[1], a.Linv[1]);
+    const double ddz = min_image1(fx_to_double(fx_join(fi.z, li.z), a.l64[2]) - fx_to_double(fx_join(fj.z, lj.z), a.l64[2]),
+                                  a.L[2], a.Linv[2]);
+    double f, c, u;
+    if (!dpd_term_fp64(a.pair_table + (size_t)tp * PAIR_TBL, rc2, ddx, ddy, ddz, (double)(vi.x - vj.x),
+                       (double)(vi.y - vj.y), (double)(vi.z - vj.z), k0, k1, tgi, tgj, f, c, u))
+        return false;
+    dx = (float)ddx;
+    dy = (float)ddy;
+    dz = (float)ddz;
+    fdr = (float)f;
+    fc = (float)c;
+    e = (float)u;
+    return true;
+}
+
 // DPD pair in the FP32-force step: FP32 on the exact fixed-point displacement,
 // FP64 from the full 64-bit positions within 0.2 % of r_cut^2 (the weight
 // (1 - r / r_cut)^(s/2) is steep there, and the cutoff decision is the oracle's);
-// velocities from the step's snapshot (float4: v, 1/m)
+// velocities and tag from the step's snapshot (float4: v, tag bits)
 template<bool ONE = false>
 AZP_D void pair_term_dpd_fx(const MDArgs& a, const uint4& fi, const uint4& fj, uint32_t i, uint32_t j,
                             const float* s_rec, const double* s_rc2, AccFx& acc, bool vir, const float4& vi,
@@ -900,8 +928,8 @@ AZP_D void pair_term_dpd_fx(const MDArgs& a, const uint4& fi, const uint4& fj, u
     const float* rec = s_rec + (size_t)tp * PAIR_TBL;
     const float rc2 = rec[PAIR_REC];
     if (!(rc2 > 0.0f) || rs >= rc2 * 1.000004f) return;
-    const float4 vj = reinterpret_cast<const float4*>(a.dvel)[j];
-    const uint32_t tgj = a.tag[j];
+    const float4 vj = __ldg(reinterpret_cast<const float4*>(a.dvel) + j);
+    const uint32_t tgj = __float_as_uint(vj.w);
     if (rs >= rc2 * 0.998f && a.contact_q) {
         // within 0.2 % of r_cut^2 in a cubic box: the cutoff decided and 1 - r / r_cut
         // formed from the exact integer difference r_cut^2 - r^2, the rest in FP32
@@ -924,17 +952,9 @@ AZP_D void pair_term_dpd_fx(const MDArgs& a, const uint4& fi, const uint4& fj, u
         return;
     }
     if (rs >= rc2 * 0.998f) {
-        const uint4 li = a.flo[i], lj = a.flo[j];
-        const double ddx = min_image1(fx_to_double(fx_join(fi.x, li.x), a.l64[0]) - fx_to_double(fx_join(fj.x, lj.x), a.l64[0]),
-                                      a.L[0], a.Linv[0]);
-        const double ddy = min_image1(fx_to_double(fx_join(fi.y, li.y), a.l64[1]) - fx_to_double(fx_join(fj.y, lj.y), a.l64[1]),
-                                      a.L[1], a.Linv[1]);
-        const double ddz = min_image1(fx_to_double(fx_join(fi.z, li.z), a.l64[2]) - fx_to_double(fx_join(fj.z, lj.z), a.l64[2]),
-                                      a.L[2], a.Linv[2]);
-        double fdr, fc, e;
-        if (dpd_term_fp64(a.pair_table + (size_t)tp * PAIR_TBL, s_rc2[tp], ddx, ddy, ddz, (double)(vi.x - vj.x),
-                          (double)(vi.y - vj.y), (double)(vi.z - vj.z), k0, k1, tgi, tgj, fdr, fc, e))
-            acc.add_split((float)ddx, (float)ddy, (float)ddz, (float)fdr, (float)fc, (float)e, vir);
+        float ddx, ddy, ddz, fdr, fc, e;
+        if (dpd_near_cutoff_fp64(a, fi, fj, i, j, tp, s_rc2[tp], vi, vj, tgi, tgj, k0, k1, ddx, ddy, ddz, fdr, fc, e))
+            acc.add_split(ddx, ddy, ddz, fdr, fc, e, vir);
         return;
     }
     const float rcinv = rec[0], A = rec[2];
@@ -1003,6 +1023,12 @@ AZP_D void bond_term_fx_image(const MDArgs& a, const uint4& fi, const uint4& li,
     acc.add(dx, dy, dz, fdr, en, vir);
 }
 
+
+// DPD: queued partners per lane, and the margin of the scan's r_cut^2: above the
+// 4e-6 at which pair_term_dpd_fx itself stops, by the difference of the two FP32
+// forms of r^2 (each within 1e-6)
+constexpr uint32_t DPD_QUEUE_FX = 16;
+constexpr float DPD_SCREEN = 1.00001f;
 
 // neighbours gathered per batch: the list indices of a batch are loaded first,
 // then their positions, so each thread keeps this many gathers in flight
@@ -1195,6 +1221,7 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
     __shared__ __align__(16) uint4 st_lo[STAGE ? FX_BLOCK : 1];
     __shared__ __align__(16) uint4 st_fb[STAGE ? FX_BLOCK : 1];
     __shared__ uint32_t st_tag[STAGE ? FX_BLOCK : 1];
+    __shared__ uint32_t s_queue[std::is_same<PE, DpdEngine>::value ? DPD_QUEUE_FX * FX_BLOCK : 1];
     if constexpr (STAGE) {
         if (active && sub == 0) {
             if constexpr (STAGE_V) {
@@ -1211,10 +1238,8 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
     uint4 fi = make_uint4(0u, 0u, 0u, 0u);
     uint32_t n = 0u;
     if constexpr (!std::is_same<PE, NoPair>::value) n = active ? min(__ldg(a.counts + i), a.max_nn) : 0u;
-#if AZP_FX_PREFETCH || AZP_FX_UNIFORM
     // the warp's longest list row
     const uint32_t nmax = __reduce_max_sync(0xffffffffu, n);
-#endif
 #if AZP_FX_PREFETCH
     {
         const uint32_t i0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> a.tpp_shift;
@@ -1225,22 +1250,63 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
         }
     }
 #endif
-    if (active) {
-        fi = __ldg(a.fix + i);
-        // ---------------------------------------------------------------- pair
-        if constexpr (!std::is_same<PE, NoPair>::value) {
-            const uint32_t* col = a.nbrs + i;
-            uint32_t k0 = 0, k1 = 0, tgi = 0;
-            float4 vi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if constexpr (std::is_same<PE, DpdEngine>::value) {
-                dpd_key(a, force_timestep<INTEG>(a), k0, k1);
-                tgi = __ldg(a.tag + i);
-                vi = reinterpret_cast<const float4*>(a.dvel)[i];
+    if (active) fi = __ldg(a.fix + i);
+    // -------------------------------------------------------------------- DPD pairs
+    if constexpr (std::is_same<PE, DpdEngine>::value) {
+        // Two phases, as the FP64 step: the scan queues the partners inside
+        // r_cut, the warp then evaluates its queues together (a Philox draw
+        // and the weight a pair cost far more than the scan). Bit 31 marks
+        // the first partner of a batch, so that the batch sums are the ones
+        // of a walk that evaluates as it goes.
+        uint32_t* queue = s_queue + threadIdx.x;
+        const uint32_t* col = a.nbrs + i;
+        uint32_t k0 = 0, k1 = 0, tgi = 0;
+        float4 vi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        dpd_key(a, force_timestep<INTEG>(a), k0, k1);
+        if (active) {
+            vi = __ldg(reinterpret_cast<const float4*>(a.dvel) + i);
+            tgi = __float_as_uint(vi.w);
+        }
+        uint32_t nq = 0;
+        for (uint32_t kb = 0; kb < nmax; kb += FX_BATCH * tpp) {
+            uint32_t jj[FX_BATCH];
+            uint4 fj[FX_BATCH];
+            const uint32_t k = kb + sub * FX_BATCH;
+#pragma unroll
+            for (int u = 0; u < FX_BATCH; ++u) jj[u] = k + u < n ? __ldg(col + (size_t)(k + u) * a.N) : 0u;
+#pragma unroll
+            for (int u = 0; u < FX_BATCH; ++u) fj[u] = __ldg(a.fix + jj[u]);
+            uint32_t mark = 0x80000000u;
+#pragma unroll
+            for (int u = 0; u < FX_BATCH; ++u) {
+                const float dx = (float)(int32_t)(fi.x - fj[u].x) * a.sfix[0];
+                const float dy = (float)(int32_t)(fi.y - fj[u].y) * a.sfix[1];
+                const float dz = (float)(int32_t)(fi.z - fj[u].z) * a.sfix[2];
+                const float rc2 = s_rec[(size_t)(ONE ? 0u : fi.w * a.ntypes + fj[u].w) * PAIR_TBL + PAIR_REC];
+                if (k + u < n && rc2 > 0.0f && dx * dx + dy * dy + dz * dz < rc2 * DPD_SCREEN) {
+                    queue[FX_BLOCK * nq++] = jj[u] | mark;
+                    mark = 0u;
+                }
             }
+            if (kb + FX_BATCH * tpp < nmax && !__any_sync(0xffffffffu, nq > DPD_QUEUE_FX - FX_BATCH)) continue;
+            for (uint32_t m = 0; m < nq; ++m) {
+                const uint32_t e = queue[FX_BLOCK * m];
+                if (e & 0x80000000u) acc.commit(vir);
+                const uint32_t j = e & 0x7fffffffu;
+                pair_term_dpd_fx<ONE>(a, fi, __ldg(a.fix + j), i, j, s_rec, s_rc2, acc, vir, vi, tgi, k0, k1);
+            }
+            nq = 0;
+        }
+        acc.commit(vir);
+    }
+    if (active) {
+        // ---------------------------------------------------------------- pair
+        if constexpr (!std::is_same<PE, NoPair>::value && !std::is_same<PE, DpdEngine>::value) {
+            const uint32_t* col = a.nbrs + i;
 #if AZP_FX_UNIFORM
             // every lane walks to the warp's longest row; slots past a lane's own
             // row are masked (no per-lane loop exit)
-            const uint32_t kend = std::is_same<PE, DpdEngine>::value ? n : nmax;
+            const uint32_t kend = nmax;
 #else
             const uint32_t kend = n;
 #endif
@@ -1250,11 +1316,13 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
             uint32_t jn[FX_BATCH];
 #pragma unroll
             for (int u = 0; u < FX_BATCH; ++u) {
-                const uint32_t k = sub + u * tpp;
+                const uint32_t k = sub * FX_BATCH + u;
                 jn[u] = k < n ? __ldg(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
             }
 #endif
-            for (uint32_t kb = sub; kb < kend; kb += FX_BATCH * tpp) {
+            // a lane's batch is FX_BATCH consecutive entries, so that the batch sums (and
+            // with them the force) do not depend on the threads per particle
+            for (uint32_t kb = sub * FX_BATCH; kb < kend; kb += FX_BATCH * tpp) {
                 uint32_t jj[FX_BATCH];
                 uint4 fj[FX_BATCH];
 #if AZP_FX_PIPE
@@ -1263,7 +1331,7 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
 #else
 #pragma unroll
                 for (int u = 0; u < FX_BATCH; ++u) {
-                    const uint32_t k = kb + u * tpp;
+                    const uint32_t k = kb + u;
                     jj[u] = k < n ? __ldg(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
                 }
 #endif
@@ -1278,21 +1346,18 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
 #if AZP_FX_PIPE
 #pragma unroll
                 for (int u = 0; u < FX_BATCH; ++u) {
-                    const uint32_t k = kb + (FX_BATCH + u) * tpp;
+                    const uint32_t k = kb + FX_BATCH * tpp + u;
                     jn[u] = k < n ? __ldg(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
                 }
 #endif
 #pragma unroll
                 for (int u = 0; u < FX_BATCH; ++u) {
-                    if constexpr (std::is_same<PE, DpdEngine>::value) {
-                        if (kb + u * tpp < n)
-                            pair_term_dpd_fx<ONE>(a, fi, fj[u], i, jj[u], s_rec, s_rc2, acc, vir, vi, tgi, k0, k1);
-                    } else {
+                    {
 #if AZP_FX_UNIFORM
-                        pair_term_fx_masked<PE, TILE, ONE>(a, fi, fj[u], i, jj[u], kb + u * tpp < n, s_rec, s_rc2,
+                        pair_term_fx_masked<PE, TILE, ONE>(a, fi, fj[u], i, jj[u], kb + u < n, s_rec, s_rc2,
                                                            acc, vir, trec);
 #else
-                        if (kb + u * tpp < n) pair_term_fx<PE, ONE>(a, fi, fj[u], i, jj[u], s_rec, s_rc2, acc, vir);
+                        if (kb + u < n) pair_term_fx<PE, ONE>(a, fi, fj[u], i, jj[u], s_rec, s_rc2, acc, vir);
 #endif
                     }
                 }
@@ -1312,8 +1377,8 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
             }
         } else if constexpr (!std::is_same<BE, NoBond>::value) {
             const uint32_t nb = __ldg(a.bt_n + i);
-            for (uint32_t k0 = sub; k0 < nb; k0 += 2u * tpp) {
-                const uint32_t k1 = k0 + tpp;
+            for (uint32_t k0 = 2u * sub; k0 < nb; k0 += 2u * tpp) {
+                const uint32_t k1 = k0 + 1u;
                 const uint2 e0 = __ldg(a.bt + (size_t)k0 * a.N + i);
                 const uint2 e1 = k1 < nb ? __ldg(a.bt + (size_t)k1 * a.N + i) : make_uint2(i, 0u);
                 const uint4 f0 = __ldg(a.fix + e0.x);
@@ -1466,7 +1531,7 @@ int launch_md_t(const MDArgs& a, cudaStream_t s)
                 smem_k = (size_t)TILE_CAP * sizeof(uint4);
             }
         }
-        if (smem_k > 32 * 1024)
+        if (smem_k > 8 * 1024)  // beside up to 33 KB of static shared memory
             AZP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
         k<<<blocks, FX_BLOCK, smem_k, s>>>(a);
         AZP_CHECK_LAUNCH("k_md_step_fx");

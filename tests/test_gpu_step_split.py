@@ -80,3 +80,17 @@ def test_fp64_step_at_every_split(orc, N, rcut, mode, tpp):
 def test_fp64_step_with_bonds(orc, tpp):
     dx, f, u, w = _run(orc, 901, 1.5, "none", "fp64", tpp, bonds=True)
     assert dx < 1e-9 and f < 1e-10 and u < 1e-12 and w < 1e-11
+
+
+@pytest.mark.parametrize("tpp", [0, 1, 2, 4, 8, 16, 32])
+@pytest.mark.parametrize("N,rcut,mode", [(1025, 2.9, "shift"), (700, 1.2, "none"), (1501, 2.5, "xplor")])
+def test_fp32_step_at_every_split(orc, N, rcut, mode, tpp):
+    # the FP32 force budget of the other tests; the virial sums up to 130 FP32 terms
+    dx, f, u, w = _run(orc, N, rcut, mode, "fp32", tpp)
+    assert dx < 1e-6 and f < 1e-5 and u < 1e-6 and w < 1e-5
+
+
+@pytest.mark.parametrize("tpp", [1, 4, 32])
+def test_fp32_step_with_bonds(orc, tpp):
+    dx, f, u, w = _run(orc, 901, 1.5, "none", "fp32", tpp, bonds=True)
+    assert dx < 1e-6 and f < 1e-5 and u < 1e-6 and w < 1e-5
