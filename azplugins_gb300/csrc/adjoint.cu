@@ -18,6 +18,7 @@
 #include "evaluators.cuh"
 #include "nlist_impl.cuh"
 #include "pair.cuh"
+#include "walk64.cuh"
 
 namespace azp
 {
@@ -62,52 +63,52 @@ struct PairDerivs {
     double phi, dphi_ds, dphi_dp[4], de_dp[4];
 };
 
-// PerturbedLennardJones, written out. p = (sigma_6, epsilon_x_4, lambda, rwcasq).
-AZP_D PairDerivs plj_derivs(const D5* rec, double s)
-{
-    PairDerivs r;
-    const double lj1 = rec[0].v, lj2 = rec[1].v, lam = rec[2].v, rwcasq = rec[3].v;
-    // dlj/dp from the dual record: lj1 = e4 s6^2, lj2 = e4 s6
-    const double dlj1_ds6 = rec[0].d[1], dlj1_de4 = rec[0].d[2];
-    const double dlj2_ds6 = rec[1].d[1], dlj2_de4 = rec[1].d[2];
-    const double x2 = 1.0 / s;
-    const double r6 = x2 * x2 * x2;
-    const double phi_lj = x2 * r6 * (12.0 * lj1 * r6 - 6.0 * lj2);
-    const double e_lj = r6 * (lj1 * r6 - lj2);
-    const double dphi_lj = x2 * x2 * r6 * (-84.0 * lj1 * r6 + 24.0 * lj2);
-    const double dphi_dlj1 = 12.0 * x2 * r6 * r6, dphi_dlj2 = -6.0 * x2 * r6;
-    const double de_dlj1 = r6 * r6, de_dlj2 = -r6;
-    const double dphi_lj_ds6 = dphi_dlj1 * dlj1_ds6 + dphi_dlj2 * dlj2_ds6;
-    const double dphi_lj_de4 = dphi_dlj1 * dlj1_de4 + dphi_dlj2 * dlj2_de4;
-    const double de_lj_ds6 = de_dlj1 * dlj1_ds6 + de_dlj2 * dlj2_ds6;
-    const double de_lj_de4 = de_dlj1 * dlj1_de4 + de_dlj2 * dlj2_de4;
-    if (s < rwcasq) {
-        // WCA core: U_LJ + eps (1 - lambda), eps = e4 / 4
-        r.phi = phi_lj;
-        r.dphi_ds = dphi_lj;
-        r.dphi_dp[0] = dphi_lj_ds6;
-        r.dphi_dp[1] = dphi_lj_de4;
-        r.dphi_dp[2] = 0.0;
-        r.de_dp[0] = de_lj_ds6;
-        r.de_dp[1] = de_lj_de4 + rec[4].d[2];   // d wca_shift / d e4
-        r.de_dp[2] = rec[4].d[3];               // d wca_shift / d lambda
-    } else {
-        r.phi = lam * phi_lj;
-        r.dphi_ds = lam * dphi_lj;
-        r.dphi_dp[0] = lam * dphi_lj_ds6;
-        r.dphi_dp[1] = lam * dphi_lj_de4;
-        r.dphi_dp[2] = phi_lj;
-        r.de_dp[0] = lam * de_lj_ds6;
-        r.de_dp[1] = lam * de_lj_de4;
-        r.de_dp[2] = e_lj;
+// PerturbedLennardJones, written out. p = (sigma_6, epsilon_x_4, lambda, rwcasq);
+// rwcasq only moves the (continuous) branch point. With G.d (Gdd) and
+// g = (dL/dU_i + dL/dU_j) / 2 of a pair, its parameter gradient (twice it: each
+// ordered pair carries half) is a combination of five sums with the per-type
+// constants of the dual record, so a pair adds to the sums alone:
+//   a1 = f r^-12 (12 r^-2 Gdd + g), a2 = -f r^-6 (6 r^-2 Gdd + g) with f = 1 in the
+//   WCA core and lambda outside (d/dlj1, d/dlj2); tail = Gdd phi + g e of the bare
+//   potential outside the core (d/dlambda); core = g in the core (the WCA shift);
+//   all = g (the energy shift at r_cut).
+struct PljSums {
+    double a1 = 0.0, a2 = 0.0, tail = 0.0, core = 0.0, all = 0.0;
+    // gp[4] of these sums for one type pair
+    AZP_D void combine(const D5* rec, double* gp) const
+    {
+        const D5 &lj1 = rec[0], &lj2 = rec[1], &shift = rec[PerturbedLJ::SHIFT_SLOT];
+        // dlj/dp from the dual record: lj1 = e4 s6^2, lj2 = e4 s6
+        gp[0] += a1 * lj1.d[1] + a2 * lj2.d[1] - all * shift.d[1];
+        gp[1] += a1 * lj1.d[2] + a2 * lj2.d[2] + core * rec[4].d[2] - all * shift.d[2];
+        gp[2] += tail + core * rec[4].d[3] - all * shift.d[3];
+        gp[3] -= all * shift.d[4];
     }
-    r.dphi_dp[3] = 0.0;  // rwcasq only moves the (continuous) branch point
-    r.de_dp[3] = 0.0;
-    // energy shift at r_cut (zero unless shifting)
-    const D5& sh = rec[PerturbedLJ::SHIFT_SLOT];
-    for (int m = 0; m < 4; ++m) r.de_dp[m] -= sh.d[1 + m];
-    return r;
-}
+    // one pair: phi and phi', and its terms of the sums
+    AZP_D void add(const D5* rec, double s, double Gdd, double g, double& phi, double& dphi_ds)
+    {
+        const double lj1 = rec[0].v, lj2 = rec[1].v;
+        const double x2 = rcp(s);
+        const double r6 = x2 * x2 * x2;
+        const double x8 = x2 * r6;
+        const double p = x8 * fma(12.0 * lj1, r6, -6.0 * lj2);
+        const double d = x2 * x8 * fma(-84.0 * lj1, r6, 24.0 * lj2);
+        const double u = x2 * Gdd;
+        const double t1 = r6 * fma(12.0, u, g);  // times r^-6 below
+        const double t2 = fma(6.0, u, g);
+        const bool inner = less_nonneg(s, rec[3].v);
+        // f r^-6: the factor of both potential terms
+        const double f = inner ? 1.0 : rec[2].v;
+        const double fr6 = f * r6;
+        phi = f * p;
+        dphi_ds = f * d;
+        a1 = fma(fr6, t1, a1);
+        a2 = fma(-fr6, t2, a2);
+        all += g;
+        if (inner) core += g;
+        else tail = fma(g * r6, fma(lj1, r6, -lj2), fma(Gdd, p, tail));
+    }
+};
 
 template<class Eval> AZP_D PairDerivs dual_derivs(const D5* rec, double s)
 {
@@ -127,52 +128,77 @@ template<class Eval> AZP_D PairDerivs dual_derivs(const D5* rec, double s)
     return r;
 }
 
-// WRITTEN: the hand-written PerturbedLennardJones derivatives (no smoothing);
-// otherwise the dual-number path. Separate instantiations keep the dual
-// records' registers out of the hand-written kernel.
-template<class Eval, bool WRITTEN>
+// The adjoint of one force call. FORM 0: the dual-number path; 1: the hand-written
+// PerturbedLennardJones derivatives (no smoothing), 2: the same for one particle
+// type, whose sums are combined once per particle. Separate instantiations keep the
+// dual records' registers out of the hand-written kernels. FP64-pipe bound: partners
+// inside r_cut by the FP32 scan of walk64.cuh.
+constexpr int ADJ_DUAL = 0, ADJ_PLJ = 1, ADJ_PLJ_ONE = 2;
+template<class Eval, int FORM>
 __global__ void __launch_bounds__(ADJ_BLOCK) k_pair_adjoint(AdjArgs a)
 {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* s_cut = reinterpret_cast<double*>(smem_raw);
+    float* s_thr = reinterpret_cast<float*>(s_cut + 2 * a.ntypes * a.ntypes);
+    uint32_t* s_queue = reinterpret_cast<uint32_t*>(s_thr + a.ntypes * a.ntypes);
+    const WalkBox box = walk_box(a.L);
+    for (uint32_t t = threadIdx.x; t < a.ntypes * a.ntypes; t += blockDim.x) {
+        const D5* rec = a.table + (size_t)t * PAIR_TBL;
+        const bool on = Eval::enabled(rec);
+        s_cut[2 * t] = on ? rec[PAIR_REC].v : 0.0;
+        s_cut[2 * t + 1] = cut_low(s_cut[2 * t]);
+        s_thr[t] = walk_threshold(box, rec[PAIR_REC].v, on);
+    }
+    __syncthreads();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int tpp = a.tpp;
+    const uint32_t tpp = (uint32_t)a.tpp;
     const uint32_t i = gid / tpp;
     const uint32_t sub = gid % tpp;
     const bool active = i < a.N;
-    double gx = 0, gy = 0, gz = 0, gp[4] = {0, 0, 0, 0};
+    const double h0 = half_edge(a.L[0]), h1 = half_edge(a.L[1]), h2 = half_edge(a.L[2]);
+    double4_32a pi = make_double4_32a(0.0, 0.0, 0.0, 0.0), Gi = pi;
     if (active) {
-        const double4_32a pi = a.pos[i];
-        const double4_32a Gi = a.grad[i];
-        const uint32_t ti = type_of(pi.w);
-        const uint32_t n = min(a.counts[i], a.max_nn);
-        for (uint32_t k = sub; k < n; k += tpp) {
-            const uint32_t j = a.nbrs[(size_t)k * a.N + i];
-            const double4_32a pj = a.pos[j];
-            const double dx = min_image1(pi.x - pj.x, a.L[0], a.Linv[0]);
-            const double dy = min_image1(pi.y - pj.y, a.L[1], a.Linv[1]);
-            const double dz = min_image1(pi.z - pj.z, a.L[2], a.Linv[2]);
-            const double s = rsq_exact(dx, dy, dz);
-            const uint32_t tp = ti * a.ntypes + type_of(pj.w);
-            const D5* rec = a.table + (size_t)tp * PAIR_TBL;
-            const D5* cut = rec + PAIR_REC;
-            if (!(s < cut[0].v) || !Eval::enabled(rec)) continue;
-            PairDerivs q;
-            if constexpr (WRITTEN)
-                q = plj_derivs(rec, s);
-            else
-                q = dual_derivs<Eval>(rec, s);
-            const double4_32a Gj = a.grad[j];
-            const double Gx = Gi.x - Gj.x, Gy = Gi.y - Gj.y, Gz = Gi.z - Gj.z;
-            const double g = 0.5 * (Gi.w + Gj.w);
-            const double Gdd = Gx * dx + Gy * dy + Gz * dz;
-            const double c2 = 2.0 * q.dphi_ds * Gdd - g * q.phi;
-            gx += q.phi * Gx + c2 * dx;
-            gy += q.phi * Gy + c2 * dy;
-            gz += q.phi * Gz + c2 * dz;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) gp[m] += 0.5 * (Gdd * q.dphi_dp[m] + g * q.de_dp[m]);
-        }
+        pi = a.pos[i];
+        Gi = a.grad[i];
     }
-    for (int m = tpp >> 1; m > 0; m >>= 1) {
+    const uint32_t row = active ? type_of(pi.w) * a.ntypes : 0u;
+    double gx = 0, gy = 0, gz = 0, gp[4] = {0, 0, 0, 0};
+    PljSums sums;
+    walk_fp64(a.pos, a.nbrs, a.N, i, active, active ? min(a.counts[i], a.max_nn) : 0u, tpp, pi, s_thr + row, box,
+              s_queue, [&](uint32_t j) {
+                  const double4_32a pj = a.pos[j];
+                  const double dx = min_image_if(pi.x - pj.x, h0, a.L[0], a.Linv[0]);
+                  const double dy = min_image_if(pi.y - pj.y, h1, a.L[1], a.Linv[1]);
+                  const double dz = min_image_if(pi.z - pj.z, h2, a.L[2], a.Linv[2]);
+                  const uint32_t tp = row + type_of(pj.w);
+                  const D5* rec = a.table + (size_t)tp * PAIR_TBL;
+                  double s;
+                  if (!pair_inside(dx, dy, dz, s_cut + 2 * tp, s)) return;
+                  const double4_32a Gj = a.grad[j];
+                  const double Gx = Gi.x - Gj.x, Gy = Gi.y - Gj.y, Gz = Gi.z - Gj.z;
+                  const double g = 0.5 * (Gi.w + Gj.w);
+                  const double Gdd = Gx * dx + Gy * dy + Gz * dz;
+                  double phi, dphi_ds;
+                  if constexpr (FORM == ADJ_DUAL) {
+                      const PairDerivs q = dual_derivs<Eval>(rec, s);
+                      phi = q.phi;
+                      dphi_ds = q.dphi_ds;
+#pragma unroll
+                      for (int m = 0; m < 4; ++m) gp[m] += Gdd * q.dphi_dp[m] + g * q.de_dp[m];
+                  } else if constexpr (FORM == ADJ_PLJ) {
+                      PljSums one;
+                      one.add(rec, s, Gdd, g, phi, dphi_ds);
+                      one.combine(rec, gp);
+                  } else {
+                      sums.add(rec, s, Gdd, g, phi, dphi_ds);
+                  }
+                  const double c2 = 2.0 * dphi_ds * Gdd - g * phi;
+                  gx = fma(c2, dx, fma(phi, Gx, gx));
+                  gy = fma(c2, dy, fma(phi, Gy, gy));
+                  gz = fma(c2, dz, fma(phi, Gz, gz));
+              });
+    if constexpr (FORM == ADJ_PLJ_ONE) sums.combine(a.table, gp);
+    for (uint32_t m = tpp >> 1; m > 0; m >>= 1) {
         gx += __shfl_xor_sync(0xffffffffu, gx, m);
         gy += __shfl_xor_sync(0xffffffffu, gy, m);
         gz += __shfl_xor_sync(0xffffffffu, gz, m);
@@ -183,8 +209,9 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_pair_adjoint(AdjArgs a)
         a.grad_pos[3 * (size_t)i] = gx;
         a.grad_pos[3 * (size_t)i + 1] = gy;
         a.grad_pos[3 * (size_t)i + 2] = gz;
+        // (each ordered pair carries half of the parameter gradient)
         if (a.grad_params)
-            for (int c = 0; c < 4; ++c) a.grad_params[4 * (size_t)i + c] = gp[c];
+            for (int c = 0; c < 4; ++c) a.grad_params[4 * (size_t)i + c] = 0.5 * gp[c];
     }
 }
 
@@ -272,10 +299,15 @@ int launch_adj(const azp_system* sys, azp_nlist* nl, const double* params, const
     a.xplor = mode == AZP_MODE_XPLOR;
     const size_t threads = (size_t)sys->N * a.tpp;
     const uint32_t blocks = (uint32_t)((threads + ADJ_BLOCK - 1) / ADJ_BLOCK);
-    if (std::is_same<Eval, PerturbedLJ>::value && !a.xplor)
-        k_pair_adjoint<PerturbedLJ, true><<<blocks, ADJ_BLOCK, 0, s>>>(a);
-    else
-        k_pair_adjoint<Eval, false><<<blocks, ADJ_BLOCK, 0, s>>>(a);
+    const size_t smem = nt2 * (2 * sizeof(double) + sizeof(float)) + walk_queue_words(ADJ_BLOCK) * sizeof(uint32_t);
+    if (std::is_same<Eval, PerturbedLJ>::value && !a.xplor) {
+        if (a.ntypes == 1)
+            k_pair_adjoint<PerturbedLJ, ADJ_PLJ_ONE><<<blocks, ADJ_BLOCK, smem, s>>>(a);
+        else
+            k_pair_adjoint<PerturbedLJ, ADJ_PLJ><<<blocks, ADJ_BLOCK, smem, s>>>(a);
+    } else {
+        k_pair_adjoint<Eval, ADJ_DUAL><<<blocks, ADJ_BLOCK, smem, s>>>(a);
+    }
     AZP_CHECK_LAUNCH("k_pair_adjoint");
     return AZP_OK;
 }

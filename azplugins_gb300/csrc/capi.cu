@@ -281,6 +281,7 @@ int azp_pair_forces(const azp_system* sys, azp_nlist* nl, int kind, const double
     a.nbrs = nl->nbrs;
     a.max_nn = nl->max_nn;
     a.table = nl->table;
+    a.xplor = shift_mode == AZP_MODE_XPLOR ? 1 : 0;
     a.force = out->force;
     a.virial = out->virial;
     a.pitch = out->virial_pitch ? out->virial_pitch : sys->N;

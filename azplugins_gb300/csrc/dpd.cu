@@ -20,6 +20,7 @@
 #include "nlist_impl.cuh"
 #include "pair.cuh"
 #include "philox.cuh"
+#include "walk64.cuh"
 
 namespace azp
 {
@@ -84,12 +85,15 @@ __global__ void k_vel_f(const double4_32a* __restrict__ vel, uint32_t N, float4*
 // usual choices) as square roots, which agree with pow to an ulp or two and
 // avoid its cost (in FP64 a pow costs as much as the rest of the pair); any
 // other exponent through pow
+static __device__ __noinline__ double dpd_weight_pow(double x, double h) { return pow(x, h); }
 AZP_D double dpd_weight(double x, double h)
 {
-    if (h == 0.5) return sqrt(x);
-    if (h == 0.25) return sqrt(sqrt(x));
-    if (h == 1.0) return x;
-    return pow(x, h);
+    // (the first root is shared by the lanes of h = 1/2 and 1/4; pow out of line)
+    const bool half = h == 0.5, quarter = h == 0.25;
+    if (!half && !quarter && h != 1.0) return dpd_weight_pow(x, h);
+    if (half || quarter) x = d_sqrt(x);
+    if (quarter) x = d_sqrt(x);
+    return x;
 }
 
 AZP_D float dpd_weight_f(float x, float h)
@@ -122,20 +126,29 @@ AZP_D bool dpd_pair_fp64(const DpdArgs& a, const double* c, const double4_32a& p
                          const double4_32a& vi, const double4_32a& vj, uint32_t tgi, uint32_t tgj, double& dx,
                          double& dy, double& dz, double& fdr, double& fc, double& e)
 {
-    dx = min_image1(pi.x - pj.x, a.L[0], a.Linv[0]);
-    dy = min_image1(pi.y - pj.y, a.L[1], a.Linv[1]);
-    dz = min_image1(pi.z - pj.z, a.L[2], a.Linv[2]);
-    const double rs = rsq_exact(dx, dy, dz);
-    if (!(rs < c[0])) return false;
-    const double rinv = 1.0 / sqrt(rs);
-    const double r = 1.0 / rinv;
+    dx = min_image_if(pi.x - pj.x, half_edge(a.L[0]), a.L[0], a.Linv[0]);
+    dy = min_image_if(pi.y - pj.y, half_edge(a.L[1]), a.L[1], a.Linv[1]);
+    dz = min_image_if(pi.z - pj.z, half_edge(a.L[2]), a.L[2], a.Linv[2]);
+    double rs, rinv;
+    const double cut[2] = {c[0], cut_low(c[0])};
+    if (!pair_inside(dx, dy, dz, cut, rs)) return false;
+    const double r = d_sqrt(rs, rinv);
     const double dot = dx * (vi.x - vj.x) + dy * (vi.y - vj.y) + dz * (vi.z - vj.z);
     fc = c[3] * (rinv - c[1]);
-    const double wR = dpd_weight(fmax(1.0 - r * c[1], 0.0), c[5]) * rinv;  // never below 0 (r < r_cut)
+    const double wR = dpd_weight(nonneg(1.0 - r * c[1]), c[5]) * rinv;  // never below 0 (r < r_cut)
     const double alpha = dpd_alpha(a.k0, a.k1, tgi, tgj);
     fdr = fc - c[4] * wR * wR * dot + c[6] * wR * alpha;
     e = c[3] * (c[2] - r) - 0.5 * c[3] * c[1] * (c[0] - rs);
     return true;
+}
+
+// the same out of line, for the FP32 kernel's rare pairs (its registers do not
+// count against the pair loop)
+static __device__ __noinline__ bool dpd_pair_fp64_call(const DpdArgs& a, const double* c, uint32_t i, uint32_t j,
+                                                       double& dx, double& dy, double& dz, double& fdr, double& fc,
+                                                       double& e)
+{
+    return dpd_pair_fp64(a, c, a.pos[i], a.pos[j], a.vel[i], a.vel[j], a.tag[i], a.tag[j], dx, dy, dz, fdr, fc, e);
 }
 
 template<typename R> struct DpdAcc;
@@ -215,9 +228,9 @@ template<> struct DpdAcc<float> {
 };
 
 // FP32: at most 64 registers a thread (4 blocks an SM): the kernel is latency
-// bound and gains more from resident warps than from registers
+// bound and gains more from resident warps than from registers; FP64: 2 blocks
 template<typename R, int TPP>
-__global__ void __launch_bounds__(DPD_BLOCK, std::is_same<R, float>::value ? 4 : 1) k_dpd(DpdArgs a)
+__global__ void __launch_bounds__(DPD_BLOCK, std::is_same<R, float>::value ? 4 : 2) k_dpd(DpdArgs a)
 {
     // the type-pair table in FP64 (FP64 pairs) and, for the FP32 path, as floats
     // (converted once per block, not per pair)
@@ -229,28 +242,41 @@ __global__ void __launch_bounds__(DPD_BLOCK, std::is_same<R, float>::value ? 4 :
         s_tbl[t] = a.table[t];
         if constexpr (std::is_same<R, float>::value) s_tf[t] = (float)a.table[t];
     }
-    __syncthreads();
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = gid / TPP;
     const uint32_t sub = gid % TPP;
     const bool active = i < a.N;
     DpdAcc<R> acc;
+    if constexpr (std::is_same<R, double>::value) {
+        // FP64-pipe bound: partners inside r_cut by the FP32 scan (the thresholds
+        // take the place of the float table)
+        const WalkBox box = walk_box(a.L);
+        for (uint32_t t = threadIdx.x; t < nt2; t += blockDim.x)
+            s_tf[t] = walk_threshold(box, a.table[(size_t)t * DPD_TBL], true);
+        __syncthreads();
+        double4_32a pi = make_double4_32a(0.0, 0.0, 0.0, 0.0), vi = pi;
+        uint32_t tgi = 0u;
+        if (active) {
+            pi = a.pos[i];
+            vi = a.vel[i];
+            tgi = a.tag[i];
+        }
+        const uint32_t row = active ? type_of(pi.w) * a.ntypes : 0u;
+        walk_fp64(a.pos, a.nbrs, a.N, i, active, active ? min(a.counts[i], a.max_nn) : 0u, (uint32_t)TPP, pi, s_tf + row,
+                  box, s_queue, [&](uint32_t j) {
+                      const double4_32a pj = a.pos[j];
+                      const double* c = s_tbl + (size_t)(row + type_of(pj.w)) * DPD_TBL;
+                      double dx, dy, dz, fdr, fc, e;
+                      if (dpd_pair_fp64(a, c, pi, pj, vi, a.vel[j], tgi, a.tag[j], dx, dy, dz, fdr, fc, e))
+                          acc.add(dx, dy, dz, fdr, fc, e);
+                  });
+    } else {
+        __syncthreads();
+    }
     if (active) {
         const uint32_t n = min(a.counts[i], a.max_nn);
         const uint32_t tgi = a.tag[i];
-        if constexpr (std::is_same<R, double>::value) {
-            const double4_32a pi = a.pos[i];
-            const double4_32a vi = a.vel[i];
-            const uint32_t ti = type_of(pi.w);
-            for (uint32_t k = sub; k < n; k += TPP) {
-                const uint32_t j = a.nbrs[(size_t)k * a.N + i];
-                const double4_32a pj = a.pos[j];
-                const double* c = s_tbl + (size_t)(ti * a.ntypes + type_of(pj.w)) * DPD_TBL;
-                double dx, dy, dz, fdr, fc, e;
-                if (!dpd_pair_fp64(a, c, pi, pj, vi, a.vel[j], tgi, a.tag[j], dx, dy, dz, fdr, fc, e)) continue;
-                acc.add(dx, dy, dz, fdr, fc, e);
-            }
-        } else {
+        if constexpr (std::is_same<R, float>::value) {
             const uint4 fi = a.fixed[i];
             const float4 vi = a.vel_f[i];
             const uint32_t ti = fi.w;
@@ -335,8 +361,7 @@ __global__ void __launch_bounds__(DPD_BLOCK, std::is_same<R, float>::value ? 4 :
                     // other boxes: such pairs (about 0.3 % of them) in FP64 from the
                     // FP64 state, which also decides the cutoff as the oracle does
                     double ddx, ddy, ddz, dfdr, dfc, de;
-                    if (dpd_pair_fp64(a, c, a.pos[i], a.pos[j], a.vel[i], a.vel[j], tgi, a.tag[j], ddx, ddy, ddz, dfdr,
-                                      dfc, de))
+                    if (dpd_pair_fp64_call(a, c, i, j, ddx, ddy, ddz, dfdr, dfc, de))
                         acc.add((float)ddx, (float)ddy, (float)ddz, (float)dfdr, (float)dfc, (float)de);
                 }
             }
@@ -412,7 +437,8 @@ extern "C" int azp_dpd_forces(const azp_system* sys, azp_nlist* nl, const double
     a.virial = out->virial;
     a.pitch = out->virial_pitch ? out->virial_pitch : sys->N;
     const size_t smem = (size_t)nt2 * DPD_TBL * (sizeof(double) + sizeof(float)) +
-                        (out->precision == AZP_FP32 ? (size_t)DPD_BLOCK * DPD_QUEUE * sizeof(uint32_t) : 0);
+                        (out->precision == AZP_FP32 ? (size_t)DPD_BLOCK * DPD_QUEUE * sizeof(uint32_t)
+                                                    : walk_queue_words(DPD_BLOCK) * sizeof(uint32_t));
     if (out->precision == AZP_FP32) {
         launch_to_fixed(a.pos, nl->fixed, sys->N, sys->box, s);
         k_vel_f<<<(sys->N + 255) / 256, 256, 0, s>>>(a.vel, sys->N, nl->vel_f);

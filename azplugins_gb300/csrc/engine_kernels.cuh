@@ -312,12 +312,15 @@ AZP_D void dpd_key(const MDArgs& a, unsigned long long ts, uint32_t& k0, uint32_
     stream_key(AZP_RNG_DPD_GENERAL_WEIGHT, ts, a.seed, k0, k1);
 }
 
+// (the first root is shared by the lanes of h = 1/2 and 1/4; pow out of line)
+static __device__ __noinline__ double dpd_weight_pow(double x, double h) { return pow(x, h); }
 AZP_D double dpd_weight_engine(double x, double h)
 {
-    if (h == 0.5) return d_sqrt(x);
-    if (h == 0.25) return d_sqrt(d_sqrt(x));
-    if (h == 1.0) return x;
-    return pow(x, h);
+    const bool half = h == 0.5, quarter = h == 0.25;
+    if (!half && !quarter && h != 1.0) return dpd_weight_pow(x, h);
+    if (half || quarter) x = d_sqrt(x);
+    if (quarter) x = d_sqrt(x);
+    return x;
 }
 
 AZP_D float dpd_weight_engine_f(float x, float h)
@@ -353,7 +356,7 @@ AZP_D bool dpd_term_fp64(const double* rec, double rcutsq, double dx, double dy,
                          double& e)
 {
     const double rs = rsq_exact(dx, dy, dz);
-    if (!(rs < rcutsq)) return false;
+    if (!less_nonneg(rs, rcutsq)) return false;
     const double rcinv = rec[0], rc = rec[1], A = rec[2], gamma = rec[3];
     double rinv;
     const double r = d_sqrt(rs, rinv);
@@ -371,14 +374,14 @@ AZP_D bool dpd_term_fp64(const double* rec, double rcutsq, double dx, double dy,
 // energy shift it needs) and the cap of the overlap relaxation. Out of line, with an
 // evaluation of its own, so that the plain step computes no energy for it.
 template<class PE>
-static __device__ __noinline__ double adjusted_fp64(const MDArgs& a, const double* rec, double rsq, double& e)
+static __device__ __noinline__ double2 adjusted_fp64(const MDArgs& a, const double* rec, double rsq)
 {
-    double fdr;
+    double fdr, e;
     PE::eval(rec, rsq, fdr, e);
     e -= rec[PE::SHIFT_SLOT];
     xplor(rec + PAIR_REC, rsq, fdr, e);
     if (a.capped && fdr * fdr * rsq > a.fcap * a.fcap) fdr = copysign(a.fcap / sqrt(rsq), fdr);
-    return fdr;
+    return make_double2(fdr, e);
 }
 
 // FP64 step: FP64 positions, forces and integration, the oracle's rounding for
@@ -407,16 +410,17 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
     double* s_gamma = reinterpret_cast<double*>(smem_raw);
     double* s_noise = s_gamma + a.ntypes;
     double* s_rec = s_noise + a.ntypes;
-    double* s_bond = s_rec + nt2 * PAIR_TBL;
+    double* s_bond = s_rec + nt2 * REC64;
     double* s_sum = s_bond + a.nbondtypes * BOND_REC;
     const uint32_t tpp = (uint32_t)a.tpp;
     const uint32_t P = MD_BLOCK >> a.tpp_shift;  // particles of the block
     float* s_screen = reinterpret_cast<float*>(s_sum + (tpp > 1u ? Acc64<OUT>::WORDS * P : 0u));
     if constexpr (PAIR) {
-        for (uint32_t t = threadIdx.x; t < nt2 * PAIR_TBL; t += blockDim.x) s_rec[t] = a.pair_table[t];
         for (uint32_t t = threadIdx.x; t < nt2; t += blockDim.x) {
             const double* rec = a.pair_table + (size_t)t * PAIR_TBL;
-            s_screen[t] = PE::enabled(rec) ? __double2float_ru(rec[PAIR_REC] * (1.0 + (double)a.screen)) : -1.0f;
+            const bool on = PE::enabled(rec);
+            prepare64<PE>(rec, on, s_rec + (size_t)t * REC64);
+            s_screen[t] = on ? __double2float_ru(rec[PAIR_REC] * (1.0 + (double)a.screen)) : -1.0f;
         }
     }
     if constexpr (!std::is_same<BE, NoBond>::value)
@@ -490,23 +494,24 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
                 const double dx = min_image_if(pi.x - pj.x, half0, a.L[0], a.Linv[0]);
                 const double dy = min_image_if(pi.y - pj.y, half1, a.L[1], a.Linv[1]);
                 const double dz = min_image_if(pi.z - pj.z, half2, a.L[2], a.Linv[2]);
-                const double* rec = s_rec + (size_t)(row + type_of(pj.w)) * PAIR_TBL;
-                const double* cut = rec + PAIR_REC;
+                const uint32_t tp = row + type_of(pj.w);
+                const double* rec = s_rec + (size_t)tp * REC64;
                 double fdr, e;
                 if constexpr (DPD) {
                     const double4_32a vj = reinterpret_cast<const double4_32a*>(a.dvel)[j];
                     double fc;
-                    if (dpd_term_fp64(rec, cut[0], dx, dy, dz, vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, k0, k1, tgi,
+                    if (dpd_term_fp64(rec, rec[CUT64], dx, dy, dz, vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, k0, k1, tgi,
                                       a.tag[j], fdr, fc, e))
                         acc.add(dx, dy, dz, fdr, fc, e);
                 } else {
-                    const double rsq = rsq_exact(dx, dy, dz);
-                    if (!less_nonneg(rsq, cut[0])) continue;
+                    double rsq;
+                    if (!pair_inside(dx, dy, dz, rec + CUT64, rsq)) continue;
                     if (a.xplor | a.capped) {
-                        fdr = adjusted_fp64<PE>(a, rec, rsq, e);
+                        const double2 fe = adjusted_fp64<PE>(a, a.pair_table + (size_t)tp * PAIR_TBL, rsq);
+                        fdr = fe.x;
+                        e = fe.y;
                     } else {
-                        PE::eval(rec, rsq, fdr, e);
-                        if (OUT) e -= rec[PE::SHIFT_SLOT];
+                        Pair64<PE>::template force64<OUT>(rec, rsq, fdr, e);
                     }
                     acc.add(dx, dy, dz, fdr, fdr, e);
                 }
@@ -1536,7 +1541,7 @@ int launch_md_t(const MDArgs& a, cudaStream_t s)
         k<<<blocks, FX_BLOCK, smem_k, s>>>(a);
         AZP_CHECK_LAUNCH("k_md_step_fx");
     } else {
-        const size_t smem = 2 * a.ntypes * sizeof(double) + nt2 * PAIR_TBL * sizeof(double) +
+        const size_t smem = 2 * a.ntypes * sizeof(double) + nt2 * REC64 * sizeof(double) +
                             (size_t)a.nbondtypes * BOND_REC * sizeof(double) + nt2 * sizeof(float) +
                             (a.tpp > 1 ? (size_t)(MD_BLOCK / a.tpp) * (a.out ? 10 : 3) * sizeof(double) : 0) +
                             (std::is_same<PE, NoPair>::value ? 0 : MD_BLOCK * (MD_QUEUE + 1) * sizeof(uint32_t));

@@ -339,6 +339,60 @@ template<class Eval> AZP_HD void load_bond_record(const double* p, double* q)
     for (int k = 0; k < AZP_BOND_PARAM_DOUBLES; ++k) q[k] = k < Eval::REC_DOUBLES ? p[k] : 0.0;
 }
 
+// FP64 record of a type pair as the FP64 loops read it from shared memory: the
+// evaluator's kernel record, then rcutsq (0 where the pair is off) and cut_low of it.
+// force64 gives force / r and, with ENERGY, the shifted energy.
+constexpr int REC64 = 14;
+constexpr int CUT64 = 12;
+#ifdef __CUDACC__
+template<class E> struct Pair64 {
+    AZP_D static void prepare(const double* tbl, double* q)
+    {
+        for (int k = 0; k < PAIR_REC; ++k) q[k] = tbl[k];
+        for (int k = PAIR_REC; k < CUT64; ++k) q[k] = 0.0;
+    }
+    template<bool ENERGY> AZP_D static void force64(const double* q, double rsq, double& fdr, double& e)
+    {
+        E::eval(q, rsq, fdr, e);
+        if constexpr (ENERGY) e -= q[E::SHIFT_SLOT];
+    }
+};
+// PerturbedLJ: 12 lj1, 6 lj2, lj1, lj2 and the energy offset, outside the WCA core
+// (times lambda) and inside it, then r_wca^2: the branch chooses coefficients and
+// costs no FP64 instruction
+template<> struct Pair64<PerturbedLJ> {
+    AZP_D static void prepare(const double* tbl, double* q)
+    {
+        const double lam = tbl[2], shift = tbl[PerturbedLJ::SHIFT_SLOT];
+        q[5] = tbl[5];
+        q[6] = tbl[6];
+        q[7] = tbl[0];
+        q[8] = tbl[1];
+        q[9] = tbl[4] - shift;
+        for (int k = 0; k < 4; ++k) q[k] = lam * q[5 + k];
+        q[4] = -shift;
+        q[10] = tbl[3];
+        q[11] = 0.0;
+    }
+    template<bool ENERGY> AZP_D static void force64(const double* q, double rsq, double& fdr, double& e)
+    {
+        const double* c = q + (less_nonneg(rsq, q[10]) ? 5 : 0);
+        const double r2inv = rcp(rsq);
+        const double r6inv = r2inv * r2inv * r2inv;
+        fdr = r2inv * r6inv * fma(c[0], r6inv, -c[1]);
+        if constexpr (ENERGY) e = fma(r6inv, fma(c[2], r6inv, -c[3]), c[4]);
+        else e = 0.0;
+    }
+};
+// the record of one type pair from its table entry (PAIR_TBL doubles)
+template<class E> AZP_D void prepare64(const double* tbl, bool on, double* q)
+{
+    Pair64<E>::prepare(tbl, q);
+    q[CUT64] = on ? tbl[PAIR_REC] : 0.0;
+    q[CUT64 + 1] = cut_low(q[CUT64]);
+}
+#endif
+
 // XPLOR smoothing of (fdr, e) for ronsq <= rsq < rcutsq (HOOMD pair.Pair mode
 // "xplor"): S = (rc2 - r2)^2 (rc2 + 2 r2 - 3 ro2) / (rc2 - ro2)^3.
 template<typename R> AZP_HD void xplor(const R* cut, R rsq, R& fdr, R& e)

@@ -100,5 +100,19 @@ AZP_D double min_image_if(double v, double half, double L, double Linv)
     if (magnitude_above(v, half)) v = min_image_call(v, L, Linv);
     return v;
 }
+
+// r^2 of a pair and whether it is below rcutsq as the oracle decides it (rsq_exact).
+// cut: rcutsq and rcutsq (1 - 2^-48). Below the second the fused sum, within
+// 2^-51 of the rounded one, decides; the pairs between take the exact one.
+static __device__ __noinline__ bool below_exact(double dx, double dy, double dz, double rcutsq)
+{
+    return rsq_exact(dx, dy, dz) < rcutsq;
+}
+AZP_D bool pair_inside(double dx, double dy, double dz, const double* cut, double& rsq)
+{
+    rsq = fma(dz, dz, fma(dy, dy, dx * dx));
+    return less_nonneg(rsq, cut[1]) || below_exact(dx, dy, dz, cut[0]);
+}
+AZP_D double cut_low(double rcutsq) { return rcutsq * (1.0 - 3.552713678800501e-15); }
 #endif
 }  // namespace azp

@@ -31,6 +31,7 @@ struct PairArgs {
     void* force;           // double4_32a / float4 [N]
     void* virial;          // [6][pitch] or null
     uint32_t pitch;
+    int xplor;             // mode xplor: some type pair may be smoothed
 };
 
 // host: fill table for one evaluator kind from reference param records

@@ -99,6 +99,7 @@ extern "C" int azp_pair_forces_static(const azp_system* sys, const uint32_t* cou
     a.counts = counts;
     a.nbrs = neighbors;
     a.max_nn = max_neighbors;
+    a.xplor = shift_mode == AZP_MODE_XPLOR ? 1 : 0;
     a.table = table;
     a.force = out->force;
     a.virial = out->virial;
