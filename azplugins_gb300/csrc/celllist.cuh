@@ -150,7 +150,12 @@ void launch_nlist_build(const double4_32a* pos, const uint4* fixed, uint32_t N, 
                         const ListCut* cuts, uint32_t ntypes, const uint32_t* ex_n, const uint32_t* ex_keys,
                         uint32_t ex_width, const uint32_t* keys, uint32_t* counts, uint32_t* nbrs,
                         uint32_t max_nn, uint32_t* flags, const uint32_t* gate, cudaStream_t s,
-                        const uint4* lo, double rlist_min, const uint32_t* tile = nullptr);
+                        const uint4* lo, double rlist_min, const uint32_t* tile = nullptr,
+                        const uint4* words = nullptr);
+// words (with members): fixed in cell order, which the build a warp per chunk reads
+// (warp_list_build); without it the members are gathered one thread per particle.
+bool warp_list_build(uint32_t N, const CellGrid& g, bool sorted);
+void launch_cell_words(const uint4* fixed, const uint32_t* members, uint32_t N, uint4* words, cudaStream_t s);
 // tile != NULL: particles in cell order (members NULL), entries encoded for the
 // block records of launch_tile_table.
 

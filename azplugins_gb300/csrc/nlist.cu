@@ -90,9 +90,12 @@ void make_list_cuts(const double* r_cut, uint32_t ntypes, double r_buff, const a
     }
     const double Lmax = std::max(box.L[0], std::max(box.L[1], box.L[2]));
     // worst-case relative error of the FP32 fixed-point rsq: float rounding of
-    // three components and their squares (< 1e-6) plus the fixed-point rounding
-    // of both positions (L 2^-33 each) against the smallest list radius.
+    // three components and their squares (< 1e-6), of the two coordinates relative
+    // to a particle of the cell where the warp build forms them so (each below 1.6
+    // r_list_max, so < 1e-6 r_max / r_min together), plus the fixed-point rounding of
+    // both positions (L 2^-33 each) against the smallest list radius.
     double delta = 4e-6;
+    if (rmax > 0.0) delta = 3e-6 + 2e-6 * rmax / rmin;
     if (rmax > 0.0) delta = std::max(delta, 16.0 * Lmax * 2.3283064365386963e-10 / rmin);
     for (uint32_t t = 0; t < ntypes * ntypes; ++t) {
         ListCut c;
@@ -395,6 +398,292 @@ __global__ void __launch_bounds__(NLIST_BLOCK)
     if (n > max_nn) atomicMax(&flags[0], n);
 }
 
+// The list with a warp per chunk of cell-ordered particles. A warp takes CH consecutive
+// slots of the cell order, the particles of one cell at a time. The slot ranges of their
+// stencil rows are laid end to end (bounds read and summed by the lanes together) and
+// walked 32 candidates a step, each loaded once, a step ahead, and tested against every
+// particle of the chunk: a ballot ranks the hits, which are appended to the particles' rows
+// in shared memory. Rows with excluded partners or candidates of the band are then compacted
+// there, and the rows written out with the chunk's particles side by side. Order and
+// contents are those of k_nlist_build_threads.
+// words: the candidates' fixed-point words in cell order (fixed itself when SORTED).
+// Particles whose types have smaller list radii than the grid's walk fewer cells.
+// REF: coordinates as floats relative to the chunk's first particle, so that a test
+// costs no integer conversion (16 a clock and SM); grids with at least 2 reach + 3 cells on
+// every axis, where the minimum image relative to that particle is the pair's for all
+// pairs in range.
+constexpr int NLW_WARPS = 4;
+constexpr uint32_t NLW_ROW = 192;   // entries of a row held in shared memory; the rest go to the list at once
+constexpr uint32_t NLW_RANGES = 2 * 9 * 9;  // stencil rows (reach <= 4) and their wrapped parts
+template<bool ONE_TYPE, bool SORTED, bool REF, int CH>
+__global__ void __launch_bounds__(NLW_WARPS * 32)
+    k_nlist_build_warps(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed,
+                        const uint4* __restrict__ words, uint32_t N, BoxArgs bx, CellGrid g,
+                        const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ members,
+                        const uint32_t* __restrict__ cell_of, const ListCut* __restrict__ cuts, uint32_t ntypes,
+                        const uint32_t* __restrict__ ex_n, const uint32_t* __restrict__ ex_keys,
+                        uint32_t* __restrict__ counts, uint32_t* __restrict__ nbrs, uint32_t max_nn,
+                        uint32_t* __restrict__ flags, const uint32_t* __restrict__ gate, const uint4* __restrict__ lo)
+{
+    if (gated_off(gate)) return;
+    __shared__ uint32_t s_rows[NLW_WARPS][CH][NLW_ROW];
+    __shared__ uint2 s_range[NLW_WARPS][NLW_RANGES + 1];  // (first candidate, first slot) of each range
+    __shared__ int s_reach[MAX_LIST_TYPES][3];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ListCut* s_cut = reinterpret_cast<ListCut*>(smem_raw);
+    float* s_hi = reinterpret_cast<float*>(s_cut + ntypes * ntypes);
+    float* s_lo = s_hi + ntypes * ntypes;
+    for (uint32_t t = threadIdx.x; t < ntypes * ntypes; t += blockDim.x) {
+        s_cut[t] = cuts[t];
+        s_hi[t] = cuts[t].hi;
+        s_lo[t] = cuts[t].lo;
+    }
+    for (uint32_t t = threadIdx.x; t < ntypes; t += blockDim.x) {
+        // cells beyond ceil(r / width) lie further than the type's largest list radius
+        double r2 = 0.0;
+        for (uint32_t u = 0; u < ntypes; ++u) r2 = fmax(r2, cuts[t * ntypes + u].rlistsq);
+        const double r = sqrt(r2) * (1.0 + 1e-5);
+        for (int d = 0; d < 3; ++d) s_reach[t][d] = min(g.reach[d], (int)ceil(r * g.scale[d]));
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t(*rows)[NLW_ROW] = s_rows[threadIdx.x >> 5];
+    uint2* range = s_range[threadIdx.x >> 5];
+    const ListCut cut0 = s_cut[0];
+    const int dx = g.dim[0], dy = g.dim[1], dz = g.dim[2];
+    const uint32_t s_begin = (blockIdx.x * NLW_WARPS + (threadIdx.x >> 5)) * CH;
+    const uint32_t s_end = min(s_begin + CH, N);
+    for (uint32_t sa = s_begin; sa < s_end;) {
+        // the slots from sa on that share its cell
+        const uint32_t my_slot = min(sa + lane, s_end - 1u);
+        const uint32_t my_i = SORTED ? my_slot : __ldg(members + my_slot);
+        const uint32_t my_cell = __ldg(cell_of + my_i);
+        const uint4 my_word = __ldg(words + my_slot);
+        const uint32_t cc = __shfl_sync(0xffffffffu, my_cell, 0);
+        const uint32_t same = __ballot_sync(0xffffffffu, my_cell == cc && sa + lane < s_end);
+        const uint32_t cnt = (uint32_t)__ffs(~same) - 1u;  // CH < 32: some lane is off
+        uint32_t pi[CH], n[CH];
+        uint4 pw[CH];
+        float px[CH], py[CH], pz[CH];
+        const uint4 ref = make_uint4(__shfl_sync(0xffffffffu, my_word.x, 0), __shfl_sync(0xffffffffu, my_word.y, 0),
+                                     __shfl_sync(0xffffffffu, my_word.z, 0), 0u);
+        int r0 = 0, r1 = 0, r2 = 0;
+#pragma unroll
+        for (int p = 0; p < CH; ++p) {
+            pi[p] = __shfl_sync(0xffffffffu, my_i, p);
+            pw[p].x = __shfl_sync(0xffffffffu, my_word.x, p);
+            pw[p].y = __shfl_sync(0xffffffffu, my_word.y, p);
+            pw[p].z = __shfl_sync(0xffffffffu, my_word.z, p);
+            pw[p].w = ONE_TYPE ? 0u : __shfl_sync(0xffffffffu, my_word.w, p);
+            n[p] = 0u;
+            px[p] = (float)(int32_t)(pw[p].x - ref.x) * bx.sfix[0];
+            py[p] = (float)(int32_t)(pw[p].y - ref.y) * bx.sfix[1];
+            pz[p] = (float)(int32_t)(pw[p].z - ref.z) * bx.sfix[2];
+            if (p < (int)cnt) {
+                const int* r = s_reach[pw[p].w];
+                r0 = max(r0, r[0]);
+                r1 = max(r1, r[1]);
+                r2 = max(r2, r[2]);
+            }
+            pw[p].w *= ntypes;
+        }
+        const int cx = (int)(cc % (uint32_t)dx);
+        const int cy = (int)((cc / (uint32_t)dx) % (uint32_t)dy);
+        const int cz = (int)(cc / ((uint32_t)dx * (uint32_t)dy));
+        // the x-cells as in k_nlist_build_threads: one range, and the wrapped part
+        int x0 = cx - r0, x1 = cx + r0, wb = 1, we = 0;
+        if (x0 < 0) {
+            wb = dx + x0;
+            we = dx - 1;
+            x0 = 0;
+        }
+        if (x1 >= dx) {
+            wb = 0;
+            we = x1 - dx;
+            x1 = dx - 1;
+        }
+        const bool wrap = wb <= we;
+        const uint32_t parts = wrap ? 2u : 1u;
+        const uint32_t ny = 2u * r1 + 1u;
+        const uint32_t nr = ny * (2u * r2 + 1u) * parts;
+        uint32_t total = 0u;
+        for (uint32_t q0 = 0; q0 < nr; q0 += 32u) {
+            const uint32_t q = q0 + lane;
+            uint32_t sb = 0u, len = 0u;
+            if (q < nr) {
+                const uint32_t row = q / parts, part = q - row * parts;
+                int oz = cz - r2 + (int)(row / ny), oy = cy - r1 + (int)(row % ny);
+                oz += (oz < 0) ? dz : 0;
+                oz -= (oz >= dz) ? dz : 0;
+                oy += (oy < 0) ? dy : 0;
+                oy -= (oy >= dy) ? dy : 0;
+                const uint32_t rb = ((uint32_t)oz * dy + oy) * dx;
+                sb = __ldg(cell_start + rb + (part ? wb : x0));
+                len = __ldg(cell_start + rb + (part ? we : x1) + 1) - sb;
+            }
+            uint32_t sum = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+                if ((int)lane >= o) sum += v;
+            }
+            if (q < nr) range[q] = make_uint2(total + sum - len, sb);
+            total += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0u) range[nr] = make_uint2(0xffffffffu, 0u);
+        __syncwarp();
+        bool band = false;
+        uint32_t q = 0u;
+        // slot of candidate c (rising by 32 a call)
+        const auto slot_of = [&](uint32_t c) -> uint32_t {
+            while (range[q + 1u].x <= c) ++q;
+            const uint2 r = range[q];
+            return r.y + (c - r.x);
+        };
+        uint32_t sl = lane < total ? slot_of(lane) : 0u;
+        uint4 w = __ldg(words + sl);
+        uint32_t j = SORTED ? sl : __ldg(members + sl);
+        for (uint32_t c0 = 0; c0 < total; c0 += 32u) {
+            const bool on = c0 + lane < total;
+            const uint4 wc = w;
+            const uint32_t jc = j;
+            if (c0 + 32u + lane < total) {
+                sl = slot_of(c0 + 32u + lane);
+                w = __ldg(words + sl);
+                j = SORTED ? sl : __ldg(members + sl);
+            }
+            // a lane without a candidate stands outside every radius
+            float qx = 0.0f, qy = 0.0f, qz = on ? 0.0f : INFINITY;
+            if (REF && on) {
+                qx = (float)(int32_t)(wc.x - ref.x) * bx.sfix[0];
+                qy = (float)(int32_t)(wc.y - ref.y) * bx.sfix[1];
+                qz = (float)(int32_t)(wc.z - ref.z) * bx.sfix[2];
+            }
+            const float* hi = s_hi + (ONE_TYPE ? 0u : wc.w);
+            const float* lo_ = s_lo + (ONE_TYPE ? 0u : wc.w);
+#pragma unroll
+            for (int p = 0; p < CH; ++p) {
+                if (p >= (int)cnt) break;
+                float ddx, ddy, ddz;
+                if constexpr (REF) {
+                    ddx = px[p] - qx;
+                    ddy = py[p] - qy;
+                    ddz = pz[p] - qz;
+                } else {
+                    ddx = (float)(int32_t)(pw[p].x - wc.x) * bx.sfix[0];
+                    ddy = (float)(int32_t)(pw[p].y - wc.y) * bx.sfix[1];
+                    ddz = (float)(int32_t)(pw[p].z - wc.z) * bx.sfix[2] - qz;
+                }
+                const float rs = ddx * ddx + ddy * ddy + ddz * ddz;
+                const bool hit = (rs < (ONE_TYPE ? cut0.hi : hi[pw[p].w])) & (jc != pi[p]);
+                const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+                if (hit) {
+                    const uint32_t k = n[p] + __popc(hits & lt);
+                    const bool sure = rs < (ONE_TYPE ? cut0.lo : lo_[pw[p].w]);
+                    const uint32_t e = sure ? jc : (jc | NL_BAND);
+                    band = band || !sure;
+                    if (k < NLW_ROW) rows[p][k] = e;
+                    else if (k < max_nn) nbrs[(size_t)k * N + pi[p]] = e;
+                }
+                n[p] += __popc(hits);
+            }
+        }
+        band = __any_sync(0xffffffffu, band);
+        // compaction, in order, of the rows that may hold what does not belong
+        uint32_t kept[CH], kept_max = 0u;
+#pragma unroll
+        for (int p = 0; p < CH; ++p) {
+            kept[p] = 0u;
+            if (p >= (int)cnt) continue;
+            const uint32_t i = pi[p];
+            // the particle itself counts as listed for the capacity, as in
+            // k_nlist_build_threads, whose scan takes it in
+            const uint32_t raw = n[p] + ((ONE_TYPE ? cut0.hi : s_hi[pw[p].w + pw[p].w / ntypes]) > 0.0f ? 1u : 0u);
+            const uint32_t stored = min(n[p], max_nn);
+            const uint32_t nex = ex_n ? __ldg(ex_n + i) : 0u;
+            uint32_t m = stored;
+            if (band || nex) {
+                m = 0u;
+                for (uint32_t k0 = 0; k0 < stored; k0 += 32u) {
+                    const uint32_t k = k0 + lane;
+                    bool keep = k < stored;
+                    uint32_t e = 0u;
+                    if (keep) {
+                        e = k < NLW_ROW ? rows[p][k] : nbrs[(size_t)k * N + i];
+                        if (e & NL_BAND) {
+                            // the oracle's exact FP64 decision
+                            e &= ~NL_BAND;
+                            const double r2l = ONE_TYPE ? cut0.rlistsq : s_cut[pw[p].w + __ldg(fixed + e).w].rlistsq;
+                            keep = nl_exact_within(i, e, r2l, bx, pos, fixed, lo);
+                        }
+                        for (uint32_t x = 0; x < nex; ++x) keep = keep && __ldg(ex_keys + (size_t)x * N + i) != e;
+                    }
+                    const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+                    if (keep) {
+                        const uint32_t d = m + __popc(mask & lt);
+                        if (d < NLW_ROW) rows[p][d] = e;
+                        else nbrs[(size_t)d * N + i] = e;
+                    }
+                    __syncwarp();
+                    m += __popc(mask);
+                }
+            }
+            kept[p] = min(m, NLW_ROW);
+            kept_max = max(kept_max, kept[p]);
+            if (lane == 0u) {
+                counts[i] = raw > max_nn ? raw : m;
+                if (raw > max_nn) atomicMax(&flags[0], raw);
+            }
+        }
+        __syncwarp();
+        // the chunk's rows side by side: lanes of consecutive particles
+        {
+            constexpr uint32_t STEP = 32u / CH;
+            const uint32_t p = lane % CH, kk = lane / CH;
+            uint32_t i = 0u, m = 0u;
+#pragma unroll
+            for (int u = 0; u < CH; ++u)
+                if (u == (int)p && u < (int)cnt) {
+                    i = pi[u];
+                    m = kept[u];
+                }
+            for (uint32_t k = kk; k < kept_max; k += STEP)
+                if (k < m) nbrs[(size_t)k * N + i] = rows[p][k];
+        }
+        __syncwarp();
+        sa += cnt;
+    }
+}
+
+// the words of the particles in cell order
+__global__ void k_cell_words(const uint4* __restrict__ fixed, const uint32_t* __restrict__ members, uint32_t N,
+                             uint4* __restrict__ words)
+{
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < N) words[s] = fixed[members[s]];
+}
+
+void launch_cell_words(const uint4* fixed, const uint32_t* members, uint32_t N, uint4* words, cudaStream_t s)
+{
+    if (N == 0) return;
+    k_cell_words<<<(N + 255) / 256, 256, 0, s>>>(fixed, members, N, words);
+}
+
+// Whether a grid's list is built a warp per chunk: the candidates of a particle's
+// stencil row must give the warp's lanes work. Particles already in cell order read
+// their candidates side by side a thread per particle as well, so there the line lies
+// higher. Measured (microseconds per build, thread / warp per chunk; candidates per row):
+//   LJ fluid, N = 103,823 (93)       caller's order 1,075 / 333, cell order 637 / 317
+//   colloid mixture, N = 65,537 (28) caller's order 1,554 / 297, cell order 885 / 284
+//   DPD fluid, N = 262,144 (21)      caller's order 561 / 305, cell order 333 / 309;
+//                                    inside the engine 153 / 220
+//   melt, N = 1,048,600 (9)          417 / 822
+bool warp_list_build(uint32_t N, const CellGrid& g, bool sorted)
+{
+    return (double)N / g.ncell * (2 * g.reach[0] + 1) >= (sorted ? 24.0 : 12.0);
+}
+
 // Block records of the shared-memory tiles: for every stencil row of the block's
 // TILE_P particles, the range of particle indices that row's x-ranges cover
 // (cx - 1 .. cx + 1 clipped to the row; the wrapped cell at an x face stays
@@ -539,12 +828,33 @@ void launch_nlist_build(const double4_32a* pos, const uint4* fixed, uint32_t N, 
                         const ListCut* cuts, uint32_t ntypes, const uint32_t* ex_n, const uint32_t* ex_keys,
                         uint32_t ex_width, const uint32_t* keys, uint32_t* counts, uint32_t* nbrs,
                         uint32_t max_nn, uint32_t* flags, const uint32_t* gate, cudaStream_t s, const uint4* lo,
-                        double rlist_min, const uint32_t* tile)
+                        double rlist_min, const uint32_t* tile, const uint4* words)
 {
     (void)ex_width;
     (void)rlist_min;
     if (N == 0) return;
     const BoxArgs bx = box_args(box);
+    if (!keys && !tile && (!members || words) && warp_list_build(N, g, !members)) {
+        bool ref = true;
+        for (int d = 0; d < 3; ++d) ref = ref && g.dim[d] >= 2 * g.reach[d] + 3;
+        const size_t smem = (sizeof(ListCut) + 2 * sizeof(float)) * ntypes * ntypes;
+        // small systems: four particles a warp, for more warps
+        const bool few = N < 40000u;
+        const uint32_t per = NLW_WARPS * (few ? 4u : 8u);
+        const uint32_t nb = (N + per - 1) / per;
+        const auto go = [&](auto kernel) {
+            kernel<<<nb, NLW_WARPS * 32, smem, s>>>(pos, fixed, members ? words : fixed, N, bx, g, cell_start, members,
+                                                    cell_of, cuts, ntypes, ex_n, ex_keys, counts, nbrs, max_nn, flags,
+                                                    gate, lo);
+        };
+#define AZP_NLW(ONE, SORTED)                                                                              \
+    (ref ? (few ? go(k_nlist_build_warps<ONE, SORTED, true, 4>) : go(k_nlist_build_warps<ONE, SORTED, true, 8>)) \
+         : (few ? go(k_nlist_build_warps<ONE, SORTED, false, 4>) : go(k_nlist_build_warps<ONE, SORTED, false, 8>)))
+        if (ntypes == 1) members ? AZP_NLW(true, false) : AZP_NLW(true, true);
+        else members ? AZP_NLW(false, false) : AZP_NLW(false, true);
+#undef AZP_NLW
+        return;
+    }
     const uint32_t blocks = (N + NLIST_BLOCK - 1) / NLIST_BLOCK;
 #define AZP_NL_ARGS                                                                                              \
     pos, fixed, N, bx, g, cell_start, members, cell_of, cuts, ntypes, ex_n, ex_keys, keys, counts, nbrs, max_nn, \
@@ -577,6 +887,7 @@ void free_nl(azp_nlist* nl)
     cudaFree(nl->nbrs);
     cudaFree(nl->cuts);
     cudaFree(nl->fixed);
+    cudaFree(nl->words);
     cudaFree(nl->cell_of);
     cudaFree(nl->slot);
     cudaFree(nl->members);
@@ -632,6 +943,7 @@ azp_nlist* azp_nlist_create(uint32_t N, uint32_t ntypes, uint32_t max_neighbors,
     if (!st && (e = cudaMalloc(&nl->nbrs, sizeof(uint32_t) * n1 * nl->max_nn)) != cudaSuccess) fail(e, "nlist nbrs");
     if (!st && (e = cudaMalloc(&nl->cuts, sizeof(azp::ListCut) * ntypes * ntypes)) != cudaSuccess) fail(e, "cuts");
     if (!st && (e = cudaMalloc(&nl->fixed, sizeof(uint4) * n1)) != cudaSuccess) fail(e, "fixed");
+    if (!st && (e = cudaMalloc(&nl->words, sizeof(uint4) * n1)) != cudaSuccess) fail(e, "words");
     if (!st && (e = cudaMalloc(&nl->cell_of, sizeof(uint32_t) * n1)) != cudaSuccess) fail(e, "cell_of");
     if (!st && (e = cudaMalloc(&nl->slot, sizeof(uint32_t) * n1)) != cudaSuccess) fail(e, "slot");
     if (!st && (e = cudaMalloc(&nl->members, sizeof(uint32_t) * n1)) != cudaSuccess) fail(e, "members");
@@ -726,9 +1038,11 @@ int azp_nlist_build(azp_nlist* nl, const azp_system* sys, void* stream)
         st = azp::exclusive_scan(nl->cell_count, nl->cell_start, g.ncell, nl->scan_tmp, s);
         if (st) return st;
         azp::launch_cell_scatter(nl->cell_of, nl->slot, nl->cell_start, nl->members, N, g.ncell, s);
+        const bool words = azp::warp_list_build(N, g, false);
+        if (words) azp::launch_cell_words(nl->fixed, nl->members, N, nl->words, s);
         azp::launch_nlist_build(pos, nl->fixed, N, sys->box, g, nl->cell_start, nl->members, nl->cell_of, nl->cuts,
                                 nl->ntypes, nl->ex_n, nl->ex_keys, nl->ex_width, nullptr, nl->counts, nl->nbrs,
-                                nl->max_nn, nl->flags, nullptr, s, nullptr, rmin);
+                                nl->max_nn, nl->flags, nullptr, s, nullptr, rmin, nullptr, words ? nl->words : nullptr);
         AZP_CHECK_LAUNCH("azp_nlist_build");
         uint32_t need = 0;
         AZP_CUDA_TRY(cudaMemcpyAsync(&need, nl->flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -16,6 +16,7 @@ struct azp_nlist {
     uint32_t* nbrs = nullptr;
     azp::ListCut* cuts = nullptr;
     uint4* fixed = nullptr;
+    uint4* words = nullptr;  // fixed in cell order (builds a warp per chunk)
     uint32_t* cell_of = nullptr;
     uint32_t* slot = nullptr;
     uint32_t* members = nullptr;
