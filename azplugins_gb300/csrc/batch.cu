@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_b_cell_sort(const uint32_t*
 {
     if (gated_off(gate)) return;
     __shared__ uint32_t s_rows[kSortWarps][kMaxSortedCell];
-    sort_cells_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5]);
+    sort_cells_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5], blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
 }
 
 __global__ void __launch_bounds__(kSortWarps * 32) k_b_cell_sort_crowded(const uint32_t* __restrict__ cell_start,
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_b_cell_sort_crowded(const u
 {
     if (gated_off(gate)) return;
     __shared__ uint32_t s_rows[kSortWarps][kMaxSortedCell];
-    sort_cell_per_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5]);
+    sort_cell_per_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5], blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
 }
 
 struct BPerm {

@@ -79,6 +79,31 @@ CellGrid make_grid(const azp_box& box, double rlist_max, int sub = 1);
 // the ratio of the largest to the smallest list radius, 1 to 3
 int grid_subdivision(double rlist_max, double rlist_min);
 
+// cell of a position
+__device__ __forceinline__ int cell_coord(double x, double lo, double scale, int dim)
+{
+    int c = (int)floor((x - lo) * scale);
+    if (c < 0) c += dim;
+    if (c >= dim) c -= dim;
+    return min(max(c, 0), dim - 1);
+}
+__device__ __forceinline__ uint32_t cell_of_position(const double4_32a& p, const CellGrid& g)
+{
+    const int cx = cell_coord(p.x, g.lo[0], g.scale[0], g.dim[0]);
+    const int cy = cell_coord(p.y, g.lo[1], g.scale[1], g.dim[1]);
+    const int cz = cell_coord(p.z, g.lo[2], g.scale[2], g.dim[2]);
+    return ((uint32_t)cz * g.dim[1] + cy) * g.dim[0] + cx;
+}
+// the same from the high words of a 64-bit fixed position: [-2^31, 2^31) maps
+// linearly onto [0, dim) in integer arithmetic
+__device__ __forceinline__ uint32_t cell_of_fixed(const uint4& f, const CellGrid& g)
+{
+    const uint32_t cx = (uint32_t)(((uint64_t)(f.x ^ 0x80000000u) * (uint32_t)g.dim[0]) >> 32);
+    const uint32_t cy = (uint32_t)(((uint64_t)(f.y ^ 0x80000000u) * (uint32_t)g.dim[1]) >> 32);
+    const uint32_t cz = (uint32_t)(((uint64_t)(f.z ^ 0x80000000u) * (uint32_t)g.dim[2]) >> 32);
+    return (cz * (uint32_t)g.dim[1] + cy) * (uint32_t)g.dim[0] + cx;
+}
+
 // Per type pair thresholds of the list decision (host-built, ntypes^2 entries).
 struct ListCut {
     double rlistsq;  // exact FP64 test: rsq < rlistsq
@@ -184,15 +209,14 @@ void make_list_cuts(const double* r_cut, uint32_t ntypes, double r_buff, const a
 // the fixed-point shadow, for the smallest positive of n cutoffs
 float screen_margin(const double* r_cut, uint32_t n, const azp_box& box);
 
-// The cells of one warp, 32 consecutive cells from (global warp index) * 32: a
+// The cells of one warp, 32 consecutive cells from warp * 32: a
 // lane sorts its own cell when it holds at most kSerialCell members, then the
 // warp sorts the larger ones together, one after another (warp_sort_cell).
-__device__ __forceinline__ void sort_cells_warp(const uint32_t* __restrict__ cell_start,
-                                                uint32_t* __restrict__ members, uint32_t ncell,
-                                                uint32_t* __restrict__ s_row)
+__device__ __forceinline__ void sort_cells_warp(const uint32_t* cell_start, uint32_t* __restrict__ members,
+                                                uint32_t ncell, uint32_t* __restrict__ s_row, uint32_t warp)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t c = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32u + lane;
+    const uint32_t c = warp * 32u + lane;
     uint32_t b = 0u, e = 0u;
     if (c < ncell) {
         b = cell_start[c];
@@ -211,13 +235,11 @@ __device__ __forceinline__ void sort_cells_warp(const uint32_t* __restrict__ cel
 }
 
 // Crowded grids (more than kSerialCell particles per cell on average): one warp
-// per cell, so that the cells are sorted side by side instead of 32 after one
+// per cell (c), so that the cells are sorted side by side instead of 32 after one
 // another in each warp.
-__device__ __forceinline__ void sort_cell_per_warp(const uint32_t* __restrict__ cell_start,
-                                                   uint32_t* __restrict__ members, uint32_t ncell,
-                                                   uint32_t* __restrict__ s_row)
+__device__ __forceinline__ void sort_cell_per_warp(const uint32_t* cell_start, uint32_t* __restrict__ members,
+                                                   uint32_t ncell, uint32_t* __restrict__ s_row, uint32_t c)
 {
-    const uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (c >= ncell) return;  // warp-uniform
     const uint32_t b = cell_start[c], e = cell_start[c + 1];
     if (e - b <= kSerialCell) {

@@ -18,6 +18,7 @@
 #include "celllist.cuh"
 #include "engine.cuh"
 #include "engine_kernels.cuh"
+#include "rebuild_device.cuh"
 #include "scan.cuh"
 
 namespace azp
@@ -35,6 +36,18 @@ int launch_md_step(int pair_kind, int bond_kind, int precision, int integ, const
     }
 }
 
+int launch_md_run(int pair_kind, int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s)
+{
+    switch (pair_kind) {
+    case -1: return launch_run_nopair(bond_kind, precision, integ, r, s);
+    case AZP_PAIR_PERTURBED_LJ: return launch_run_plj(bond_kind, precision, integ, r, s);
+    case AZP_PAIR_EXPANDED_YUKAWA: return launch_run_eyuk(bond_kind, precision, integ, r, s);
+    case AZP_PAIR_HERTZ: return launch_run_hertz(bond_kind, precision, integ, r, s);
+    case AZP_PAIR_COLLOID: return launch_run_colloid(bond_kind, precision, integ, r, s);
+    default: return AZP_ERR_UNSUPPORTED;
+    }
+}
+
 // ---------------------------------------------------------------- rebuild kernels
 __global__ void k_zero_gated(uint32_t* __restrict__ p, uint32_t n, const uint32_t* __restrict__ gate)
 {
@@ -42,45 +55,12 @@ __global__ void k_zero_gated(uint32_t* __restrict__ p, uint32_t n, const uint32_
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = 0u;
 }
 
-struct PermArgs {
-    const uint32_t* members;
-    double4_32a *pos, *t_pos;   // pos NULL in FP32-force mode (the fixed words move instead)
-    uint4 *fix, *t_fix;         // FP32-force mode: high and low fixed words, masses
-    uint4 *lo, *t_lo;
-    double *mass, *t_mass;
-    uint4* fix_build;           // FP32-force mode: receives the new high words too
-    double4_32a *vel, *t_vel;
-    double *accel, *t_accel;
-    int *image, *t_image;
-    uint32_t *tag, *t_tag, *rtag;
-    double *diam, *t_diam;
-    uint32_t *cell_of, *t_cell;
-    uint32_t N;
-};
-
 // temps[s] <- arrays[members[s]]
 __global__ void k_perm_gather(PermArgs a, const uint32_t* __restrict__ gate)
 {
     if (gated_off(gate)) return;
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.N) return;
-    const uint32_t o = a.members[s];
-    if (a.pos) a.t_pos[s] = a.pos[o];
-    if (a.fix) {
-        a.t_fix[s] = a.fix[o];
-        a.t_lo[s] = a.lo[o];
-        a.t_mass[s] = a.mass[o];
-    }
-    a.t_vel[s] = a.vel[o];
-    a.t_accel[3 * s] = a.accel[3 * o];
-    a.t_accel[3 * s + 1] = a.accel[3 * o + 1];
-    a.t_accel[3 * s + 2] = a.accel[3 * o + 2];
-    a.t_image[3 * s] = a.image[3 * o];
-    a.t_image[3 * s + 1] = a.image[3 * o + 1];
-    a.t_image[3 * s + 2] = a.image[3 * o + 2];
-    a.t_tag[s] = a.tag[o];
-    if (a.diam) a.t_diam[s] = a.diam[o];
-    a.t_cell[s] = a.cell_of[o];
+    if (s < a.N) perm_gather(a, s);
 }
 
 // arrays[s] <- temps[s]; rtag[tag[s]] = s
@@ -88,49 +68,17 @@ __global__ void k_perm_back(PermArgs a, const uint32_t* __restrict__ gate)
 {
     if (gated_off(gate)) return;
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.N) return;
-    if (a.pos) a.pos[s] = a.t_pos[s];
-    if (a.fix) {
-        const uint4 f = a.t_fix[s];
-        a.fix[s] = f;
-        a.fix_build[s] = f;
-        a.lo[s] = a.t_lo[s];
-        a.mass[s] = a.t_mass[s];
-    }
-    a.vel[s] = a.t_vel[s];
-    a.accel[3 * s] = a.t_accel[3 * s];
-    a.accel[3 * s + 1] = a.t_accel[3 * s + 1];
-    a.accel[3 * s + 2] = a.t_accel[3 * s + 2];
-    a.image[3 * s] = a.t_image[3 * s];
-    a.image[3 * s + 1] = a.t_image[3 * s + 1];
-    a.image[3 * s + 2] = a.t_image[3 * s + 2];
-    const uint32_t t = a.t_tag[s];
-    a.tag[s] = t;
-    a.rtag[t] = s;
-    if (a.diam) a.diam[s] = a.t_diam[s];
-    a.cell_of[s] = a.t_cell[s];
+    if (s < a.N) a.rtag[perm_back(a, s)] = s;
 }
 
 // per-particle bond table and exclusions in the new index order, from the
 // tag-order master table [k * N + tag]
-__global__ void k_bond_table(const uint32_t* __restrict__ tag, const uint32_t* __restrict__ rtag,
-                             const uint32_t* __restrict__ n_tag, const uint32_t* __restrict__ partner_tag,
-                             const uint32_t* __restrict__ type_tag, uint32_t N, uint32_t* __restrict__ bt_n,
-                             uint2* __restrict__ bt, uint32_t* __restrict__ ex_n, uint32_t* __restrict__ ex_idx,
-                             int exclude, const uint32_t* __restrict__ gate)
+__global__ void k_bond_table(BondTableArgs b, const uint32_t* __restrict__ tag, const uint32_t* __restrict__ rtag,
+                             uint32_t N, const uint32_t* __restrict__ gate)
 {
     if (gated_off(gate)) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const uint32_t t = tag[i];
-    const uint32_t n = n_tag[t];
-    for (uint32_t k = 0; k < n; ++k) {
-        const uint32_t p = rtag[partner_tag[(size_t)k * N + t]];
-        bt[(size_t)k * N + i] = make_uint2(p, type_tag[(size_t)k * N + t]);
-        if (exclude) ex_idx[(size_t)k * N + i] = p;
-    }
-    bt_n[i] = n;
-    if (ex_n) ex_n[i] = exclude ? n : 0u;
+    if (i < N) bond_row(b, rtag, i, tag[i], N);
 }
 
 // The kind of this list build, as two gates for the kernels that differ between
@@ -744,6 +692,8 @@ __global__ void __launch_bounds__(STATE_BLOCK)
 
 using namespace azp;
 
+constexpr uint32_t RUN_SYNC = 32, FLAG_WORDS = 64;
+
 struct azp_md {
     uint32_t N = 0, ntypes = 0, nbt = 0;
     int precision = AZP_FP64, pair_kind = -1, shift_mode = 0, bond_kind = -1, method = 0;
@@ -844,6 +794,7 @@ struct azp_md {
     int* d_img0 = nullptr;
     // control
     uint32_t* flags = nullptr;  // [0] rebuild request [1] error bits [2] builds [3] max count [4] ticket
+                                // from RUN_SYNC, on a line of their own: the persistent run's words
     unsigned long long* d_ts = nullptr;
     uint64_t timestep = 0;
     // outputs
@@ -871,6 +822,8 @@ struct azp_md {
     double* snap_acc = nullptr;
     int* snap_img = nullptr;
     double* snap_diam = nullptr;
+    // whether this engine's steps go as persistent launches (k_md_run)
+    bool run_kernel = false;
     // graphs
     bool use_graphs = true;
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // pair of mid steps starting at cur = 0 / 1
@@ -1044,29 +997,9 @@ MDArgs base_args(azp_md* m)
     return a;
 }
 
-// the list rebuild, gated by flags[0] (gate) or unconditional (gate NULL), with the
-// re-sort of the particles into cell order when due (or forced)
-int enqueue_rebuild(azp_md* m, cudaStream_t s, const uint32_t* gate, bool force_sort)
+PermArgs perm_args(azp_md* m)
 {
-    const uint32_t N = m->N;
-    if (N == 0) return AZP_OK;
-    const uint32_t nb = blocks_for(N, 256);
-    k_zero_gated<<<std::min<uint32_t>(blocks_for(m->grid.ncell, 256), 1024), 256, 0, s>>>(m->cell_count, m->grid.ncell,
-                                                                                          gate);
     const bool fx = m->precision == AZP_FP32;
-    if (fx) launch_cell_assign_fx(m->fix[m->cur], N, m->grid, m->cell_of, m->slot, m->cell_count, s, gate);
-    else launch_cell_assign(m->pos[m->cur], N, m->grid, m->cell_of, m->slot, m->cell_count, s, gate);
-    int st = exclusive_scan(m->cell_count, m->cell_start, m->grid.ncell, m->scan_tmp, s, gate);
-    if (st) return st;
-    launch_cell_scatter(m->cell_of, m->slot, m->cell_start, m->members, N, m->grid.ncell, s, gate);
-    // shared-memory tiles need the cell order at every build
-    const bool sparse = (uint64_t)N <= 4ull * m->grid.ncell && m->grid.reach[0] <= 1 && m->grid.reach[1] <= 1 &&
-                        m->grid.reach[2] <= 1;
-    const uint32_t every = m->sort_every ? m->sort_every : (sparse ? 4u : 1u);
-    const int force = force_sort || every <= 1 || m->tile_tab != nullptr;
-    k_sort_decide<<<1, 1, 0, s>>>(gate, every, force, m->sort_gate);
-    const uint32_t* g_sort = m->sort_gate;
-    const uint32_t* g_keep = m->sort_gate + 2;
     PermArgs p;
     p.members = m->members;
     p.pos = fx ? nullptr : m->pos[m->cur];
@@ -1093,13 +1026,54 @@ int enqueue_rebuild(azp_md* m, cudaStream_t s, const uint32_t* gate, bool force_
     p.t_diam = m->t_diam;
     p.cell_of = m->cell_of;
     p.t_cell = m->t_cell;
-    p.N = N;
+    p.N = m->N;
+    return p;
+}
+
+BondTableArgs bond_table_args(azp_md* m)
+{
+    BondTableArgs b{};
+    if (m->bond_kind >= 0)
+        b = BondTableArgs{m->bt_n_tag, m->bt_partner_tag, m->bt_type_tag, m->bt_n, m->bt, m->ex_n, m->ex_idx,
+                          m->exclude_bonds};
+    return b;
+}
+
+// list builds from one re-sort of the particles to the next; 1: every build
+uint32_t sort_period(const azp_md* m)
+{
+    const bool sparse = (uint64_t)m->N <= 4ull * m->grid.ncell && m->grid.reach[0] <= 1 && m->grid.reach[1] <= 1 &&
+                        m->grid.reach[2] <= 1;
+    return m->sort_every ? m->sort_every : (sparse ? 4u : 1u);
+}
+
+// the list rebuild, gated by flags[0] (gate) or unconditional (gate NULL), with the
+// re-sort of the particles into cell order when due (or forced)
+int enqueue_rebuild(azp_md* m, cudaStream_t s, const uint32_t* gate, bool force_sort)
+{
+    const uint32_t N = m->N;
+    if (N == 0) return AZP_OK;
+    const uint32_t nb = blocks_for(N, 256);
+    k_zero_gated<<<std::min<uint32_t>(blocks_for(m->grid.ncell, 256), 1024), 256, 0, s>>>(m->cell_count, m->grid.ncell,
+                                                                                          gate);
+    const bool fx = m->precision == AZP_FP32;
+    if (fx) launch_cell_assign_fx(m->fix[m->cur], N, m->grid, m->cell_of, m->slot, m->cell_count, s, gate);
+    else launch_cell_assign(m->pos[m->cur], N, m->grid, m->cell_of, m->slot, m->cell_count, s, gate);
+    int st = exclusive_scan(m->cell_count, m->cell_start, m->grid.ncell, m->scan_tmp, s, gate);
+    if (st) return st;
+    launch_cell_scatter(m->cell_of, m->slot, m->cell_start, m->members, N, m->grid.ncell, s, gate);
+    // shared-memory tiles need the cell order at every build
+    const uint32_t every = sort_period(m);
+    const int force = force_sort || every <= 1 || m->tile_tab != nullptr;
+    k_sort_decide<<<1, 1, 0, s>>>(gate, every, force, m->sort_gate);
+    const uint32_t* g_sort = m->sort_gate;
+    const uint32_t* g_keep = m->sort_gate + 2;
+    const PermArgs p = perm_args(m);
     // the re-sorting build: the particles' arrays and the bond table in cell order
     k_perm_gather<<<nb, 256, 0, s>>>(p, g_sort);
     k_perm_back<<<nb, 256, 0, s>>>(p, g_sort);
     if (m->bond_kind >= 0)
-        k_bond_table<<<nb, 256, 0, s>>>(m->tag, m->rtag, m->bt_n_tag, m->bt_partner_tag, m->bt_type_tag, N, m->bt_n,
-                                        m->bt, m->ex_n, m->ex_idx, m->exclude_bonds, g_sort);
+        k_bond_table<<<nb, 256, 0, s>>>(bond_table_args(m), m->tag, m->rtag, N, g_sort);
     if (!fx) launch_to_fixed2(m->pos[m->cur], m->fix[m->cur], m->fix_build, N, m->box, s, gate);
     // the order-keeping build: the new reference positions (the re-sort writes
     // them in FP32-force mode, launch_to_fixed2 in FP64 mode)
@@ -1175,6 +1149,62 @@ int enqueue_step1(azp_md* m, cudaStream_t s)
         m->group_types);
     AZP_CHECK_LAUNCH("k_md_step1");
     m->launches += 1;
+    return AZP_OK;
+}
+
+bool is_capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+// `steps` mid steps as one persistent launch (k_md_run); it leaves no rebuild pending
+constexpr uint64_t RUN_STEPS = 256;  // per launch, so that other streams get their turn
+int enqueue_run(azp_md* m, int integ, uint64_t steps, cudaStream_t s)
+{
+    RunArgs r{};
+    const int cur = m->cur;
+    for (int par = 0; par < 2; ++par) {
+        m->cur = par;
+        r.step[par] = base_args(m);
+        r.step[par].next = 1;
+        RebuildArgs& b = r.rebuild[par];
+        b.perm = perm_args(m);
+        b.bonds = bond_table_args(m);
+        const bool fx = m->precision == AZP_FP32;
+        b.list = ListArgs{fx ? nullptr : m->pos[par], m->fix[par], fx ? m->lo[par] : nullptr, m->N, m->ntypes,
+                          box_args(m->box), m->grid, m->cell_start, m->members, m->cell_of, m->cuts, m->ex_n, m->ex_idx,
+                          nullptr, m->counts, m->nbrs, m->max_nn, m->flags + 3};
+        for (int d = 0; d < 3; ++d) b.Linv[d] = 1.0 / m->box.L[d];
+        b.slot = m->slot;
+        b.cell_count = m->cell_count;
+        b.scan_tmp = m->scan_tmp;
+        b.cell_of = m->cell_of;
+        b.members = m->members;
+        b.cell_start = m->cell_start;
+        b.sort_gate = m->sort_gate;
+        b.sort_every = sort_period(m);
+        b.force_sort = b.sort_every <= 1;
+        b.crowded = crowded_grid(m->N, m->grid.ncell) ? 1 : 0;
+        b.words = m->fix[par ^ 1];
+        b.by_reference = list_by_reference(m->grid) ? 1 : 0;
+        b.has_list = m->pair_kind >= 0;
+    }
+    m->cur = cur;
+    r.blocks = (uint32_t)(((size_t)m->N * m->tpp + RUN_BLOCK - 1) / RUN_BLOCK);
+    r.sync = m->flags + RUN_SYNC;
+    r.request = r.sync + 4;
+    while (steps > 0) {
+        r.steps = (uint32_t)std::min(steps, RUN_STEPS);
+        r.cur = m->cur;
+        const int st = launch_md_run(m->pair_kind, m->bond_kind, m->precision, integ, r, s);
+        if (st) return st;
+        m->launches += 1;
+        m->cur ^= (int)(r.steps & 1u);
+        steps -= r.steps;
+    }
     return AZP_OK;
 }
 
@@ -1333,6 +1363,7 @@ int errors_from_flags(const azp_md* m, const uint32_t* f)
     if (f[3] > m->max_nn) return AZP_ERR_NLIST_OVERFLOW;
     if (f[1] & AZP_EBIT_BOND) return AZP_ERR_BOND;
     if (f[1] & AZP_EBIT_NONFINITE) return AZP_ERR_NONFINITE;
+    if (f[1] & AZP_EBIT_TIMEOUT) return AZP_ERR_TIMEOUT;
     return AZP_OK;
 }
 
@@ -1589,7 +1620,7 @@ azp_md* azp_md_create(const azp_md_config* c, int* status)
     ALLOC(m->slot, N);
     ALLOC(m->members, N);
     ALLOC(m->counts, N);
-    ALLOC(m->flags, 8);
+    ALLOC(m->flags, FLAG_WORDS);
     ALLOC(m->sort_gate, 8);
     CTRY(cudaMemset(m->sort_gate, 0, sizeof(uint32_t) * 8));
     ALLOC(m->d_ts, 1);
@@ -1604,7 +1635,7 @@ azp_md* azp_md_create(const azp_md_config* c, int* status)
     ALLOC(m->d_noise, c->ntypes);
     if (c->pair_kind == AZP_PAIR_DPD_GENERAL_WEIGHT) ALLOC(m->d_dvel, (size_t)4 * N);
     if (m->bond_kind == AZP_BOND_IMAGE_HARMONIC) ALLOC(m->d_img0, (size_t)3 * N);
-    CTRY(cudaMemset(m->flags, 0, sizeof(uint32_t) * 8));
+    CTRY(cudaMemset(m->flags, 0, sizeof(uint32_t) * FLAG_WORDS));
     CTRY(cudaMemcpy(m->d_gamma, m->gamma.data(), sizeof(double) * c->ntypes, cudaMemcpyHostToDevice));
     {
         // noise amplitude per type, with the operations of the reference's
@@ -1782,6 +1813,9 @@ azp_md* azp_md_create(const azp_md_config* c, int* status)
                                       0x1p-18 * (0.5 * L1 + (double)wall_field_extent(wf) + reach_max) + 1e-5);
     }
     CTRY(cudaStreamCreateWithFlags(&m->graph_stream, cudaStreamNonBlocking));
+    const char* env_run = std::getenv("AZP_RUN_KERNEL");
+    m->run_kernel = m->use_graphs && !m->d_dvel && !m->d_img0 && !m->d_wall_f && !m->tile_tab &&
+                    m->grid.ncell <= RUN_MAX_CELLS && !(env_run && env_run[0] == '0');
 #undef ALLOC
 #undef CTRY
     if (status) *status = AZP_OK;
@@ -1836,7 +1870,7 @@ int azp_md_set_state(azp_md* m, const double* pos, const double* vel, const doub
     m->timestep = timestep;
     const unsigned long long ts = timestep;
     AZP_CUDA_TRY(cudaMemcpyAsync(m->d_ts, &ts, sizeof(ts), cudaMemcpyHostToDevice, s));
-    AZP_CUDA_TRY(cudaMemsetAsync(m->flags, 0, sizeof(uint32_t) * 8, s));
+    AZP_CUDA_TRY(cudaMemsetAsync(m->flags, 0, sizeof(uint32_t) * FLAG_WORDS, s));
     int st = AZP_OK;
     bool placed = false;
     uint32_t flags_seen[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -2053,6 +2087,18 @@ int azp_md_run(azp_md* m, uint64_t steps, void* stream)
         st = enqueue_step1(m, s);
         if (st) return st;
     }
+    bool settled = false;  // no rebuild can be pending
+    // (a capture of the stream is refused below, where the graphs are launched)
+    if (m->run_kernel && mid >= 1 && !is_capturing(s)) {
+        st = enqueue_run(m, integ, mid, s);
+        if (st == AZP_ERR_UNSUPPORTED) {  // refused before the first launch
+            m->run_kernel = false;
+        } else {
+            if (st) return st;
+            mid = 0;
+            settled = true;
+        }
+    }
     if (m->use_graphs && mid >= 2) {
         for (int p = 0; p < 2; ++p)
             if (!m->gexec[p]) {
@@ -2076,7 +2122,7 @@ int azp_md_run(azp_md* m, uint64_t steps, void* stream)
         --mid;
     }
     if (integ == MD_INTEG_LANGEVIN) {
-        st = rebuild_if_requested(m, s);
+        if (!settled) st = rebuild_if_requested(m, s);
         if (st) return st;
         st = enqueue_step(m, integ, 0, 1, s, 0, 0);
         if (st) return st;

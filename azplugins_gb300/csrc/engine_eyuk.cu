@@ -8,4 +8,9 @@ int launch_md_eyuk(int bond_kind, int precision, int integ, const MDArgs& a, cud
 {
     return launch_md_pe<ExpandedYukawa>(bond_kind, precision, integ, a, s);
 }
+
+int launch_run_eyuk(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s)
+{
+    return launch_run_pe<ExpandedYukawa>(bond_kind, precision, integ, r, s);
+}
 }  // namespace azp

@@ -8,4 +8,9 @@ int launch_md_hertz(int bond_kind, int precision, int integ, const MDArgs& a, cu
 {
     return launch_md_pe<Hertz>(bond_kind, precision, integ, a, s);
 }
+
+int launch_run_hertz(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s)
+{
+    return launch_run_pe<Hertz>(bond_kind, precision, integ, r, s);
+}
 }  // namespace azp

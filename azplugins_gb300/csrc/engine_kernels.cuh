@@ -9,12 +9,16 @@
 // integrate.cu) and through them the reference lines cited there.
 #pragma once
 
+#include <algorithm>
+
 #include "barrier.cuh"
 #include "celllist.cuh"
 #include "engine.cuh"
+#include "nlist_device.cuh"
 #include "philox.cuh"
 #include "evaluators.cuh"
 #include "pair.cuh"
+#include "rebuild_device.cuh"
 
 namespace azp
 {
@@ -296,14 +300,9 @@ AZP_D bool displaced(const uint4& f, const uint4& fb, const float* sfix, float t
 }
 
 // ---------------------------------------------------------------- DPD in the step
-// The timestep whose forces a step evaluates (the DPD draw's timestep): a
-// Langevin step at t evaluates t + 1 (HOOMD computes the net force of t + 1
-// between the halves), a forces-only launch its own timestep.
-template<int INTEG> AZP_D unsigned long long force_timestep(const MDArgs& a)
-{
-    return *a.d_timestep + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull);
-}
-
+// The timestep whose forces a step at ts evaluates (the DPD draw's timestep): a
+// Langevin step evaluates ts + 1 (HOOMD computes the net force of ts + 1 between the
+// halves), a forces-only launch its own timestep.
 // alpha in (-1, 1) of the pair (tags ti, tj): the first 64-bit word of the
 // pair's Philox block, stream (AZP_RNG_DPD_GENERAL_WEIGHT, timestep, seed),
 // counter {0, min tag, max tag, 0}, as azp_dpd_forces draws it
@@ -400,10 +399,12 @@ static __device__ __noinline__ double2 adjusted_fp64(const MDArgs& a, const doub
 constexpr uint32_t MD_QUEUE = 16;  // queued candidates per lane of a particle
 constexpr int MD_SCAN = 4;         // list entries a lane scans per pass
 
-template<class PE, class BE, int INTEG, bool OUT>
-__global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
+// The body for the block-th MD_BLOCK / tpp particles at timestep ts; whether the calling
+// thread's particle asks for a list rebuild. smem_raw: md_step_smem bytes. NC: loads of
+// the particle arrays through the read-only path (nothing in the launch writes them).
+template<class PE, class BE, int INTEG, bool OUT, bool NC>
+AZP_D bool md_step_body(const MDArgs& a, uint32_t block, unsigned long long ts, unsigned char* smem_raw)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr bool PAIR = !std::is_same<PE, NoPair>::value;
     constexpr bool DPD = std::is_same<PE, DpdEngine>::value;
     const uint32_t nt2 = a.ntypes * a.ntypes;
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
 
     const double half0 = 0.5 * a.L[0], half1 = 0.5 * a.L[1], half2 = 0.5 * a.L[2];
     Acc64<OUT> acc;
-    uint32_t i = blockIdx.x * P + (threadIdx.x >> a.tpp_shift);
+    uint32_t i = block * P + (threadIdx.x >> a.tpp_shift);
     bool active = i < a.N;
     double4_32a pi = make_double4_32a(0.0, 0.0, 0.0, 0.0);
     if (active) pi = a.pos[i];
@@ -448,16 +449,16 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
         // a row of 16 entries per lane and one of padding, against bank conflicts
         uint32_t* queue = reinterpret_cast<uint32_t*>(s_screen + nt2) + (threadIdx.x & ~(tpp - 1u)) * (MD_QUEUE + 1u);
         const uint32_t full = tpp * (MD_QUEUE - MD_SCAN);
-        const uint32_t n = active ? min(__ldg(a.counts + i), a.max_nn) : 0u;
+        const uint32_t n = active ? min(ld_ro<NC>(a.counts + i), a.max_nn) : 0u;
         const uint32_t nmax = __reduce_max_sync(0xffffffffu, n);
         const uint32_t row = type_of(pi.w) * a.ntypes;
         uint4 fi = make_uint4(0u, 0u, 0u, 0u);
         uint32_t k0 = 0, k1 = 0, tgi = 0;
         double4_32a vi{};
         if (active) {
-            fi = __ldg(a.fix + i);
+            fi = ld_ro<NC>(a.fix + i);
             if constexpr (DPD) {
-                dpd_key(a, force_timestep<INTEG>(a), k0, k1);
+                dpd_key(a, ts + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), k0, k1);
                 tgi = a.tag[i];
                 vi = reinterpret_cast<const double4_32a*>(a.dvel)[i];
             }
@@ -470,10 +471,10 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
 #pragma unroll
             for (int u = 0; u < MD_SCAN; ++u) {
                 const uint32_t k = kb + sub + u * tpp;
-                jj[u] = k < n ? __ldg(col + (size_t)k * a.N) : 0xffffffffu;
+                jj[u] = k < n ? ld_ro<NC>(col + (size_t)k * a.N) : 0xffffffffu;
             }
 #pragma unroll
-            for (int u = 0; u < MD_SCAN; ++u) fj[u] = __ldg(a.fix + (jj[u] != 0xffffffffu ? jj[u] : 0u));
+            for (int u = 0; u < MD_SCAN; ++u) fj[u] = ld_ro<NC>(a.fix + (jj[u] != 0xffffffffu ? jj[u] : 0u));
 #pragma unroll
             for (int u = 0; u < MD_SCAN; ++u) {
                 const float dx = (float)(int32_t)(fi.x - fj[u].x) * a.sfix[0];
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
     }
     if (tpp > 1u) {
         // one thread per particle from here on: the block's first P
-        i = blockIdx.x * P + threadIdx.x;
+        i = block * P + threadIdx.x;
         active = threadIdx.x < P && i < a.N;
         if constexpr (PAIR) {
             __syncthreads();
@@ -537,9 +538,9 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
     if (active) {
         // ---------------------------------------------------------------- bonds
         if constexpr (!std::is_same<BE, NoBond>::value) {
-            const uint32_t nb = __ldg(a.bt_n + i);
+            const uint32_t nb = ld_ro<NC>(a.bt_n + i);
             for (uint32_t k = 0; k < nb; ++k) {
-                const uint2 e2 = __ldg(a.bt + (size_t)k * a.N + i);
+                const uint2 e2 = ld_ro<NC>(a.bt + (size_t)k * a.N + i);
                 const double4_32a pj = a.pos[e2.x];
                 double dx, dy, dz;
                 if constexpr (bond_uses_image<BE>::value) {
@@ -572,7 +573,7 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
         if (a.bar_geom >= 0) {
             // the barrier's force joins the net force (src/HarmonicBarrier.h:149-180)
             double fb[3] = {0.0, 0.0, 0.0};
-            barrier_fp64(a, pi, *a.d_timestep + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), fb, Ub);
+            barrier_fp64(a, pi, ts + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), fb, Ub);
             Fx += fb[0];
             Fy += fb[1];
             Fz += fb[2];
@@ -601,7 +602,6 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
             for (int c = 0; c < 6; ++c) a.out_virial[(size_t)c * a.N + i] = wv[c];
         }
         if constexpr (INTEG != MD_FORCES_ONLY) {
-            const unsigned long long ts = *a.d_timestep;
             double4_32a p = pi;
             const uint32_t ti = type_of(p.w);
             const uint32_t tg = a.tag[i];
@@ -692,7 +692,25 @@ __global__ void __launch_bounds__(MD_BLOCK) k_md_step(MDArgs a)
             }
         }
     }
-    if constexpr (INTEG != MD_FORCES_ONLY) finish_step(a, want_rebuild);
+    return want_rebuild;
+}
+
+template<class PE, class BE, int INTEG, bool OUT>
+__global__ void __launch_bounds__(MD_BLOCK) k_md_step(const __grid_constant__ MDArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const bool want = md_step_body<PE, BE, INTEG, OUT, true>(a, blockIdx.x, *a.d_timestep, smem_raw);
+    if constexpr (INTEG != MD_FORCES_ONLY) finish_step(a, want);
+}
+
+// dynamic shared memory of k_md_step
+template<class PE> inline size_t md_step_smem(const MDArgs& a)
+{
+    const size_t nt2 = (size_t)a.ntypes * a.ntypes;
+    return 2 * a.ntypes * sizeof(double) + nt2 * REC64 * sizeof(double) +
+           (size_t)a.nbondtypes * BOND_REC * sizeof(double) + nt2 * sizeof(float) +
+           (a.tpp > 1 ? (size_t)(MD_BLOCK / a.tpp) * (a.out ? 10 : 3) * sizeof(double) : 0) +
+           (std::is_same<PE, NoPair>::value ? 0 : MD_BLOCK * (MD_QUEUE + 1) * sizeof(uint32_t));
 }
 
 // ---------------------------------------------------------------- FP32-force step
@@ -782,11 +800,11 @@ AZP_D long long fx_rsq_rounded(const uint4& fi, const uint4& li, const uint4& fj
                     iz = axis(fi.z, li.z, fj.z, lj.z);
     return ix * ix + iy * iy + iz * iz;
 }
-template<class PE>
+template<class PE, bool NC>
 AZP_D void gap_args(const MDArgs& a, const uint4& fi, const uint4& fj, uint32_t i, uint32_t j, uint32_t tp,
                     float& rsq, float& dq)
 {
-    const uint4 li = __ldg(a.flo + i), lj = __ldg(a.flo + j);
+    const uint4 li = ld_ro<NC>(a.flo + i), lj = ld_ro<NC>(a.flo + j);
 #if AZP_COLLOID_GAP == 2
     if (a.contact_q) {
         const long long q = fx_rsq_rounded(fi, li, fj, lj);
@@ -807,7 +825,7 @@ AZP_D void gap_args(const MDArgs& a, const uint4& fi, const uint4& fj, uint32_t 
 
 // ONE: a single-type system; the type pair is 0 at compile time, so the record
 // lookups resolve to the caller's registers
-template<class PE, bool ONE = false>
+template<class PE, bool ONE, bool NC>
 AZP_D void pair_term_fx(const MDArgs& a, const uint4& fi, const uint4& fj, uint32_t i, uint32_t j,
                         const float* s_rec, const double* s_rc2, AccFx& acc, bool vir)
 {
@@ -827,7 +845,7 @@ AZP_D void pair_term_fx(const MDArgs& a, const uint4& fi, const uint4& fj, uint3
             // the cancelling contact difference (colloid point-sphere and
             // sphere-sphere forms) formed exactly
             float rg, dq;
-            gap_args<PE>(a, fi, fj, i, j, tp, rg, dq);
+            gap_args<PE, NC>(a, fi, fj, i, j, tp, rg, dq);
             PE::eval_gap(rec, rg, dq, fdr, e);
         } else {
             PE::eval(rec, rsq, fdr, e);
@@ -845,7 +863,7 @@ AZP_D void pair_term_fx(const MDArgs& a, const uint4& fi, const uint4& fj, uint3
 // outside r_cut: the evaluator runs on every lane (at r_cut where the pair does
 // not count) and the pair's terms are masked, so a batch has no per-lane exits;
 // only the rare candidate in the band around r_cut takes the exact FP64 branch
-template<class PE, bool TILE = false, bool ONE = false>
+template<class PE, bool TILE, bool ONE, bool NC>
 AZP_D void pair_term_fx_masked(const MDArgs& a, const uint4& fi, const uint4& fj, uint32_t i, uint32_t ent, bool ok,
                                const float* s_rec, const double* s_rc2, AccFx& acc, bool vir,
                                const uint32_t* trec = nullptr)
@@ -876,7 +894,7 @@ AZP_D void pair_term_fx_masked(const MDArgs& a, const uint4& fi, const uint4& fj
         float rg = rs, dq = 0.0f;
         if (PE::gap_form(rec)) {
             dq = PE::contact2_f(rec) - rs;
-            if (in) gap_args<PE>(a, fi, fj, i, jof(), tp, rg, dq);
+            if (in) gap_args<PE, NC>(a, fi, fj, i, jof(), tp, rg, dq);
         }
         PE::eval_any(rec, rg, dq, fdr, e);
     } else {
@@ -920,7 +938,7 @@ static __device__ __noinline__ bool dpd_near_cutoff_fp64(const MDArgs& a, const 
 // FP64 from the full 64-bit positions within 0.2 % of r_cut^2 (the weight
 // (1 - r / r_cut)^(s/2) is steep there, and the cutoff decision is the oracle's);
 // velocities and tag from the step's snapshot (float4: v, tag bits)
-template<bool ONE = false>
+template<bool ONE, bool NC>
 AZP_D void pair_term_dpd_fx(const MDArgs& a, const uint4& fi, const uint4& fj, uint32_t i, uint32_t j,
                             const float* s_rec, const double* s_rc2, AccFx& acc, bool vir, const float4& vi,
                             uint32_t tgi, uint32_t k0, uint32_t k1)
@@ -933,7 +951,7 @@ AZP_D void pair_term_dpd_fx(const MDArgs& a, const uint4& fi, const uint4& fj, u
     const float* rec = s_rec + (size_t)tp * PAIR_TBL;
     const float rc2 = rec[PAIR_REC];
     if (!(rc2 > 0.0f) || rs >= rc2 * 1.000004f) return;
-    const float4 vj = __ldg(reinterpret_cast<const float4*>(a.dvel) + j);
+    const float4 vj = ld_ro<NC>(reinterpret_cast<const float4*>(a.dvel) + j);
     const uint32_t tgj = __float_as_uint(vj.w);
     if (rs >= rc2 * 0.998f && a.contact_q) {
         // within 0.2 % of r_cut^2 in a cubic box: the cutoff decided and 1 - r / r_cut
@@ -1009,16 +1027,16 @@ AZP_D float unwrapped_fx(uint32_t hi_i, uint32_t lo_i, uint32_t hi_j, uint32_t l
 
 // one ImageHarmonic bond of particle i (fixed words fi / li, images g[3] of the
 // step's start) with partner j in the FP32-force step
-template<class BE, bool ONE = false>
+template<class BE, bool ONE, bool NC>
 AZP_D void bond_term_fx_image(const MDArgs& a, const uint4& fi, const uint4& li, const int* g, uint32_t j,
                               uint32_t btype, const float* s_bond, AccFx& acc, bool vir)
 {
-    const uint4 fj = __ldg(a.fix + j);
-    const uint4 lj = __ldg(a.flo + j);
+    const uint4 fj = ld_ro<NC>(a.fix + j);
+    const uint4 lj = ld_ro<NC>(a.flo + j);
     const int* gj = a.img0 + 3 * (size_t)j;
-    const float dx = unwrapped_fx(fi.x, li.x, fj.x, lj.x, g[0] - __ldg(gj), a.sfix[0]);
-    const float dy = unwrapped_fx(fi.y, li.y, fj.y, lj.y, g[1] - __ldg(gj + 1), a.sfix[1]);
-    const float dz = unwrapped_fx(fi.z, li.z, fj.z, lj.z, g[2] - __ldg(gj + 2), a.sfix[2]);
+    const float dx = unwrapped_fx(fi.x, li.x, fj.x, lj.x, g[0] - ld_ro<NC>(gj), a.sfix[0]);
+    const float dy = unwrapped_fx(fi.y, li.y, fj.y, lj.y, g[1] - ld_ro<NC>(gj + 1), a.sfix[1]);
+    const float dz = unwrapped_fx(fi.z, li.z, fj.z, lj.z, g[2] - ld_ro<NC>(gj + 2), a.sfix[2]);
     const float rsq = dx * dx + dy * dy + dz * dz;
     float fdr, en;
     if (!BE::eval_f(s_bond + (ONE ? 0u : btype) * BOND_F, rsq, fdr, en)) {
@@ -1152,10 +1170,11 @@ AZP_D void prefetch_warp_rows(const MDArgs& a, uint32_t i0, uint32_t i_last, uin
 // TILE (single-type systems, TILE_P particles per block, one thread each): the
 // block's neighbour ranges are staged in shared memory first and the list
 // entries address them there (celllist.cuh, TILE_GLOBAL entries are gathered)
-template<class PE, class BE, int INTEG, bool OUT, bool ONE, bool TILE = false>
-__global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_md_step_fx(MDArgs a)
+// The body for the block-th FX_BLOCK / tpp particles at timestep ts; whether the calling
+// thread's particle asks for a list rebuild (NC as in md_step_body)
+template<class PE, class BE, int INTEG, bool OUT, bool ONE, bool TILE, bool NC>
+AZP_D bool md_step_fx_body(const MDArgs& a, uint32_t block, unsigned long long ts, unsigned char* smem_raw)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t nt2 = a.ntypes * a.ntypes;
     double* s_rc2 = reinterpret_cast<double*>(smem_raw);
     float* s_rec = reinterpret_cast<float*>(s_rc2 + nt2);
@@ -1184,12 +1203,12 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
         s_noise = &one_noise;
         if constexpr (TILE) {
             // stage the block's neighbour ranges: coalesced 16-byte copies
-            trec = a.tile + (size_t)blockIdx.x * TILE_REC;
-            const uint32_t nr = __ldg(trec);
+            trec = a.tile + (size_t)block * TILE_REC;
+            const uint32_t nr = ld_ro<NC>(trec);
             uint4* st = reinterpret_cast<uint4*>(smem_raw);
             for (uint32_t k = 0; k < nr; ++k) {
-                const uint32_t b = __ldg(trec + 2 + 3 * k), e = __ldg(trec + 3 + 3 * k), off = __ldg(trec + 4 + 3 * k);
-                for (uint32_t q = threadIdx.x; q < e - b; q += blockDim.x) st[off + q] = __ldg(a.fix + b + q);
+                const uint32_t b = ld_ro<NC>(trec + 2 + 3 * k), e = ld_ro<NC>(trec + 3 + 3 * k), off = ld_ro<NC>(trec + 4 + 3 * k);
+                for (uint32_t q = threadIdx.x; q < e - b; q += blockDim.x) st[off + q] = ld_ro<NC>(a.fix + b + q);
             }
             __syncthreads();
         }
@@ -1211,7 +1230,7 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
     }
 
     const uint32_t tpp = (uint32_t)a.tpp;
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t gid = block * blockDim.x + threadIdx.x;
     const uint32_t i = gid >> a.tpp_shift;
     const uint32_t sub = gid & (tpp - 1u);
     const bool active = i < a.N;
@@ -1235,19 +1254,20 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
             }
             cp_async16(&st_lo[threadIdx.x], a.flo + i);
             cp_async16(&st_fb[threadIdx.x], a.fix_build + i);
-            cp_async4(&st_tag[threadIdx.x], a.tag + i);
+            if constexpr (NC) cp_async4(&st_tag[threadIdx.x], a.tag + i);
+            else st_tag[threadIdx.x] = a.tag[i];  // (a 4-byte cp.async goes through L1 lines of earlier steps)
             cp_async_commit();
         }
     }
     AccFx acc;
     uint4 fi = make_uint4(0u, 0u, 0u, 0u);
     uint32_t n = 0u;
-    if constexpr (!std::is_same<PE, NoPair>::value) n = active ? min(__ldg(a.counts + i), a.max_nn) : 0u;
+    if constexpr (!std::is_same<PE, NoPair>::value) n = active ? min(ld_ro<NC>(a.counts + i), a.max_nn) : 0u;
     // the warp's longest list row
     const uint32_t nmax = __reduce_max_sync(0xffffffffu, n);
 #if AZP_FX_PREFETCH
     {
-        const uint32_t i0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> a.tpp_shift;
+        const uint32_t i0 = (block * blockDim.x + (threadIdx.x & ~31u)) >> a.tpp_shift;
         if (i0 < a.N) {
             const uint32_t i_last = min(i0 + (32u >> a.tpp_shift) - 1u, a.N - 1u);
             prefetch_warp_rows(a, i0, i_last, std::is_same<PE, NoPair>::value ? 0u : nmax,
@@ -1255,7 +1275,7 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
         }
     }
 #endif
-    if (active) fi = __ldg(a.fix + i);
+    if (active) fi = ld_ro<NC>(a.fix + i);
     // -------------------------------------------------------------------- DPD pairs
     if constexpr (std::is_same<PE, DpdEngine>::value) {
         // Two phases, as the FP64 step: the scan queues the partners inside
@@ -1267,9 +1287,9 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
         const uint32_t* col = a.nbrs + i;
         uint32_t k0 = 0, k1 = 0, tgi = 0;
         float4 vi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        dpd_key(a, force_timestep<INTEG>(a), k0, k1);
+        dpd_key(a, ts + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), k0, k1);
         if (active) {
-            vi = __ldg(reinterpret_cast<const float4*>(a.dvel) + i);
+            vi = ld_ro<NC>(reinterpret_cast<const float4*>(a.dvel) + i);
             tgi = __float_as_uint(vi.w);
         }
         uint32_t nq = 0;
@@ -1278,9 +1298,9 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
             uint4 fj[FX_BATCH];
             const uint32_t k = kb + sub * FX_BATCH;
 #pragma unroll
-            for (int u = 0; u < FX_BATCH; ++u) jj[u] = k + u < n ? __ldg(col + (size_t)(k + u) * a.N) : 0u;
+            for (int u = 0; u < FX_BATCH; ++u) jj[u] = k + u < n ? ld_ro<NC>(col + (size_t)(k + u) * a.N) : 0u;
 #pragma unroll
-            for (int u = 0; u < FX_BATCH; ++u) fj[u] = __ldg(a.fix + jj[u]);
+            for (int u = 0; u < FX_BATCH; ++u) fj[u] = ld_ro<NC>(a.fix + jj[u]);
             uint32_t mark = 0x80000000u;
 #pragma unroll
             for (int u = 0; u < FX_BATCH; ++u) {
@@ -1298,7 +1318,7 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
                 const uint32_t e = queue[FX_BLOCK * m];
                 if (e & 0x80000000u) acc.commit(vir);
                 const uint32_t j = e & 0x7fffffffu;
-                pair_term_dpd_fx<ONE>(a, fi, __ldg(a.fix + j), i, j, s_rec, s_rc2, acc, vir, vi, tgi, k0, k1);
+                pair_term_dpd_fx<ONE, NC>(a, fi, ld_ro<NC>(a.fix + j), i, j, s_rec, s_rc2, acc, vir, vi, tgi, k0, k1);
             }
             nq = 0;
         }
@@ -1322,7 +1342,7 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
 #pragma unroll
             for (int u = 0; u < FX_BATCH; ++u) {
                 const uint32_t k = sub * FX_BATCH + u;
-                jn[u] = k < n ? __ldg(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
+                jn[u] = k < n ? ld_ro<NC>(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
             }
 #endif
             // a lane's batch is FX_BATCH consecutive entries, so that the batch sums (and
@@ -1337,32 +1357,32 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
 #pragma unroll
                 for (int u = 0; u < FX_BATCH; ++u) {
                     const uint32_t k = kb + u;
-                    jj[u] = k < n ? __ldg(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
+                    jj[u] = k < n ? ld_ro<NC>(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
                 }
 #endif
                 if constexpr (TILE) {
 #pragma unroll
                     for (int u = 0; u < FX_BATCH; ++u)
-                        fj[u] = (jj[u] & TILE_GLOBAL) ? __ldg(a.fix + (jj[u] & ~TILE_GLOBAL)) : s_tile[jj[u]];
+                        fj[u] = (jj[u] & TILE_GLOBAL) ? ld_ro<NC>(a.fix + (jj[u] & ~TILE_GLOBAL)) : s_tile[jj[u]];
                 } else {
 #pragma unroll
-                    for (int u = 0; u < FX_BATCH; ++u) fj[u] = __ldg(a.fix + jj[u]);
+                    for (int u = 0; u < FX_BATCH; ++u) fj[u] = ld_ro<NC>(a.fix + jj[u]);
                 }
 #if AZP_FX_PIPE
 #pragma unroll
                 for (int u = 0; u < FX_BATCH; ++u) {
                     const uint32_t k = kb + FX_BATCH * tpp + u;
-                    jn[u] = k < n ? __ldg(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
+                    jn[u] = k < n ? ld_ro<NC>(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
                 }
 #endif
 #pragma unroll
                 for (int u = 0; u < FX_BATCH; ++u) {
                     {
 #if AZP_FX_UNIFORM
-                        pair_term_fx_masked<PE, TILE, ONE>(a, fi, fj[u], i, jj[u], kb + u < n, s_rec, s_rc2,
+                        pair_term_fx_masked<PE, TILE, ONE, NC>(a, fi, fj[u], i, jj[u], kb + u < n, s_rec, s_rc2,
                                                            acc, vir, trec);
 #else
-                        if (kb + u < n) pair_term_fx<PE, ONE>(a, fi, fj[u], i, jj[u], s_rec, s_rc2, acc, vir);
+                        if (kb + u < n) pair_term_fx<PE, ONE, NC>(a, fi, fj[u], i, jj[u], s_rec, s_rc2, acc, vir);
 #endif
                     }
                 }
@@ -1371,23 +1391,23 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
         }
         // ---------------------------------------------------------------- bonds
         if constexpr (bond_uses_image<BE>::value) {
-            const uint32_t nb = __ldg(a.bt_n + i);
-            const uint4 li = __ldg(a.flo + i);
-            const int g[3] = {__ldg(a.img0 + 3 * (size_t)i), __ldg(a.img0 + 3 * (size_t)i + 1),
-                              __ldg(a.img0 + 3 * (size_t)i + 2)};
+            const uint32_t nb = ld_ro<NC>(a.bt_n + i);
+            const uint4 li = ld_ro<NC>(a.flo + i);
+            const int g[3] = {ld_ro<NC>(a.img0 + 3 * (size_t)i), ld_ro<NC>(a.img0 + 3 * (size_t)i + 1),
+                              ld_ro<NC>(a.img0 + 3 * (size_t)i + 2)};
             for (uint32_t k = sub; k < nb; k += tpp) {
-                const uint2 e = __ldg(a.bt + (size_t)k * a.N + i);
-                bond_term_fx_image<BE, ONE>(a, fi, li, g, e.x, e.y, s_bond, acc, vir);
+                const uint2 e = ld_ro<NC>(a.bt + (size_t)k * a.N + i);
+                bond_term_fx_image<BE, ONE, NC>(a, fi, li, g, e.x, e.y, s_bond, acc, vir);
                 acc.commit(vir);
             }
         } else if constexpr (!std::is_same<BE, NoBond>::value) {
-            const uint32_t nb = __ldg(a.bt_n + i);
+            const uint32_t nb = ld_ro<NC>(a.bt_n + i);
             for (uint32_t k0 = 2u * sub; k0 < nb; k0 += 2u * tpp) {
                 const uint32_t k1 = k0 + 1u;
-                const uint2 e0 = __ldg(a.bt + (size_t)k0 * a.N + i);
-                const uint2 e1 = k1 < nb ? __ldg(a.bt + (size_t)k1 * a.N + i) : make_uint2(i, 0u);
-                const uint4 f0 = __ldg(a.fix + e0.x);
-                const uint4 f1 = __ldg(a.fix + e1.x);
+                const uint2 e0 = ld_ro<NC>(a.bt + (size_t)k0 * a.N + i);
+                const uint2 e1 = k1 < nb ? ld_ro<NC>(a.bt + (size_t)k1 * a.N + i) : make_uint2(i, 0u);
+                const uint4 f0 = ld_ro<NC>(a.fix + e0.x);
+                const uint4 f1 = ld_ro<NC>(a.fix + e1.x);
                 bond_term_fx<BE, ONE>(a, fi, f0, e0.y, s_bond, acc, vir);
                 if (k1 < nb) bond_term_fx<BE, ONE>(a, fi, f1, e1.y, s_bond, acc, vir);
                 acc.commit(vir);
@@ -1401,7 +1421,7 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
         float fb[3] = {0.0f, 0.0f, 0.0f}, ub = 0.0f;
         if (a.bar_geom >= 0)
             // the barrier's force joins the net force (src/HarmonicBarrier.h:149-180)
-            barrier_fx(a, fi, *a.d_timestep + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), fb, ub);
+            barrier_fx(a, fi, ts + (INTEG == MD_INTEG_LANGEVIN ? 1ull : 0ull), fb, ub);
         // the walls' force and energy (k_walls_fx, launched right before the step)
         const float4 fw = a.wall_kind >= 0 ? a.wall_f[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if constexpr (OUT) {
@@ -1424,9 +1444,8 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
         }
         if constexpr (INTEG != MD_FORCES_ONLY) {
             if constexpr (STAGE) cp_async_wait_all();
-            const unsigned long long ts = *a.d_timestep;
             const uint32_t ti = fi.w;
-            const uint32_t tg = STAGE ? st_tag[threadIdx.x] : __ldg(a.tag + i);
+            const uint32_t tg = STAGE ? st_tag[threadIdx.x] : ld_ro<NC>(a.tag + i);
             const float fx = acc.fx.s + (acc.fx.c + (fb[0] + fw.x));
             const float fy = acc.fy.s + (acc.fy.c + (fb[1] + fw.y));
             const float fz = acc.fz.s + (acc.fz.c + (fb[2] + fw.z));
@@ -1508,7 +1527,154 @@ __global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_m
             }
         }
     }
-    if constexpr (INTEG != MD_FORCES_ONLY) finish_step(a, want_rebuild);
+    return want_rebuild;
+}
+
+template<class PE, class BE, int INTEG, bool OUT, bool ONE, bool TILE = false>
+__global__ void __launch_bounds__(FX_BLOCK, (fx_min_blocks<PE, OUT, ONE>())) k_md_step_fx(const __grid_constant__ MDArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const bool want = md_step_fx_body<PE, BE, INTEG, OUT, ONE, TILE, true>(a, blockIdx.x, *a.d_timestep, smem_raw);
+    if constexpr (INTEG != MD_FORCES_ONLY) finish_step(a, want);
+}
+
+// dynamic shared memory of k_md_step_fx (without tiles)
+inline size_t md_step_fx_smem(const MDArgs& a)
+{
+    const size_t nt2 = (size_t)a.ntypes * a.ntypes;
+    return nt2 * sizeof(double) + nt2 * PAIR_TBL * sizeof(float) + (size_t)a.nbondtypes * BOND_F * sizeof(float) +
+           2 * a.ntypes * sizeof(float);
+}
+
+// ---------------------------------------------------------------- persistent run
+// r.steps timesteps in one cooperative launch: each step is the body of the step kernels
+// over the launch's blocks, then a grid barrier, then the rebuild when a particle asked
+// for one. Launched kernel by kernel, a step of a small system waits longer for the graph's
+// conditional node and launches (8 to 10 us) than it computes; here it waits for one
+// barrier. The particle arrays change within the launch, so the bodies load them with
+// plain loads (NC false), which the barriers' fences order.
+// Bound: in a step, as the step kernels, until the step is shorter than the barrier and
+// the load latencies of its chain (6.4 us at 216 particles); in a rebuild, the seven
+// barriers and the chain list -> cell -> particles of each phase. Microseconds per step with
+// the rebuilds, graph and this kernel: FP32 LJ fluid 28.5 and 18.6 at 1,000 particles,
+// 30.5 and 21.6 at 4,096, 72.0 and 63.7 at 54,872; FP32 melt 31.3 and 16.9 at 10,000;
+// FP64 fluid 52.8 and 42.3 at 4,096. Three FP32 blocks per SM: with two, steps past 304
+// blocks go in two turns; with four, 64 registers spill and the 54,872 take 75.2.
+// The request of step s goes to word s mod 3, so that a block that is already in the next
+// step cannot change what a slower one still reads; the word after next is cleared.
+template<class PE, class BE, int INTEG, bool FX, bool ONE>
+__global__ void __launch_bounds__(RUN_BLOCK, FX ? 3 : 2) k_md_run(const __grid_constant__ RunArgs r)
+{
+    static_assert(FX_BLOCK == RUN_BLOCK && MD_BLOCK == RUN_BLOCK, "one block size");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ uint32_t s_word;
+    const uint32_t tid = blockIdx.x * RUN_BLOCK + threadIdx.x, nth = gridDim.x * RUN_BLOCK;
+    uint32_t* flags = r.step[0].flags;
+    const unsigned long long ts0 = *r.step[0].d_timestep;
+    uint32_t gen = load_relaxed(r.sync + 1);
+    bool wanted = *(volatile uint32_t*)(flags) != 0u, failed = *(volatile uint32_t*)(flags + 1) != 0u;
+    if (*(volatile uint32_t*)(flags + 1) & AZP_EBIT_TIMEOUT) return;  // the barrier's words are unsound
+    for (uint32_t c = tid; c < r.rebuild[0].list.g.ncell; c += nth) r.rebuild[0].cell_count[c] = 0u;
+    if (tid < 6u) r.request[tid] = 0u;
+    if (!grid_barrier(r, gen, &s_word)) return;
+    int par = r.cur;
+    for (uint32_t s = 0; s < r.steps; ++s) {
+        if (wanted && !failed && !rebuild_cooperative<FX>(r, par, gen, smem_raw, &s_word)) return;
+        const MDArgs& a = r.step[par];
+        bool want = false;
+        // blocks beyond the launch's own are taken as they become free
+        uint32_t* next = r.request + 3u + s % 3u;
+        for (uint32_t b = blockIdx.x; b < r.blocks;) {
+            if constexpr (FX)
+                want |= md_step_fx_body<PE, BE, INTEG, false, ONE, false, false>(a, b, ts0 + s, smem_raw);
+            else
+                want |= md_step_body<PE, BE, INTEG, false, false>(a, b, ts0 + s, smem_raw);
+            if (r.blocks <= gridDim.x) break;
+            if (threadIdx.x == 0u) s_word = atomicAdd(next, 1u);
+            __syncthreads();
+            b = gridDim.x + s_word;
+            __syncthreads();  // s_word, and the body's shared memory
+        }
+        uint32_t* word = r.request + s % 3u;
+        if (__any_sync(0xffffffffu, want) && (threadIdx.x & 31u) == 0u) atomicOr(word, 1u);
+        if (threadIdx.x == 0u && *(volatile uint32_t*)(flags + 1) != 0u) atomicOr(word, 2u);
+        if (!grid_barrier(r, gen, &s_word)) return;
+        const uint32_t got = *(volatile uint32_t*)word;
+        if (tid == 0u) {
+            r.request[(s + 2u) % 3u] = 0u;
+            r.request[3u + (s + 2u) % 3u] = 0u;
+        }
+        wanted = (got & 1u) != 0u;
+        failed = failed || (got & 2u) != 0u;
+        par ^= 1;
+    }
+    // a rebuild asked for by the last step, for the launch that follows
+    if (wanted && !failed && !rebuild_cooperative<FX>(r, par, gen, smem_raw, &s_word)) return;
+    if (tid == 0u) {
+        if (wanted && failed) flags[0] = 1u;
+        *r.step[0].d_timestep_rw = ts0 + r.steps;
+    }
+}
+
+template<class PE, class BE, int INTEG, bool FX, bool ONE>
+int launch_run_k(const RunArgs& r, cudaStream_t s)
+{
+    auto k = k_md_run<PE, BE, INTEG, FX, ONE>;
+    const size_t step = FX ? md_step_fx_smem(r.step[0]) : md_step_smem<PE>(r.step[0]);
+    const size_t smem = std::max(step, rebuild_smem(r.step[0].ntypes));
+    int dev = 0, sms = 0, per_sm = 0;
+    AZP_CUDA_TRY(cudaGetDevice(&dev));
+    AZP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    AZP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    AZP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)RUN_BLOCK, smem));
+    const uint32_t most = (uint32_t)(per_sm * sms);
+    // The line against the step-by-step run (the launch is refused before anything is
+    // enqueued). FP32: a step must fit the resident blocks at once, for in this kernel the
+    // body has 80 registers and the rebuild's phases share the residency: graph and this
+    // kernel 113.9 and 111.7 us per step at 432 blocks (fluid 110,592), but 54.5 and 63.4
+    // at 500 (colloid 8,000), 42.9 and 46.6 at 513 (melt 131,300), 173 and 271 at 4,097.
+    // FP64, whose longer steps refill the SMs block by block: a thread per particle must
+    // fit, for the rebuild; 73.9 and 61.9 (melt 40,000), 580 and 573 (colloid 65,537),
+    // but 122.6 and 122.1 at 131,300 and 319 and 348 at 400,000.
+    if (most == 0 || (FX ? r.blocks > most : r.step[0].N > most * RUN_BLOCK)) return AZP_ERR_UNSUPPORTED;
+    // at least a few blocks, for the rebuild
+    const uint32_t grid = std::min(std::max(r.blocks, 16u), most);
+    RunArgs args = r;
+    void* params[] = {&args};
+    AZP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k, dim3(grid), dim3(RUN_BLOCK), params, smem, s));
+    return AZP_OK;
+}
+
+template<class PE, class BE>
+int launch_run_be(int precision, int integ, const RunArgs& r, cudaStream_t s)
+{
+    // the forms that need a kernel of their own before each step (DPD and ImageHarmonic
+    // snapshots, FP32 walls) run step by step
+    if constexpr (!std::is_same<PE, DpdEngine>::value && !bond_uses_image<BE>::value) {
+        const bool one = r.step[0].one_type != 0;
+        if (integ == MD_INTEG_LANGEVIN) {
+            if (precision == AZP_FP64) return launch_run_k<PE, BE, MD_INTEG_LANGEVIN, false, false>(r, s);
+            return one ? launch_run_k<PE, BE, MD_INTEG_LANGEVIN, true, true>(r, s)
+                       : launch_run_k<PE, BE, MD_INTEG_LANGEVIN, true, false>(r, s);
+        }
+        if (integ == MD_INTEG_BROWNIAN) {
+            if (precision == AZP_FP64) return launch_run_k<PE, BE, MD_INTEG_BROWNIAN, false, false>(r, s);
+            return one ? launch_run_k<PE, BE, MD_INTEG_BROWNIAN, true, true>(r, s)
+                       : launch_run_k<PE, BE, MD_INTEG_BROWNIAN, true, false>(r, s);
+        }
+    }
+    return AZP_ERR_UNSUPPORTED;
+}
+
+template<class PE>
+int launch_run_pe(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s)
+{
+    switch (bond_kind) {
+    case -1: return launch_run_be<PE, NoBond>(precision, integ, r, s);
+    case AZP_BOND_QUARTIC: return launch_run_be<PE, QuarticBond>(precision, integ, r, s);
+    case AZP_BOND_DOUBLE_WELL: return launch_run_be<PE, DoubleWellBond>(precision, integ, r, s);
+    default: return AZP_ERR_UNSUPPORTED;
+    }
 }
 
 template<class PE, class BE, typename R, int INTEG>
@@ -1518,10 +1684,8 @@ int launch_md_t(const MDArgs& a, cudaStream_t s)
     const int bs = std::is_same<R, float>::value ? FX_BLOCK : MD_BLOCK;
     const uint32_t blocks = (uint32_t)((threads + bs - 1) / bs);
     if (blocks == 0) return AZP_OK;
-    const size_t nt2 = (size_t)a.ntypes * a.ntypes;
     if constexpr (std::is_same<R, float>::value) {
-        const size_t smem = nt2 * sizeof(double) + nt2 * PAIR_TBL * sizeof(float) +
-                            (size_t)a.nbondtypes * BOND_F * sizeof(float) + 2 * a.ntypes * sizeof(float);
+        const size_t smem = md_step_fx_smem(a);
         constexpr bool can_tile = !std::is_same<PE, NoPair>::value && !std::is_same<PE, DpdEngine>::value &&
                                   !bond_uses_image<BE>::value;
         auto k = a.out ? (a.one_type ? k_md_step_fx<PE, BE, INTEG, true, true> : k_md_step_fx<PE, BE, INTEG, true, false>)
@@ -1541,10 +1705,7 @@ int launch_md_t(const MDArgs& a, cudaStream_t s)
         k<<<blocks, FX_BLOCK, smem_k, s>>>(a);
         AZP_CHECK_LAUNCH("k_md_step_fx");
     } else {
-        const size_t smem = 2 * a.ntypes * sizeof(double) + nt2 * REC64 * sizeof(double) +
-                            (size_t)a.nbondtypes * BOND_REC * sizeof(double) + nt2 * sizeof(float) +
-                            (a.tpp > 1 ? (size_t)(MD_BLOCK / a.tpp) * (a.out ? 10 : 3) * sizeof(double) : 0) +
-                            (std::is_same<PE, NoPair>::value ? 0 : MD_BLOCK * (MD_QUEUE + 1) * sizeof(uint32_t));
+        const size_t smem = md_step_smem<PE>(a);
         // a Brownian step writes no forces, a forces-only launch nothing else
         auto k = k_md_step<PE, BE, INTEG, INTEG == MD_FORCES_ONLY>;
         if constexpr (INTEG == MD_INTEG_LANGEVIN) {
@@ -1598,5 +1759,11 @@ int launch_md_eyuk(int bond_kind, int precision, int integ, const MDArgs& a, cud
 int launch_md_hertz(int bond_kind, int precision, int integ, const MDArgs& a, cudaStream_t s);
 int launch_md_colloid(int bond_kind, int precision, int integ, const MDArgs& a, cudaStream_t s);
 int launch_md_dpd(int bond_kind, int precision, int integ, const MDArgs& a, cudaStream_t s);
+// the persistent run of the same (DPD: none)
+int launch_run_nopair(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s);
+int launch_run_plj(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s);
+int launch_run_eyuk(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s);
+int launch_run_hertz(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s);
+int launch_run_colloid(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s);
 
 }  // namespace azp

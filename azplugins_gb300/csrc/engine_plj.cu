@@ -8,4 +8,9 @@ int launch_md_plj(int bond_kind, int precision, int integ, const MDArgs& a, cuda
 {
     return launch_md_pe<PerturbedLJ>(bond_kind, precision, integ, a, s);
 }
+
+int launch_run_plj(int bond_kind, int precision, int integ, const RunArgs& r, cudaStream_t s)
+{
+    return launch_run_pe<PerturbedLJ>(bond_kind, precision, integ, r, s);
+}
 }  // namespace azp

@@ -16,7 +16,7 @@
 #include <vector>
 
 #include "celllist.cuh"
-#include "fixed64.cuh"
+#include "nlist_device.cuh"
 #include "nlist_impl.cuh"
 #include "scan.cuh"
 
@@ -131,14 +131,6 @@ __global__ void k_to_fixed(const double4_32a* __restrict__ pos, uint4* __restric
     fixed[i] = f;
 }
 
-__device__ __forceinline__ int cell_coord(double x, double lo, double scale, int dim)
-{
-    int c = (int)floor((x - lo) * scale);
-    if (c < 0) c += dim;
-    if (c >= dim) c -= dim;
-    return min(max(c, 0), dim - 1);
-}
-
 __global__ void k_cell_assign(const double4_32a* __restrict__ pos, uint32_t N, CellGrid g, uint32_t* __restrict__ cell_of,
                               uint32_t* __restrict__ slot, uint32_t* __restrict__ cell_count,
                               const uint32_t* __restrict__ gate)
@@ -146,11 +138,7 @@ __global__ void k_cell_assign(const double4_32a* __restrict__ pos, uint32_t N, C
     if (gated_off(gate)) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const double4_32a p = pos[i];
-    const int cx = cell_coord(p.x, g.lo[0], g.scale[0], g.dim[0]);
-    const int cy = cell_coord(p.y, g.lo[1], g.scale[1], g.dim[1]);
-    const int cz = cell_coord(p.z, g.lo[2], g.scale[2], g.dim[2]);
-    const uint32_t c = ((uint32_t)cz * g.dim[1] + cy) * g.dim[0] + cx;
+    const uint32_t c = cell_of_position(pos[i], g);
     cell_of[i] = c;
     slot[i] = atomicAdd(&cell_count[c], 1u);
 }
@@ -173,7 +161,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_cell_sort(const uint32_t* _
 {
     if (gated_off(gate)) return;
     __shared__ uint32_t s_rows[kSortWarps][kMaxSortedCell];
-    sort_cells_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5]);
+    sort_cells_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5], blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
 }
 
 // crowded grids: a warp per cell
@@ -183,38 +171,10 @@ __global__ void __launch_bounds__(kSortWarps * 32) k_cell_sort_crowded(const uin
 {
     if (gated_off(gate)) return;
     __shared__ uint32_t s_rows[kSortWarps][kMaxSortedCell];
-    sort_cell_per_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5]);
+    sort_cell_per_warp(cell_start, members, ncell, s_rows[threadIdx.x >> 5], blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
 }
 
-struct BoxArgs {
-    double L[3], Linv[3];
-    double l64[3];  // L * 2^-64 (64-bit fixed-point unit)
-    float sfix[3];  // L * 2^-32 (fixed-point unit)
-};
-
-inline BoxArgs box_args(const azp_box& b)
-{
-    BoxArgs a;
-    for (int d = 0; d < 3; ++d) {
-        a.L[d] = b.L[d];
-        a.Linv[d] = 1.0 / b.L[d];
-        a.l64[d] = b.L[d] * 5.421010862427522e-20;
-        a.sfix[d] = (float)(b.L[d] * 2.3283064365386963e-10);
-    }
-    return a;
-}
-
-// FP64 position of particle i from its 64-bit fixed-point words (fixed64.cuh)
-__device__ __forceinline__ double4_32a fx_position(const uint4* __restrict__ hi, const uint4* __restrict__ lo,
-                                                   uint32_t i, const BoxArgs& bx)
-{
-    const uint4 h = hi[i], l = lo[i];
-    return make_double4_32a(fx_to_double(fx_join(h.x, l.x), bx.l64[0]), fx_to_double(fx_join(h.y, l.y), bx.l64[1]),
-                            fx_to_double(fx_join(h.z, l.z), bx.l64[2]), 0.0);
-}
-
-// cell of each particle from the high words of its 64-bit fixed position:
-// [-2^31, 2^31) maps linearly onto [0, dim) in integer arithmetic
+// cell of each particle from the high words of its 64-bit fixed position
 __global__ void k_cell_assign_fx(const uint4* __restrict__ fixed, uint32_t N, CellGrid g,
                                  uint32_t* __restrict__ cell_of, uint32_t* __restrict__ slot,
                                  uint32_t* __restrict__ cell_count, const uint32_t* __restrict__ gate)
@@ -222,438 +182,40 @@ __global__ void k_cell_assign_fx(const uint4* __restrict__ fixed, uint32_t N, Ce
     if (gated_off(gate)) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const uint4 f = fixed[i];
-    const uint32_t cx = (uint32_t)(((uint64_t)(f.x ^ 0x80000000u) * (uint32_t)g.dim[0]) >> 32);
-    const uint32_t cy = (uint32_t)(((uint64_t)(f.y ^ 0x80000000u) * (uint32_t)g.dim[1]) >> 32);
-    const uint32_t cz = (uint32_t)(((uint64_t)(f.z ^ 0x80000000u) * (uint32_t)g.dim[2]) >> 32);
-    const uint32_t c = (cz * (uint32_t)g.dim[1] + cy) * (uint32_t)g.dim[0] + cx;
+    const uint32_t c = cell_of_fixed(fixed[i], g);
     cell_of[i] = c;
     slot[i] = atomicAdd(&cell_count[c], 1u);
 }
 
-constexpr uint32_t MAX_LIST_TYPES = 16;  // ntypes^2 <= 256 thresholds in shared memory
-constexpr int NLIST_BLOCK = 128;
-static_assert(TILE_P % NLIST_BLOCK == 0, "a list-build block lies inside one tile block");
-constexpr uint32_t NL_EX_REG = 4;  // exclusion keys of a particle held in registers
-// Candidates in the FP32 band around r_list are appended with this mark and
-// decided exactly in the compaction pass: the scan loop then holds no call and
-// no FP64 state (measured at N = 1M: 40 registers instead of 64, the build 20 %
-// faster, the same sets).
-constexpr uint32_t NL_BAND = 0x80000000u;
-constexpr uint32_t NL_MAX_N = NL_BAND - 1;  // particle indices stay below the mark
-
-// The oracle's exact FP64 decision for a candidate inside the ambiguous band
-// of the FP32 prefilter. Out of line: a candidate lands in the band about once
-// per million.
-__device__ __noinline__ bool nl_exact_within(uint32_t i, uint32_t j, double rlistsq, const BoxArgs& bx,
-                                             const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed,
-                                             const uint4* __restrict__ lo)
-{
-    const double4_32a a = lo ? fx_position(fixed, lo, i, bx) : pos[i];
-    const double4_32a b = lo ? fx_position(fixed, lo, j, bx) : pos[j];
-    const double vx = min_image1(a.x - b.x, bx.L[0], bx.Linv[0]);
-    const double vy = min_image1(a.y - b.y, bx.L[1], bx.Linv[1]);
-    const double vz = min_image1(a.z - b.z, bx.L[2], bx.Linv[2]);
-    return rsq_exact(vx, vy, vz) < rlistsq;
-}
-
-// exclusion keys of a particle beyond the NL_EX_REG held in registers
-__device__ __noinline__ bool nl_excluded_tail(uint32_t i, uint32_t kj, uint32_t nex, uint32_t N,
-                                              const uint32_t* __restrict__ ex_keys)
-{
-    for (uint32_t e = NL_EX_REG; e < nex; ++e)
-        if (ex_keys[(size_t)e * N + i] == kj) return true;
-    return false;
-}
-
-// Full list, one thread per particle. For every (y, z) offset row of the 3x3x3
-// cell stencil, the x-neighbour cells cx-1, cx, cx+1 are consecutive cell
-// indices, so their particles are one contiguous slot range (members[s], or s
-// itself when the particles are stored in cell order); at the x faces the
-// wrapped cell is a second range. The scan per candidate is one 16-byte gather,
-// the integer minimum image and the FP32 prefilter; ONE_TYPE keeps the
-// thresholds of a single-type system in registers.
 template<bool ONE_TYPE, bool SORTED>
 __global__ void __launch_bounds__(NLIST_BLOCK)
-    k_nlist_build_threads(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed, uint32_t N, BoxArgs bx,
-                          CellGrid g, const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ members,
-                          const uint32_t* __restrict__ cell_of, const ListCut* __restrict__ cuts, uint32_t ntypes,
-                          const uint32_t* __restrict__ ex_n, const uint32_t* __restrict__ ex_keys,
-                          const uint32_t* __restrict__ keys, uint32_t* __restrict__ counts,
-                          uint32_t* __restrict__ nbrs, uint32_t max_nn, uint32_t* __restrict__ flags,
-                          const uint32_t* __restrict__ gate, const uint4* __restrict__ lo,
+    k_nlist_build_threads(const __grid_constant__ ListArgs L, const uint32_t* __restrict__ gate,
                           const uint32_t* __restrict__ tile)
 {
     if (gated_off(gate)) return;
     __shared__ ListCut s_cut[MAX_LIST_TYPES * MAX_LIST_TYPES];
     // the tile record of this block's particles (NLIST_BLOCK divides TILE_P)
     __shared__ uint32_t s_trec[TILE_REC];
-    const uint32_t nt2 = ntypes * ntypes;
-    for (uint32_t t = threadIdx.x; t < nt2; t += blockDim.x) s_cut[t] = cuts[t];
+    const uint32_t nt2 = L.ntypes * L.ntypes;
+    for (uint32_t t = threadIdx.x; t < nt2; t += blockDim.x) s_cut[t] = L.cuts[t];
     if (tile && threadIdx.x < TILE_REC)
         s_trec[threadIdx.x] = tile[(size_t)(blockIdx.x * blockDim.x / TILE_P) * TILE_REC + threadIdx.x];
     __syncthreads();
-
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const uint4 fi = __ldg(fixed + i);
-    const uint32_t row = fi.w * ntypes;
-    const ListCut cut0 = s_cut[0];
-    const uint32_t nex = ex_n ? __ldg(ex_n + i) : 0u;
-    const uint32_t cc = __ldg(cell_of + i);
-    const int dx = g.dim[0], dy = g.dim[1], dz = g.dim[2];
-    const int cx = (int)(cc % (uint32_t)dx);
-    const int cy = (int)((cc / (uint32_t)dx) % (uint32_t)dy);
-    const int cz = (int)(cc / ((uint32_t)dx * (uint32_t)dy));
-    // the x-cells cx - reach .. cx + reach: one contiguous range inside the row,
-    // and the wrapped part at an x face, contiguous too ([wb, we]; empty: wb > we)
-    int x0 = cx - g.reach[0], x1 = cx + g.reach[0], wb = 1, we = 0;
-    if (x0 < 0) {
-        wb = dx + x0;
-        we = dx - 1;
-        x0 = 0;
-    }
-    if (x1 >= dx) {
-        wb = 0;
-        we = x1 - dx;
-        x1 = dx - 1;
-    }
-    uint32_t ex[NL_EX_REG];
-#pragma unroll
-    for (uint32_t e = 0; e < NL_EX_REG; ++e) ex[e] = e < nex ? __ldg(ex_keys + (size_t)e * N + i) : 0xffffffffu;
-    uint32_t n = 0;
-    // one candidate: the integer minimum image, the FP32 prefilter, the append
-    const auto test = [&](uint32_t j, const uint4& fj) {
-        const float ddx = (float)(int32_t)(fi.x - fj.x) * bx.sfix[0];
-        const float ddy = (float)(int32_t)(fi.y - fj.y) * bx.sfix[1];
-        const float ddz = (float)(int32_t)(fi.z - fj.z) * bx.sfix[2];
-        const float rs = ddx * ddx + ddy * ddy + ddz * ddz;
-        const ListCut cut = ONE_TYPE ? cut0 : s_cut[row + fj.w];
-        // within r_list or in the band around it: appended (i itself, its
-        // excluded partners and the band candidates, marked, too; the pass
-        // below takes out what does not belong)
-        if (rs < cut.hi) {
-            if (n < max_nn) nbrs[(size_t)n * N + i] = rs < cut.lo ? j : (j | NL_BAND);
-            ++n;
-        }
-    };
-    for (int oz = -g.reach[2]; oz <= g.reach[2]; ++oz) {
-        int nz = cz + oz;
-        nz += (nz < 0) ? dz : 0;
-        nz -= (nz >= dz) ? dz : 0;
-        for (int oy = -g.reach[1]; oy <= g.reach[1]; ++oy) {
-            int ny = cy + oy;
-            ny += (ny < 0) ? dy : 0;
-            ny -= (ny >= dy) ? dy : 0;
-            const uint32_t rb = ((uint32_t)nz * dy + ny) * dx;
-            for (int part = 0; part < 2; ++part) {
-                uint32_t sb, se;
-                if (part == 0) {
-                    sb = __ldg(cell_start + rb + x0);
-                    se = __ldg(cell_start + rb + x1 + 1);
-                } else {
-                    if (wb > we) break;
-                    sb = __ldg(cell_start + rb + wb);
-                    se = __ldg(cell_start + rb + we + 1);
-                }
-#pragma unroll 4
-                for (uint32_t sl = sb; sl < se; ++sl) {
-                    const uint32_t j = SORTED ? sl : __ldg(members + sl);
-                    test(j, __ldg(fixed + j));
-                }
-            }
-        }
-    }
-    // Compact the row in place: drop i itself and the excluded partners, keeping
-    // the order. The warp-wide scan above stays a load, a test and an append; the
-    // exclusion compares run once per listed entry here instead of on every
-    // candidate iteration. Overflow is judged on the raw count, which bounds the
-    // true one, so a row that lost entries to the capacity is always reported.
-    const uint32_t stored = min(n, max_nn);
-    uint32_t m = 0;
-    for (uint32_t k = 0; k < stored; ++k) {
-        uint32_t j = nbrs[(size_t)k * N + i];
-        const bool marked = (j & NL_BAND) != 0u;
-        bool drop = false;
-        if (marked) {
-            // a candidate in the band around r_list: the oracle's exact FP64 decision
-            j &= ~NL_BAND;
-            const ListCut cut = ONE_TYPE ? cut0 : s_cut[row + __ldg(fixed + j).w];
-            drop = !nl_exact_within(i, j, cut.rlistsq, bx, pos, fixed, lo);
-        }
-        drop |= j == i;
-        if (nex && !drop) {
-            const uint32_t kj = keys ? __ldg(keys + j) : j;
-#pragma unroll
-            for (uint32_t e = 0; e < NL_EX_REG; ++e) drop |= ex[e] == kj;
-            if (nex > NL_EX_REG) drop |= nl_excluded_tail(i, kj, nex, N, ex_keys);
-        }
-        if (!drop) {
-            if (tile) nbrs[(size_t)m * N + i] = tile_encode(s_trec, j);
-            else if (m != k || marked) nbrs[(size_t)m * N + i] = j;  // a kept band entry loses its mark
-            ++m;
-        }
-    }
-    counts[i] = n > max_nn ? n : m;
-    if (n > max_nn) atomicMax(&flags[0], n);
+    nlist_thread<true, ONE_TYPE, SORTED>(L, blockIdx.x * blockDim.x + threadIdx.x, s_cut, tile ? s_trec : nullptr);
 }
 
-// The list with a warp per chunk of cell-ordered particles. A warp takes CH consecutive
-// slots of the cell order, the particles of one cell at a time. The slot ranges of their
-// stencil rows are laid end to end (bounds read and summed by the lanes together) and
-// walked 32 candidates a step, each loaded once, a step ahead, and tested against every
-// particle of the chunk: a ballot ranks the hits, which are appended to the particles' rows
-// in shared memory. Rows with excluded partners or candidates of the band are then compacted
-// there, and the rows written out with the chunk's particles side by side. Order and
-// contents are those of k_nlist_build_threads.
-// words: the candidates' fixed-point words in cell order (fixed itself when SORTED).
-// Particles whose types have smaller list radii than the grid's walk fewer cells.
-// REF: coordinates as floats relative to the chunk's first particle, so that a test
-// costs no integer conversion (16 a clock and SM); grids with at least 2 reach + 3 cells on
-// every axis, where the minimum image relative to that particle is the pair's for all
-// pairs in range.
-constexpr int NLW_WARPS = 4;
-constexpr uint32_t NLW_ROW = 192;   // entries of a row held in shared memory; the rest go to the list at once
-constexpr uint32_t NLW_RANGES = 2 * 9 * 9;  // stencil rows (reach <= 4) and their wrapped parts
 template<bool ONE_TYPE, bool SORTED, bool REF, int CH>
 __global__ void __launch_bounds__(NLW_WARPS * 32)
-    k_nlist_build_warps(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed,
-                        const uint4* __restrict__ words, uint32_t N, BoxArgs bx, CellGrid g,
-                        const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ members,
-                        const uint32_t* __restrict__ cell_of, const ListCut* __restrict__ cuts, uint32_t ntypes,
-                        const uint32_t* __restrict__ ex_n, const uint32_t* __restrict__ ex_keys,
-                        uint32_t* __restrict__ counts, uint32_t* __restrict__ nbrs, uint32_t max_nn,
-                        uint32_t* __restrict__ flags, const uint32_t* __restrict__ gate, const uint4* __restrict__ lo)
+    k_nlist_build_warps(const __grid_constant__ ListArgs L, const uint4* __restrict__ words,
+                        const uint32_t* __restrict__ gate)
 {
     if (gated_off(gate)) return;
-    __shared__ uint32_t s_rows[NLW_WARPS][CH][NLW_ROW];
-    __shared__ uint2 s_range[NLW_WARPS][NLW_RANGES + 1];  // (first candidate, first slot) of each range
-    __shared__ int s_reach[MAX_LIST_TYPES][3];
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ListCut* s_cut = reinterpret_cast<ListCut*>(smem_raw);
-    float* s_hi = reinterpret_cast<float*>(s_cut + ntypes * ntypes);
-    float* s_lo = s_hi + ntypes * ntypes;
-    for (uint32_t t = threadIdx.x; t < ntypes * ntypes; t += blockDim.x) {
-        s_cut[t] = cuts[t];
-        s_hi[t] = cuts[t].hi;
-        s_lo[t] = cuts[t].lo;
-    }
-    for (uint32_t t = threadIdx.x; t < ntypes; t += blockDim.x) {
-        // cells beyond ceil(r / width) lie further than the type's largest list radius
-        double r2 = 0.0;
-        for (uint32_t u = 0; u < ntypes; ++u) r2 = fmax(r2, cuts[t * ntypes + u].rlistsq);
-        const double r = sqrt(r2) * (1.0 + 1e-5);
-        for (int d = 0; d < 3; ++d) s_reach[t][d] = min(g.reach[d], (int)ceil(r * g.scale[d]));
-    }
+    const NlwShared sh = nlw_shared<CH>(smem_raw, L.ntypes, NLW_WARPS);
+    nlw_tables(sh, L.cuts, L.ntypes, L.g);
     __syncthreads();
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t(*rows)[NLW_ROW] = s_rows[threadIdx.x >> 5];
-    uint2* range = s_range[threadIdx.x >> 5];
-    const ListCut cut0 = s_cut[0];
-    const int dx = g.dim[0], dy = g.dim[1], dz = g.dim[2];
-    const uint32_t s_begin = (blockIdx.x * NLW_WARPS + (threadIdx.x >> 5)) * CH;
-    const uint32_t s_end = min(s_begin + CH, N);
-    for (uint32_t sa = s_begin; sa < s_end;) {
-        // the slots from sa on that share its cell
-        const uint32_t my_slot = min(sa + lane, s_end - 1u);
-        const uint32_t my_i = SORTED ? my_slot : __ldg(members + my_slot);
-        const uint32_t my_cell = __ldg(cell_of + my_i);
-        const uint4 my_word = __ldg(words + my_slot);
-        const uint32_t cc = __shfl_sync(0xffffffffu, my_cell, 0);
-        const uint32_t same = __ballot_sync(0xffffffffu, my_cell == cc && sa + lane < s_end);
-        const uint32_t cnt = (uint32_t)__ffs(~same) - 1u;  // CH < 32: some lane is off
-        uint32_t pi[CH], n[CH];
-        uint4 pw[CH];
-        float px[CH], py[CH], pz[CH];
-        const uint4 ref = make_uint4(__shfl_sync(0xffffffffu, my_word.x, 0), __shfl_sync(0xffffffffu, my_word.y, 0),
-                                     __shfl_sync(0xffffffffu, my_word.z, 0), 0u);
-        int r0 = 0, r1 = 0, r2 = 0;
-#pragma unroll
-        for (int p = 0; p < CH; ++p) {
-            pi[p] = __shfl_sync(0xffffffffu, my_i, p);
-            pw[p].x = __shfl_sync(0xffffffffu, my_word.x, p);
-            pw[p].y = __shfl_sync(0xffffffffu, my_word.y, p);
-            pw[p].z = __shfl_sync(0xffffffffu, my_word.z, p);
-            pw[p].w = ONE_TYPE ? 0u : __shfl_sync(0xffffffffu, my_word.w, p);
-            n[p] = 0u;
-            px[p] = (float)(int32_t)(pw[p].x - ref.x) * bx.sfix[0];
-            py[p] = (float)(int32_t)(pw[p].y - ref.y) * bx.sfix[1];
-            pz[p] = (float)(int32_t)(pw[p].z - ref.z) * bx.sfix[2];
-            if (p < (int)cnt) {
-                const int* r = s_reach[pw[p].w];
-                r0 = max(r0, r[0]);
-                r1 = max(r1, r[1]);
-                r2 = max(r2, r[2]);
-            }
-            pw[p].w *= ntypes;
-        }
-        const int cx = (int)(cc % (uint32_t)dx);
-        const int cy = (int)((cc / (uint32_t)dx) % (uint32_t)dy);
-        const int cz = (int)(cc / ((uint32_t)dx * (uint32_t)dy));
-        // the x-cells as in k_nlist_build_threads: one range, and the wrapped part
-        int x0 = cx - r0, x1 = cx + r0, wb = 1, we = 0;
-        if (x0 < 0) {
-            wb = dx + x0;
-            we = dx - 1;
-            x0 = 0;
-        }
-        if (x1 >= dx) {
-            wb = 0;
-            we = x1 - dx;
-            x1 = dx - 1;
-        }
-        const bool wrap = wb <= we;
-        const uint32_t parts = wrap ? 2u : 1u;
-        const uint32_t ny = 2u * r1 + 1u;
-        const uint32_t nr = ny * (2u * r2 + 1u) * parts;
-        uint32_t total = 0u;
-        for (uint32_t q0 = 0; q0 < nr; q0 += 32u) {
-            const uint32_t q = q0 + lane;
-            uint32_t sb = 0u, len = 0u;
-            if (q < nr) {
-                const uint32_t row = q / parts, part = q - row * parts;
-                int oz = cz - r2 + (int)(row / ny), oy = cy - r1 + (int)(row % ny);
-                oz += (oz < 0) ? dz : 0;
-                oz -= (oz >= dz) ? dz : 0;
-                oy += (oy < 0) ? dy : 0;
-                oy -= (oy >= dy) ? dy : 0;
-                const uint32_t rb = ((uint32_t)oz * dy + oy) * dx;
-                sb = __ldg(cell_start + rb + (part ? wb : x0));
-                len = __ldg(cell_start + rb + (part ? we : x1) + 1) - sb;
-            }
-            uint32_t sum = len;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
-                if ((int)lane >= o) sum += v;
-            }
-            if (q < nr) range[q] = make_uint2(total + sum - len, sb);
-            total += __shfl_sync(0xffffffffu, sum, 31);
-        }
-        if (lane == 0u) range[nr] = make_uint2(0xffffffffu, 0u);
-        __syncwarp();
-        bool band = false;
-        uint32_t q = 0u;
-        // slot of candidate c (rising by 32 a call)
-        const auto slot_of = [&](uint32_t c) -> uint32_t {
-            while (range[q + 1u].x <= c) ++q;
-            const uint2 r = range[q];
-            return r.y + (c - r.x);
-        };
-        uint32_t sl = lane < total ? slot_of(lane) : 0u;
-        uint4 w = __ldg(words + sl);
-        uint32_t j = SORTED ? sl : __ldg(members + sl);
-        for (uint32_t c0 = 0; c0 < total; c0 += 32u) {
-            const bool on = c0 + lane < total;
-            const uint4 wc = w;
-            const uint32_t jc = j;
-            if (c0 + 32u + lane < total) {
-                sl = slot_of(c0 + 32u + lane);
-                w = __ldg(words + sl);
-                j = SORTED ? sl : __ldg(members + sl);
-            }
-            // a lane without a candidate stands outside every radius
-            float qx = 0.0f, qy = 0.0f, qz = on ? 0.0f : INFINITY;
-            if (REF && on) {
-                qx = (float)(int32_t)(wc.x - ref.x) * bx.sfix[0];
-                qy = (float)(int32_t)(wc.y - ref.y) * bx.sfix[1];
-                qz = (float)(int32_t)(wc.z - ref.z) * bx.sfix[2];
-            }
-            const float* hi = s_hi + (ONE_TYPE ? 0u : wc.w);
-            const float* lo_ = s_lo + (ONE_TYPE ? 0u : wc.w);
-#pragma unroll
-            for (int p = 0; p < CH; ++p) {
-                if (p >= (int)cnt) break;
-                float ddx, ddy, ddz;
-                if constexpr (REF) {
-                    ddx = px[p] - qx;
-                    ddy = py[p] - qy;
-                    ddz = pz[p] - qz;
-                } else {
-                    ddx = (float)(int32_t)(pw[p].x - wc.x) * bx.sfix[0];
-                    ddy = (float)(int32_t)(pw[p].y - wc.y) * bx.sfix[1];
-                    ddz = (float)(int32_t)(pw[p].z - wc.z) * bx.sfix[2] - qz;
-                }
-                const float rs = ddx * ddx + ddy * ddy + ddz * ddz;
-                const bool hit = (rs < (ONE_TYPE ? cut0.hi : hi[pw[p].w])) & (jc != pi[p]);
-                const uint32_t hits = __ballot_sync(0xffffffffu, hit);
-                if (hit) {
-                    const uint32_t k = n[p] + __popc(hits & lt);
-                    const bool sure = rs < (ONE_TYPE ? cut0.lo : lo_[pw[p].w]);
-                    const uint32_t e = sure ? jc : (jc | NL_BAND);
-                    band = band || !sure;
-                    if (k < NLW_ROW) rows[p][k] = e;
-                    else if (k < max_nn) nbrs[(size_t)k * N + pi[p]] = e;
-                }
-                n[p] += __popc(hits);
-            }
-        }
-        band = __any_sync(0xffffffffu, band);
-        // compaction, in order, of the rows that may hold what does not belong
-        uint32_t kept[CH], kept_max = 0u;
-#pragma unroll
-        for (int p = 0; p < CH; ++p) {
-            kept[p] = 0u;
-            if (p >= (int)cnt) continue;
-            const uint32_t i = pi[p];
-            // the particle itself counts as listed for the capacity, as in
-            // k_nlist_build_threads, whose scan takes it in
-            const uint32_t raw = n[p] + ((ONE_TYPE ? cut0.hi : s_hi[pw[p].w + pw[p].w / ntypes]) > 0.0f ? 1u : 0u);
-            const uint32_t stored = min(n[p], max_nn);
-            const uint32_t nex = ex_n ? __ldg(ex_n + i) : 0u;
-            uint32_t m = stored;
-            if (band || nex) {
-                m = 0u;
-                for (uint32_t k0 = 0; k0 < stored; k0 += 32u) {
-                    const uint32_t k = k0 + lane;
-                    bool keep = k < stored;
-                    uint32_t e = 0u;
-                    if (keep) {
-                        e = k < NLW_ROW ? rows[p][k] : nbrs[(size_t)k * N + i];
-                        if (e & NL_BAND) {
-                            // the oracle's exact FP64 decision
-                            e &= ~NL_BAND;
-                            const double r2l = ONE_TYPE ? cut0.rlistsq : s_cut[pw[p].w + __ldg(fixed + e).w].rlistsq;
-                            keep = nl_exact_within(i, e, r2l, bx, pos, fixed, lo);
-                        }
-                        for (uint32_t x = 0; x < nex; ++x) keep = keep && __ldg(ex_keys + (size_t)x * N + i) != e;
-                    }
-                    const uint32_t mask = __ballot_sync(0xffffffffu, keep);
-                    if (keep) {
-                        const uint32_t d = m + __popc(mask & lt);
-                        if (d < NLW_ROW) rows[p][d] = e;
-                        else nbrs[(size_t)d * N + i] = e;
-                    }
-                    __syncwarp();
-                    m += __popc(mask);
-                }
-            }
-            kept[p] = min(m, NLW_ROW);
-            kept_max = max(kept_max, kept[p]);
-            if (lane == 0u) {
-                counts[i] = raw > max_nn ? raw : m;
-                if (raw > max_nn) atomicMax(&flags[0], raw);
-            }
-        }
-        __syncwarp();
-        // the chunk's rows side by side: lanes of consecutive particles
-        {
-            constexpr uint32_t STEP = 32u / CH;
-            const uint32_t p = lane % CH, kk = lane / CH;
-            uint32_t i = 0u, m = 0u;
-#pragma unroll
-            for (int u = 0; u < CH; ++u)
-                if (u == (int)p && u < (int)cnt) {
-                    i = pi[u];
-                    m = kept[u];
-                }
-            for (uint32_t k = kk; k < kept_max; k += STEP)
-                if (k < m) nbrs[(size_t)k * N + i] = rows[p][k];
-        }
-        __syncwarp();
-        sa += cnt;
-    }
+    nlist_chunk<true, ONE_TYPE, SORTED, REF, CH>(L, words, blockIdx.x * NLW_WARPS + (threadIdx.x >> 5), threadIdx.x >> 5,
+                                                 sh);
 }
 
 // the words of the particles in cell order
@@ -834,39 +396,35 @@ void launch_nlist_build(const double4_32a* pos, const uint4* fixed, uint32_t N, 
     (void)rlist_min;
     if (N == 0) return;
     const BoxArgs bx = box_args(box);
+    const ListArgs L{pos, fixed, lo, N, ntypes, bx, g, cell_start, members, cell_of, cuts, ex_n, ex_keys, keys,
+                     counts, nbrs, max_nn, flags};
     if (!keys && !tile && (!members || words) && warp_list_build(N, g, !members)) {
-        bool ref = true;
-        for (int d = 0; d < 3; ++d) ref = ref && g.dim[d] >= 2 * g.reach[d] + 3;
-        const size_t smem = (sizeof(ListCut) + 2 * sizeof(float)) * ntypes * ntypes;
         // small systems: four particles a warp, for more warps
         const bool few = N < 40000u;
-        const uint32_t per = NLW_WARPS * (few ? 4u : 8u);
-        const uint32_t nb = (N + per - 1) / per;
-        const auto go = [&](auto kernel) {
-            kernel<<<nb, NLW_WARPS * 32, smem, s>>>(pos, fixed, members ? words : fixed, N, bx, g, cell_start, members,
-                                                    cell_of, cuts, ntypes, ex_n, ex_keys, counts, nbrs, max_nn, flags,
-                                                    gate, lo);
+        const auto go = [&](auto kernel, size_t smem) {
+            const uint32_t per = NLW_WARPS * (few ? 4u : 8u);
+            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            kernel<<<(N + per - 1) / per, NLW_WARPS * 32, smem, s>>>(L, members ? words : fixed, gate);
         };
-#define AZP_NLW(ONE, SORTED)                                                                              \
-    (ref ? (few ? go(k_nlist_build_warps<ONE, SORTED, true, 4>) : go(k_nlist_build_warps<ONE, SORTED, true, 8>)) \
-         : (few ? go(k_nlist_build_warps<ONE, SORTED, false, 4>) : go(k_nlist_build_warps<ONE, SORTED, false, 8>)))
+        const size_t s4 = nlw_shared_bytes<4>(ntypes, NLW_WARPS), s8 = nlw_shared_bytes<8>(ntypes, NLW_WARPS);
+#define AZP_NLW(ONE, SORTED)                                                               \
+    (list_by_reference(g)                                                                  \
+         ? (few ? go(k_nlist_build_warps<ONE, SORTED, true, 4>, s4) : go(k_nlist_build_warps<ONE, SORTED, true, 8>, s8)) \
+         : (few ? go(k_nlist_build_warps<ONE, SORTED, false, 4>, s4) : go(k_nlist_build_warps<ONE, SORTED, false, 8>, s8)))
         if (ntypes == 1) members ? AZP_NLW(true, false) : AZP_NLW(true, true);
         else members ? AZP_NLW(false, false) : AZP_NLW(false, true);
 #undef AZP_NLW
         return;
     }
     const uint32_t blocks = (N + NLIST_BLOCK - 1) / NLIST_BLOCK;
-#define AZP_NL_ARGS                                                                                              \
-    pos, fixed, N, bx, g, cell_start, members, cell_of, cuts, ntypes, ex_n, ex_keys, keys, counts, nbrs, max_nn, \
-        flags, gate, lo, members ? nullptr : tile
+    if (members) tile = nullptr;
     if (ntypes == 1) {
-        if (members) k_nlist_build_threads<true, false><<<blocks, NLIST_BLOCK, 0, s>>>(AZP_NL_ARGS);
-        else k_nlist_build_threads<true, true><<<blocks, NLIST_BLOCK, 0, s>>>(AZP_NL_ARGS);
+        if (members) k_nlist_build_threads<true, false><<<blocks, NLIST_BLOCK, 0, s>>>(L, gate, tile);
+        else k_nlist_build_threads<true, true><<<blocks, NLIST_BLOCK, 0, s>>>(L, gate, tile);
     } else {
-        if (members) k_nlist_build_threads<false, false><<<blocks, NLIST_BLOCK, 0, s>>>(AZP_NL_ARGS);
-        else k_nlist_build_threads<false, true><<<blocks, NLIST_BLOCK, 0, s>>>(AZP_NL_ARGS);
+        if (members) k_nlist_build_threads<false, false><<<blocks, NLIST_BLOCK, 0, s>>>(L, gate, tile);
+        else k_nlist_build_threads<false, true><<<blocks, NLIST_BLOCK, 0, s>>>(L, gate, tile);
     }
-#undef AZP_NL_ARGS
 }
 
 void launch_cell_assign_fx(const uint4* fixed, uint32_t N, const CellGrid& g, uint32_t* cell_of, uint32_t* slot,
