@@ -41,20 +41,15 @@ struct SysInfo {
     int reach[3];
     double cscale[3];         // dim / L
     uint32_t seed;
-    uint32_t pad_;
+    uint32_t off, n;          // the replica's particles: [off, off + n)
+    uint32_t far_cells;       // every axis has 2 reach + 3 cells or more (k_b_nlist)
+    float recf[PAIR_TBL];     // rec and rcutsq as the FP32 step reads them
+    float rcutf;
     double rec[PAIR_TBL];     // pair kernel record + cut record (one type)
 };
 
 constexpr int BATCH_BLOCK = 256;      // default threads per block of the fused step
 constexpr int BATCH_BLOCK_MAX = 512;  // largest block azp_batch_set_block accepts
-
-AZP_D void comp_shfl_add(Comp& c, int m)
-{
-    const float s2 = __shfl_xor_sync(0xffffffffu, c.s, m);
-    const float c2 = __shfl_xor_sync(0xffffffffu, c.c, m);
-    c.add(s2);
-    c.c += c2;
-}
 
 // ---------------------------------------------------------------- rebuild kernels
 __global__ void k_b_zero(uint32_t* __restrict__ p, uint32_t n, const uint32_t* __restrict__ gate)
@@ -182,60 +177,165 @@ __global__ void k_b_fixed(const double4_32a* __restrict__ pos, const uint16_t* _
     fb[i] = f;
 }
 
-__global__ void __launch_bounds__(128)
-    k_b_nlist(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed, const uint16_t* __restrict__ sys,
-              uint32_t N, const SysInfo* __restrict__ info, const uint32_t* __restrict__ cell_start,
-              const uint32_t* __restrict__ cell_of, uint32_t* __restrict__ counts, uint32_t* __restrict__ nbrs,
-              uint32_t max_nn, uint32_t* __restrict__ maxcount, const uint32_t* __restrict__ gate)
+// The list, a warp per B_CHUNK consecutive particles, those of one cell at a time. The
+// stencil rows of the cell are laid end to end (nlist_chunk has the same walk) and taken 32
+// candidates a step, each loaded once and tested against every particle of the chunk; a
+// ballot ranks the hits, which go to the particles' rows side by side. Coordinates are
+// floats relative to the chunk's first particle (an integer conversion per candidate, not
+// per test); where an axis has fewer than 2 reach + 3 cells the difference is wrapped once
+// more. |coordinate| <= L / 2 <= 2.5 r_list there, which the band around r_list
+// (make_list_cuts, 5e-6) covers: both coordinates' roundings come to 2.1e-6 of r^2.
+// Bound by issue (14 or 23 instructions a test). One thread per particle and a column of
+// the list each took 1,010 us for 48 replicas (337,467 particles, 94 M entries), with
+// 32 lanes on rows of 15 to 2,800 entries; this takes 490.
+constexpr int B_CHUNK = 8;
+constexpr int B_NL_WARPS = 4;
+constexpr uint32_t B_RANGES = 2 * 3 * 3;  // stencil rows and their wrapped parts
+template<bool WRAP>
+AZP_D uint32_t b_walk(const uint4* __restrict__ fixed, const double4_32a* __restrict__ pos, const SysInfo& si,
+                      const uint2* range, uint32_t total, uint32_t first, uint32_t cnt, uint32_t* __restrict__ nbrs,
+                      uint32_t width, uint32_t max_nn)
 {
-    if (gated_off(gate)) return;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const SysInfo& si = info[sys[i]];
-    const uint4 fi = fixed[i];
-    const uint32_t c = cell_of[i] - si.cell_off;
-    const int cx = (int)(c % si.dim[0]);
-    const int cy = (int)((c / si.dim[0]) % si.dim[1]);
-    const int cz = (int)(c / ((uint32_t)si.dim[0] * si.dim[1]));
-    uint32_t n = 0;
-    for (int oz = -si.reach[2]; oz <= si.reach[2]; ++oz) {
-        int nz = cz + oz;
-        nz += (nz < 0) ? si.dim[2] : 0;
-        nz -= (nz >= si.dim[2]) ? si.dim[2] : 0;
-        for (int oy = -si.reach[1]; oy <= si.reach[1]; ++oy) {
-            int ny = cy + oy;
-            ny += (ny < 0) ? si.dim[1] : 0;
-            ny -= (ny >= si.dim[1]) ? si.dim[1] : 0;
-            for (int ox = -si.reach[0]; ox <= si.reach[0]; ++ox) {
-                int nx = cx + ox;
-                nx += (nx < 0) ? si.dim[0] : 0;
-                nx -= (nx >= si.dim[0]) ? si.dim[0] : 0;
-                const uint32_t nc = si.cell_off + ((uint32_t)nz * si.dim[1] + ny) * si.dim[0] + nx;
-                const uint32_t sb = cell_start[nc], se = cell_start[nc + 1];
-                for (uint32_t j = sb; j < se; ++j) {
-                    if (j == i) continue;
-                    const uint4 fj = fixed[j];
-                    const float dx = (float)(int32_t)(fi.x - fj.x) * si.sfix[0];
-                    const float dy = (float)(int32_t)(fi.y - fj.y) * si.sfix[1];
-                    const float dz = (float)(int32_t)(fi.z - fj.z) * si.sfix[2];
-                    const float rs = dx * dx + dy * dy + dz * dz;
-                    if (rs >= si.list_hi) continue;
-                    if (!(rs < si.list_lo)) {
-                        const double4_32a pi = pos[i];
-                        const double4_32a pj = pos[j];
-                        const double vx = min_image1(pi.x - pj.x, si.L[0], si.Linv[0]);
-                        const double vy = min_image1(pi.y - pj.y, si.L[1], si.Linv[1]);
-                        const double vz = min_image1(pi.z - pj.z, si.L[2], si.Linv[2]);
-                        if (!(rsq_exact(vx, vy, vz) < si.rlistsq)) continue;
-                    }
-                    if (n < max_nn) nbrs[(size_t)n * N + i] = j;
-                    ++n;
-                }
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lt = (1u << lane) - 1u;
+    const float sx = si.sfix[0], sy = si.sfix[1], sz = si.sfix[2];
+    const float Lx = sx * 4294967296.0f, Ly = sy * 4294967296.0f, Lz = sz * 4294967296.0f;
+    const float ix = 1.0f / Lx, iy = 1.0f / Ly, iz = 1.0f / Lz;
+    const float hi = si.list_hi, lo = si.list_lo;
+    const uint4 ref = fixed[first];
+    float px[B_CHUNK], py[B_CHUNK], pz[B_CHUNK];
+    uint32_t n[B_CHUNK];
+#pragma unroll
+    for (int p = 0; p < B_CHUNK; ++p) {
+        const uint4 f = fixed[first + min((uint32_t)p, cnt - 1u)];
+        px[p] = (float)(int32_t)(f.x - ref.x) * sx;
+        py[p] = (float)(int32_t)(f.y - ref.y) * sy;
+        pz[p] = (float)(int32_t)(f.z - ref.z) * sz;
+        n[p] = 0u;
+    }
+    uint32_t q = 0u;
+    const auto slot_of = [&](uint32_t c) -> uint32_t {
+        while (range[q + 1u].x <= c) ++q;
+        const uint2 r = range[q];
+        return r.y + (c - r.x);
+    };
+    uint32_t j = lane < total ? slot_of(lane) : 0u;
+    uint4 w = fixed[j];
+    for (uint32_t c0 = 0; c0 < total; c0 += 32u) {
+        const bool on = c0 + lane < total;
+        const uint4 wc = w;
+        const uint32_t jc = j;
+        if (c0 + 32u + lane < total) {
+            j = slot_of(c0 + 32u + lane);
+            w = fixed[j];
+        }
+        const float qx = (float)(int32_t)(wc.x - ref.x) * sx;
+        const float qy = (float)(int32_t)(wc.y - ref.y) * sy;
+        const float qz = (float)(int32_t)(wc.z - ref.z) * sz;
+        // a lane without a candidate hits nothing
+        const float hi_l = on ? hi : -1.0f;
+#pragma unroll
+        for (int p = 0; p < B_CHUNK; ++p) {
+            if (p >= (int)cnt) break;
+            float dx = px[p] - qx, dy = py[p] - qy, dz = pz[p] - qz;
+            if constexpr (WRAP) {
+                dx = fmaf(-Lx, rintf(dx * ix), dx);
+                dy = fmaf(-Ly, rintf(dy * iy), dy);
+                dz = fmaf(-Lz, rintf(dz * iz), dz);
             }
+            const float rs = dx * dx + dy * dy + dz * dz;
+            const uint32_t i = first + (uint32_t)p;
+            bool hit = (rs < hi_l) & (jc != i);
+            if (hit && !(rs < lo)) {
+                // inside the band: the exact FP64 decision
+                const double4_32a pi = pos[i];
+                const double4_32a pj = pos[jc];
+                const double vx = min_image1(pi.x - pj.x, si.L[0], si.Linv[0]);
+                const double vy = min_image1(pi.y - pj.y, si.L[1], si.Linv[1]);
+                const double vz = min_image1(pi.z - pj.z, si.L[2], si.Linv[2]);
+                hit = rsq_exact(vx, vy, vz) < si.rlistsq;
+            }
+            const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+            const uint32_t k = n[p] + __popc(hits & lt);
+            if (hit && k < max_nn) nbrs[(size_t)i * width + k] = jc;
+            n[p] += __popc(hits);
         }
     }
-    counts[i] = n;
-    if (n > max_nn) atomicMax(maxcount, n);
+    uint32_t mine = 0u;
+#pragma unroll
+    for (int p = 0; p < B_CHUNK; ++p)
+        if (p == (int)lane) mine = n[p];
+    return mine;
+}
+
+__global__ void __launch_bounds__(B_NL_WARPS * 32)
+    k_b_nlist(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed, uint32_t N,
+              const SysInfo* __restrict__ info, const uint32_t* __restrict__ cell_start,
+              const uint32_t* __restrict__ cell_of, uint32_t* __restrict__ counts, uint32_t* __restrict__ nbrs,
+              uint32_t width, uint32_t max_nn, uint32_t* __restrict__ maxcount, const uint32_t* __restrict__ gate)
+{
+    if (gated_off(gate)) return;
+    __shared__ uint2 s_range[B_NL_WARPS][B_RANGES + 1];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint2* range = s_range[warp];
+    const uint32_t s_begin = (blockIdx.x * B_NL_WARPS + warp) * B_CHUNK;
+    if (s_begin >= N) return;
+    const uint32_t s_end = min(s_begin + B_CHUNK, N);
+    for (uint32_t sa = s_begin; sa < s_end;) {
+        // the particles from sa on that share its cell (and with it the replica)
+        const uint32_t my_cell = cell_of[min(sa + lane, s_end - 1u)];
+        const uint32_t cc = __shfl_sync(0xffffffffu, my_cell, 0);
+        const uint32_t same = __ballot_sync(0xffffffffu, my_cell == cc && sa + lane < s_end);
+        const uint32_t cnt = (uint32_t)__ffs(~same) - 1u;  // B_CHUNK < 32: some lane is off
+        const SysInfo& si = info[fixed[sa].w];
+        const int ncx = si.dim[0], ncy = si.dim[1], ncz = si.dim[2];
+        const int r0 = si.reach[0], r1 = si.reach[1], r2 = si.reach[2];
+        const uint32_t c = cc - si.cell_off;
+        const int cx = (int)(c % (uint32_t)ncx);
+        const int cy = (int)((c / (uint32_t)ncx) % (uint32_t)ncy);
+        const int cz = (int)(c / ((uint32_t)ncx * (uint32_t)ncy));
+        // the x-cells of a stencil row in their order: one slot range, or two at a face
+        const int x0 = cx - r0, x1 = cx + r0;
+        const int b0 = x0 < 0 ? ncx + x0 : x0, e0 = x0 < 0 || x1 >= ncx ? ncx - 1 : x1;
+        const int e1 = x1 >= ncx ? x1 - ncx : x1;  // the second range begins at cell 0
+        const uint32_t parts = x0 < 0 || x1 >= ncx ? 2u : 1u;
+        const uint32_t ny = 2u * r1 + 1u;
+        const uint32_t nr = ny * (2u * r2 + 1u) * parts;
+        uint32_t total = 0u;
+        for (uint32_t q0 = 0; q0 < nr; q0 += 32u) {
+            const uint32_t q = q0 + lane;
+            uint32_t sb = 0u, len = 0u;
+            if (q < nr) {
+                const uint32_t row = q / parts, part = q - row * parts;
+                int oz = cz - r2 + (int)(row / ny), oy = cy - r1 + (int)(row % ny);
+                oz += (oz < 0) ? ncz : 0;
+                oz -= (oz >= ncz) ? ncz : 0;
+                oy += (oy < 0) ? ncy : 0;
+                oy -= (oy >= ncy) ? ncy : 0;
+                const uint32_t rb = si.cell_off + ((uint32_t)oz * ncy + oy) * ncx;
+                sb = cell_start[rb + (part ? 0 : b0)];
+                len = cell_start[rb + (part ? e1 : e0) + 1] - sb;
+            }
+            uint32_t sum = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+                if ((int)lane >= o) sum += v;
+            }
+            if (q < nr) range[q] = make_uint2(total + sum - len, sb);
+            total += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0u) range[nr] = make_uint2(0xffffffffu, 0u);
+        __syncwarp();
+        const uint32_t n = si.far_cells ? b_walk<false>(fixed, pos, si, range, total, sa, cnt, nbrs, width, max_nn)
+                                        : b_walk<true>(fixed, pos, si, range, total, sa, cnt, nbrs, width, max_nn);
+        if (lane < cnt) {
+            counts[sa + lane] = n;
+            if (n > max_nn) atomicMax(maxcount, n);
+        }
+        __syncwarp();
+        sa += cnt;
+    }
 }
 
 __global__ void k_b_finish(uint32_t* __restrict__ flags, const uint32_t* __restrict__ gate)
@@ -266,7 +366,7 @@ struct BStep {
     uint32_t N;
     const uint32_t* counts;
     const uint32_t* nbrs;
-    uint32_t max_nn;
+    uint32_t max_nn, width;
     double dt, kT, gamma, noise;
     int noiseless;
     FlowD flow;
@@ -275,7 +375,8 @@ struct BStep {
     uint32_t* flags;
     float disp_thresh2;
     int next;
-    int tpp;
+    const uint2* work;  // per block: (replica | log2 of the lanes per particle << 16, first particle)
+    uint32_t blocks;
     int block;  // threads per block of the launch
     cudaGraphConditionalHandle next_cond;
     int set_cond;
@@ -286,28 +387,70 @@ struct BStep {
 #define AZP_B_BATCH 4
 #endif
 constexpr int B_BATCH = AZP_B_BATCH;
-
+// blocks of BATCH_BLOCK_MAX threads an SM holds (64 registers a thread at 2): the FP32
+// step of the light evaluators is 1.3 times faster at 2 than at the 70 or so registers the
+// compiler takes at 1 (7.2 against 9.3 ms for 20 steps of 48 replicas); the others would spill
 template<class PE, typename R>
-__global__ void __launch_bounds__(BATCH_BLOCK_MAX) k_b_step(BStep a)
+constexpr int b_min_blocks()
 {
-    const int tpp = a.tpp;
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t i = gid / tpp;
-    const uint32_t sub = gid % tpp;
-    const bool active = i < a.N;
-    R fx = 0, fy = 0, fz = 0;
-    Comp cx{0.f, 0.f}, cy{0.f, 0.f}, cz{0.f, 0.f};
-    const SysInfo* si = active ? a.info + a.sys[i] : a.info;
-    if (active) {
-        R rec[PAIR_TBL];
+    return std::is_same<R, float>::value && !std::is_same<PE, Colloid>::value ? 2 : 1;
+}
+
+// particles a block of `block` threads takes at 2^lt lanes each: all its threads at once,
+// but at least a warp's worth, so that the integration runs on full warps
+AZP_HD uint32_t b_block_particles(uint32_t block, uint32_t lt) { return block >> lt > 32u ? block >> lt : 32u; }
+
+// FP32 step: 2^B_LT lanes evaluate the pairs of a particle, B_TERMS entries of its row a
+// pass, and leave their terms in shared memory; one lane per particle and axis then adds
+// them in list order. The compensated addition is not free of its order (its product is
+// fused into the first sum only), so the split of the evaluation leaves the force, and with
+// it the trajectory, as one lane walking the row has it.
+constexpr uint32_t B_LT = 2;
+constexpr uint32_t B_TERMS = B_BATCH << B_LT;
+constexpr uint32_t B_WARP_P = 32u >> B_LT;             // particles of a warp
+constexpr uint32_t B_TERM_ROW = B_TERMS * 4u + 4u;     // floats: (dx, dy, dz, f / r) and a pad against bank conflicts
+constexpr size_t b_step_smem(uint32_t block) { return (size_t)(block / 32u) * B_WARP_P * B_TERM_ROW * sizeof(float); }
+static_assert(3 * B_WARP_P <= 32, "a lane per particle and axis");
+static_assert(B_TERM_ROW % 4 == 0, "rows of 16-byte terms");
+
+// The fused step. A block takes particles of one replica; 2^lt lanes of a warp walk the
+// row of one particle, in passes over the block's particles, and its first threads
+// integrate them. Replicas differ by two orders of magnitude in the entries of a row; in
+// FP64 lt belongs to the replica (b_plan).
+// One thread per particle took 1,200 us a step for 48 replicas (94 M entries in FP32; its
+// last warps walked 2,800 entries each, one lane a row), this 390. Bound by issue
+// (about 100 instructions an entry) and the latency of the gathers.
+template<class PE, typename R>
+__global__ void __launch_bounds__(BATCH_BLOCK_MAX, (b_min_blocks<PE, R>())) k_b_step(BStep a)
+{
+    __shared__ R s_force[3][BATCH_BLOCK_MAX];
+    extern __shared__ __align__(16) float s_terms[];
+    const uint2 work = a.work[blockIdx.x];
+    const SysInfo* si = a.info + (work.x & 0xffffu);
+    const uint32_t lt = work.x >> 16;
+    const uint32_t tpp = 1u << lt;
+    const uint32_t np = min(b_block_particles(blockDim.x, lt), si->off + si->n - work.y);
+    const uint32_t sub = threadIdx.x & (tpp - 1u);
+    R rec[PAIR_TBL];
 #pragma unroll
-        for (int k = 0; k < PAIR_TBL; ++k) rec[k] = (R)si->rec[k];
-        const bool on = PE::enabled(rec);
-        const uint32_t n = on ? min(a.counts[i], a.max_nn) : 0u;
+    for (int k = 0; k < PAIR_TBL; ++k) {
+        if constexpr (std::is_same<R, double>::value)
+            rec[k] = si->rec[k];
+        else
+            rec[k] = si->recf[k];
+    }
+    const bool on = PE::enabled(rec);
+    for (uint32_t first = 0; first < np; first += blockDim.x >> lt) {
+        const uint32_t q = first + (threadIdx.x >> lt);
+        const bool active = q < np;
+        const uint32_t i = work.y + (active ? q : 0u);
+        const uint32_t n = active && on ? min(a.counts[i], a.max_nn) : 0u;
+        const uint32_t* row = a.nbrs + (size_t)i * a.width;
+        [[maybe_unused]] R fx = 0, fy = 0, fz = 0;
         if constexpr (std::is_same<R, double>::value) {
             const double4_32a pi = a.pos[i];
             for (uint32_t k = sub; k < n; k += tpp) {
-                const uint32_t j = a.nbrs[(size_t)k * a.N + i];
+                const uint32_t j = row[k];
                 const double4_32a pj = a.pos[j];
                 const double dx = min_image1(pi.x - pj.x, si->L[0], si->Linv[0]);
                 const double dy = min_image1(pi.y - pj.y, si->L[1], si->Linv[1]);
@@ -322,59 +465,84 @@ __global__ void __launch_bounds__(BATCH_BLOCK_MAX) k_b_step(BStep a)
             }
         } else {
             const uint4 fi = a.fix[i];
-            const float rc2 = (float)si->rcutsq;
-            // neighbours in batches of B_BATCH: the list entries of a batch first,
-            // then their fixed-point words, so that B_BATCH gathers are in flight;
-            // the pairs are then added in list order as one at a time would
-            const uint32_t* col = a.nbrs + i;
-            for (uint32_t kb = sub; kb < n; kb += B_BATCH * tpp) {
+            const float rc2 = si->rcutf;
+            const float rc_lo = rc2 * 0.999996f, rc_hi = rc2 * 1.000004f;
+            const float sx = si->sfix[0], sy = si->sfix[1], sz = si->sfix[2];
+            const uint32_t lane = threadIdx.x & 31u;
+            float* rows = s_terms + (threadIdx.x >> 5) * (B_WARP_P * B_TERM_ROW);
+            float4* put = reinterpret_cast<float4*>(rows + (lane >> B_LT) * B_TERM_ROW) + sub;
+            const float* get = rows + lane / 3u * B_TERM_ROW;
+            const uint32_t axis = lane % 3u;
+            const uint32_t nmax = __reduce_max_sync(0xffffffffu, n);
+            Comp sum{0.f, 0.f};
+            // the words of a pass gathered together, the list entries of the next loaded
+            // meanwhile; the evaluator runs on every lane, at r_cut where a pair does not
+            // count, so that the pairs of a lane overlap
+            uint32_t jn[B_BATCH];
+#pragma unroll
+            for (int u = 0; u < B_BATCH; ++u) {
+                const uint32_t k = sub + ((uint32_t)u << B_LT);
+                jn[u] = k < n ? __ldg(row + k) : i;
+            }
+            for (uint32_t kb = 0; kb < nmax; kb += B_TERMS) {
                 uint32_t jj[B_BATCH];
                 uint4 fj[B_BATCH];
 #pragma unroll
-                for (int u = 0; u < B_BATCH; ++u) {
-                    const uint32_t k = kb + u * tpp;
-                    jj[u] = k < n ? __ldg(col + (size_t)k * a.N) : i;
-                }
+                for (int u = 0; u < B_BATCH; ++u) jj[u] = jn[u];
 #pragma unroll
                 for (int u = 0; u < B_BATCH; ++u) fj[u] = __ldg(a.fix + jj[u]);
 #pragma unroll
                 for (int u = 0; u < B_BATCH; ++u) {
-                    if (kb + u * tpp >= n) break;
-                    const float dx = (float)(int32_t)(fi.x - fj[u].x) * si->sfix[0];
-                    const float dy = (float)(int32_t)(fi.y - fj[u].y) * si->sfix[1];
-                    const float dz = (float)(int32_t)(fi.z - fj[u].z) * si->sfix[2];
+                    const uint32_t k = kb + B_TERMS + sub + ((uint32_t)u << B_LT);
+                    jn[u] = k < n ? __ldg(row + k) : i;
+                }
+#pragma unroll
+                for (int u = 0; u < B_BATCH; ++u) {
+                    const float dx = (float)(int32_t)(fi.x - fj[u].x) * sx;
+                    const float dy = (float)(int32_t)(fi.y - fj[u].y) * sy;
+                    const float dz = (float)(int32_t)(fi.z - fj[u].z) * sz;
                     const float rsq = dx * dx + dy * dy + dz * dz;
-                    if (rsq >= rc2 * 1.000004f) continue;
-                    if (rsq >= rc2 * 0.999996f) {
+                    bool in = rsq < rc_hi && jj[u] != i;
+                    if (in && rsq >= rc_lo) {
                         const double4_32a pi = a.pos[i];
                         const double4_32a pj = a.pos[jj[u]];
                         const double vx = min_image1(pi.x - pj.x, si->L[0], si->Linv[0]);
                         const double vy = min_image1(pi.y - pj.y, si->L[1], si->Linv[1]);
                         const double vz = min_image1(pi.z - pj.z, si->L[2], si->Linv[2]);
-                        if (!(rsq_exact(vx, vy, vz) < si->rcutsq)) continue;
+                        in = rsq_exact(vx, vy, vz) < si->rcutsq;
                     }
                     float fdr, e;
-                    PE::eval(rec, rsq, fdr, e);
-                    cx.add(dx * fdr);
-                    cy.add(dy * fdr);
-                    cz.add(dz * fdr);
+                    PE::eval(rec, in ? rsq : rc2, fdr, e);
+                    put[u << B_LT] = make_float4(dx, dy, dz, in ? fdr : 0.0f);
                 }
+                __syncwarp();
+                if (lane < 3u * B_WARP_P) {
+#pragma unroll
+                    for (uint32_t m = 0; m < B_TERMS; ++m) sum.add(get[4u * m + axis] * get[4u * m + 3u]);
+                }
+                __syncwarp();
+            }
+            const uint32_t qs = first + (threadIdx.x >> 5) * B_WARP_P + lane / 3u;
+            if (lane < 3u * B_WARP_P && qs < np) s_force[axis][qs] = sum.value();
+        }
+        if constexpr (std::is_same<R, double>::value) {
+            for (uint32_t m = tpp >> 1; m > 0; m >>= 1) {
+                fx += __shfl_xor_sync(0xffffffffu, fx, m);
+                fy += __shfl_xor_sync(0xffffffffu, fy, m);
+                fz += __shfl_xor_sync(0xffffffffu, fz, m);
+            }
+            if (active && sub == 0) {
+                s_force[0][q] = fx;
+                s_force[1][q] = fy;
+                s_force[2][q] = fz;
             }
         }
     }
-    for (int m = tpp >> 1; m > 0; m >>= 1) {
-        if constexpr (std::is_same<R, double>::value) {
-            fx += __shfl_xor_sync(0xffffffffu, fx, m);
-            fy += __shfl_xor_sync(0xffffffffu, fy, m);
-            fz += __shfl_xor_sync(0xffffffffu, fz, m);
-        } else {
-            comp_shfl_add(cx, m);
-            comp_shfl_add(cy, m);
-            comp_shfl_add(cz, m);
-        }
-    }
+    __syncthreads();
     bool want = false;
-    if (active && sub == 0) {
+    if (threadIdx.x < np) {
+        const uint32_t i = work.y + threadIdx.x;
+        const R fx = s_force[0][threadIdx.x], fy = s_force[1][threadIdx.x], fz = s_force[2][threadIdx.x];
         const unsigned long long ts = *a.d_ts;
         double4_32a p = a.pos[i];
         double4_32a v = a.vel[i];
@@ -415,9 +583,9 @@ __global__ void __launch_bounds__(BATCH_BLOCK_MAX) k_b_step(BStep a)
             float r0, r1, r2;
             uniform3f(AZP_RNG_LANGEVIN_FLOW, ts, si->seed, tg, -c, 2.0f * c, r0, r1, r2);
             const float minv = __frcp_rn((float)v.w);
-            const float ax = (cx.value() + (r0 - g * ((float)v.x - ux))) * minv;
-            const float ay = (cy.value() + (r1 - g * ((float)v.y - uy))) * minv;
-            const float az = (cz.value() + (r2 - g * ((float)v.z - uz))) * minv;
+            const float ax = (fx + (r0 - g * ((float)v.x - ux))) * minv;
+            const float ay = (fy + (r1 - g * ((float)v.y - uy))) * minv;
+            const float az = (fz + (r2 - g * ((float)v.z - uz))) * minv;
             if (a.next) {
                 const float kx = dt * ax, ky = dt * ay, kz = dt * az;
                 p.x += (double)(((float)v.x + kx) * dt);
@@ -567,12 +735,11 @@ __global__ void k_b_store(const double4_32a* __restrict__ pos, const double4_32a
 template<class PE>
 int launch_b_step(int precision, const BStep& a, cudaStream_t s)
 {
-    const uint32_t blocks = (uint32_t)(((size_t)a.N * a.tpp + a.block - 1) / a.block);
-    if (blocks == 0) return AZP_OK;
+    if (a.blocks == 0) return AZP_OK;
     if (precision == AZP_FP32)
-        k_b_step<PE, float><<<blocks, a.block, 0, s>>>(a);
+        k_b_step<PE, float><<<a.blocks, a.block, b_step_smem((uint32_t)a.block), s>>>(a);
     else
-        k_b_step<PE, double><<<blocks, a.block, 0, s>>>(a);
+        k_b_step<PE, double><<<a.blocks, a.block, 0, s>>>(a);
     AZP_CHECK_LAUNCH("k_b_step");
     return AZP_OK;
 }
@@ -596,6 +763,9 @@ struct azp_batch {
     uint32_t S = 0, N = 0;
     std::vector<uint32_t> n_of, off;
     int precision = AZP_FP64, kind = 0, tpp = 1, block = BATCH_BLOCK;
+    std::vector<double> row_len;  // expected list entries per particle, by replica
+    uint2* work = nullptr;        // blocks of the fused step (b_plan), for block and tpp as they are
+    uint32_t work_blocks = 0;
     double dt = 0.005, kT = 1.0, gamma = 1.0, r_buff = 0.4;
     int noiseless = 0;
     FlowD flow{};
@@ -656,12 +826,55 @@ void b_free(azp_batch* b)
     void* ptrs[] = {b->info, b->sys_off, b->pos[0], b->pos[1], b->fix[0], b->fix[1], b->fix_build, b->vel, b->accel,
                     b->image, b->tag, b->sys, b->t_pos, b->t_vel, b->t_accel, b->t_image, b->t_tag, b->t_sys,
                     b->t_cell, b->cell_of, b->slot, b->cell_count, b->cell_start, b->members, b->scan_tmp,
-                    b->rindex, b->counts, b->nbrs, b->flags, b->d_ts};
+                    b->rindex, b->counts, b->nbrs, b->flags, b->d_ts, b->work};
     for (void* p : ptrs) cudaFree(p);
     if (b->gstream) cudaStreamDestroy(b->gstream);
 }
 
 uint32_t nblk(uint32_t n) { return (n + 255) / 256; }
+
+// words of a particle's list row: rows begin on 32-byte sectors
+uint32_t b_width(uint32_t max_nn) { return (max_nn + 7u) & ~7u; }
+
+// The blocks of the fused step, for the batch's block size and lanes per particle. FP32:
+// 2^B_LT lanes. FP64: a replica takes the smallest power of two at which a lane walks at
+// most per_lane entries of a row, 4 or more (narrower reads of a row waste its sectors),
+// b->tpp or more; per_lane is 128, where fewer sums are combined and the rows of a warp are
+// read together, and less while the lanes would not fill a quarter of the chip. Replicas
+// with the longest rows go first, so that the last blocks are short.
+int b_plan(azp_batch* b)
+{
+    int dev = 0, sms = 1;
+    AZP_CUDA_TRY(cudaGetDevice(&dev));
+    AZP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    double per_lane = 128.0;
+    const auto lanes_log2 = [&](uint32_t r) {
+        uint32_t lt = B_LT;
+        if (b->precision == AZP_FP32) return lt;
+        while (lt < 5 && (b->row_len[r] > per_lane * (1u << lt) || (1 << lt) < b->tpp)) ++lt;
+        return lt;
+    };
+    for (; per_lane > 8.0; per_lane *= 0.5) {
+        size_t lanes = 0;
+        for (uint32_t r = 0; r < b->S; ++r) lanes += (size_t)b->n_of[r] << lanes_log2(r);
+        if (lanes >= (size_t)sms * 512) break;
+    }
+    std::vector<uint32_t> order(b->S);
+    for (uint32_t r = 0; r < b->S; ++r) order[r] = r;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return b->row_len[x] > b->row_len[y]; });
+    std::vector<uint2> work;
+    for (uint32_t r : order) {
+        const uint32_t lt = lanes_log2(r);
+        const uint32_t per = b_block_particles((uint32_t)b->block, lt);
+        for (uint32_t k = 0; k < b->n_of[r]; k += per) work.push_back(make_uint2(r | lt << 16, b->off[r] + k));
+    }
+    cudaFree(b->work);
+    const int st = balloc(&b->work, work.size());
+    if (st) return st;
+    AZP_CUDA_TRY(cudaMemcpy(b->work, work.data(), sizeof(uint2) * work.size(), cudaMemcpyHostToDevice));
+    b->work_blocks = (uint32_t)work.size();
+    return AZP_OK;
+}
 
 int b_rebuild(azp_batch* b, cudaStream_t s, const uint32_t* gate)
 {
@@ -697,8 +910,10 @@ int b_rebuild(azp_batch* b, cudaStream_t s, const uint32_t* gate)
     k_b_gather<<<nblk(N), 256, 0, s>>>(p, gate);
     k_b_back<<<nblk(N), 256, 0, s>>>(p, gate);
     k_b_fixed<<<nblk(N), 256, 0, s>>>(b->pos[b->cur], b->sys, N, b->info, b->fix[b->cur], b->fix_build, gate);
-    k_b_nlist<<<(N + 127) / 128, 128, 0, s>>>(b->pos[b->cur], b->fix[b->cur], b->sys, N, b->info, b->cell_start,
-                                              b->cell_of, b->counts, b->nbrs, b->max_nn, b->flags + 3, gate);
+    constexpr uint32_t per_block = B_NL_WARPS * B_CHUNK;
+    k_b_nlist<<<(N + per_block - 1) / per_block, B_NL_WARPS * 32, 0, s>>>(
+        b->pos[b->cur], b->fix[b->cur], N, b->info, b->cell_start, b->cell_of, b->counts, b->nbrs, b_width(b->max_nn),
+        b->max_nn, b->flags + 3, gate);
     k_b_finish<<<1, 1, 0, s>>>(b->flags, gate);
     AZP_CHECK_LAUNCH("b_rebuild");
     b->launches += 12;
@@ -734,7 +949,9 @@ BStep b_args(azp_batch* b)
     a.flags = b->flags;
     const double half = 0.5 * b->r_buff;
     a.disp_thresh2 = (float)(half * half * (1.0 - 1e-5));
-    a.tpp = b->tpp;
+    a.width = b_width(b->max_nn);
+    a.work = b->work;
+    a.blocks = b->work_blocks;
     a.block = b->block;
     return a;
 }
@@ -871,7 +1088,14 @@ azp_batch* azp_batch_create(const azp_batch_config* c, int* status)
         si.list_lo = cut.lo;
         si.list_hi = cut.hi;
         si.rlistsq = cut.rlistsq;
+        const double volume = box.L[0] * box.L[1] * box.L[2];
         const CellGrid g = make_grid(box, rmax);
+        b->row_len.push_back(std::min((double)c->N[r], c->N[r] / volume * 4.18879 * rmax * rmax * rmax));
+        si.off = b->off[r];
+        si.n = c->N[r];
+        si.far_cells = 1u;
+        for (int d = 0; d < 3; ++d)
+            if (g.dim[d] < 2 * g.reach[d] + 3) si.far_cells = 0u;
         si.cell_off = cell_off;
         for (int d = 0; d < 3; ++d) {
             si.dim[d] = g.dim[d];
@@ -889,6 +1113,8 @@ azp_batch* azp_batch_create(const azp_batch_config* c, int* status)
         for (int k = 0; k < PAIR_TBL; ++k) si.rec[k] = rec[k];
         // the evaluator subtracts the shift itself in the single-system kernel; here fold it
         si.rcutsq = rec[PAIR_REC];
+        for (int k = 0; k < PAIR_TBL; ++k) si.recf[k] = (float)rec[k];
+        si.rcutf = (float)si.rcutsq;
     }
     b->ncell = cell_off;
     const uint32_t N = b->N;
@@ -925,7 +1151,7 @@ azp_batch* azp_batch_create(const azp_batch_config* c, int* status)
     BALLOC(b->cell_start, (size_t)b->ncell + 1);
     BALLOC(b->scan_tmp, scan_tmp_words(b->ncell));
     BALLOC(b->counts, N);
-    BALLOC(b->nbrs, (size_t)N * b->max_nn);
+    BALLOC(b->nbrs, (size_t)N * b_width(b->max_nn));
     BALLOC(b->flags, 8);
     BALLOC(b->d_ts, 1);
 #undef BALLOC
@@ -934,6 +1160,8 @@ azp_batch* azp_batch_create(const azp_batch_config* c, int* status)
         cudaMemset(b->flags, 0, sizeof(uint32_t) * 8) != cudaSuccess ||
         cudaStreamCreateWithFlags(&b->gstream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(record_cuda_error(cudaGetLastError(), "batch set-up"), b);
+    st = b_plan(b);
+    if (st) return fail(st, b);
     if (status) *status = AZP_OK;
     return b;
 }
@@ -993,7 +1221,7 @@ int azp_batch_set_state(azp_batch* b, const double* pos, const double* vel, cons
         if (need <= b->max_nn) break;
         cudaFree(b->nbrs);
         b->max_nn = (uint32_t)std::ceil(need * 1.3) + 8;
-        st = balloc(&b->nbrs, (size_t)N * b->max_nn);
+        st = balloc(&b->nbrs, (size_t)N * b_width(b->max_nn));
         if (st) break;
         b_free_graphs(b);
     }
@@ -1013,23 +1241,15 @@ int azp_batch_get_state(azp_batch* b, double* pos, double* vel, double* accel, i
     if (!b || !b->have_state || !pos || !vel || !accel || !image) return AZP_ERR_INVALID;
     cudaStream_t s = as_stream(stream);
     const uint32_t N = b->N;
-    double *dp, *dv, *da;
-    int* di;
-    AZP_CUDA_TRY(cudaMalloc(&dp, sizeof(double) * 4 * N));
-    AZP_CUDA_TRY(cudaMalloc(&dv, sizeof(double) * 4 * N));
-    AZP_CUDA_TRY(cudaMalloc(&da, sizeof(double) * 3 * N));
-    AZP_CUDA_TRY(cudaMalloc(&di, sizeof(int) * 3 * N));
+    // packed in the rebuild's temporaries, which hold nothing between rebuilds
+    double *dp = reinterpret_cast<double*>(b->t_pos), *dv = reinterpret_cast<double*>(b->t_vel);
     k_b_store<<<nblk(N), 256, 0, s>>>(b->pos[b->cur], b->vel, b->accel, b->image, b->tag, b->sys, b->sys_off, N, dp, dv,
-                                      da, di);
+                                      b->t_accel, b->t_image);
     AZP_CUDA_TRY(cudaMemcpyAsync(pos, dp, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, s));
     AZP_CUDA_TRY(cudaMemcpyAsync(vel, dv, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, s));
-    AZP_CUDA_TRY(cudaMemcpyAsync(accel, da, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, s));
-    AZP_CUDA_TRY(cudaMemcpyAsync(image, di, sizeof(int) * 3 * N, cudaMemcpyDeviceToHost, s));
+    AZP_CUDA_TRY(cudaMemcpyAsync(accel, b->t_accel, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, s));
+    AZP_CUDA_TRY(cudaMemcpyAsync(image, b->t_image, sizeof(int) * 3 * N, cudaMemcpyDeviceToHost, s));
     AZP_CUDA_TRY(cudaStreamSynchronize(s));
-    cudaFree(dp);
-    cudaFree(dv);
-    cudaFree(da);
-    cudaFree(di);
     return AZP_OK;
 }
 
@@ -1089,17 +1309,19 @@ int azp_batch_error(azp_batch* b, uint32_t* err_word, uint32_t* n_builds, void* 
 int azp_batch_set_block(azp_batch* b, int block)
 {
     if (!b || !(block == 64 || block == 128 || block == 256 || block == 512)) return AZP_ERR_INVALID;
-    if (b->block != block) b_free_graphs(b);
+    if (b->block == block) return AZP_OK;
+    b_free_graphs(b);
     b->block = block;
-    return AZP_OK;
+    return b_plan(b);
 }
 
 int azp_batch_set_tpp(azp_batch* b, int tpp)
 {
     if (!b || !(tpp == 1 || tpp == 2 || tpp == 4 || tpp == 8 || tpp == 16 || tpp == 32)) return AZP_ERR_INVALID;
-    if (b->tpp != tpp) b_free_graphs(b);
+    if (b->tpp == tpp) return AZP_OK;
+    b_free_graphs(b);
     b->tpp = tpp;
-    return AZP_OK;
+    return b_plan(b);
 }
 
 uint64_t azp_batch_last_launches(const azp_batch* b) { return b ? b->launches : 0; }

@@ -13,6 +13,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fp32.cuh"
 #include "fp64.cuh"
 #include <math.h>
 #include <type_traits>
@@ -135,6 +136,18 @@ struct ExpandedYukawa {
     template<typename R> AZP_HD static bool enabled(const R* rec) { return rec[0] != R(0); }
     template<typename R> AZP_HD static void eval(const R* rec, R rsq, R& fdr, R& e)
     {
+#ifdef __CUDA_ARCH__
+        if constexpr (std::is_same<R, float>::value) {
+            float r, rinv;
+            f_root(rsq, r, rinv);
+            const float s = r - rec[2];
+            const float sinv = f_rcp(s);
+            const float u = rec[0] * expf(-rec[1] * s) * sinv;
+            fdr = f_over(u * (rec[1] + sinv), r, rinv);
+            e = u;
+            return;
+        }
+#endif
         const R r = root(rsq);
         const R s = r - rec[2];
         const R sinv = rcp(s);
