@@ -187,14 +187,25 @@ __global__ void k_b_fixed(const double4_32a* __restrict__ pos, const uint16_t* _
 // (make_list_cuts, 5e-6) covers: both coordinates' roundings come to 2.1e-6 of r^2.
 // Bound by issue (14 or 23 instructions a test). One thread per particle and a column of
 // the list each took 1,010 us for 48 replicas (337,467 particles, 94 M entries), with
-// 32 lanes on rows of 15 to 2,800 entries; this takes 490.
+// 32 lanes on rows of 15 to 2,800 entries; this takes 565.
 constexpr int B_CHUNK = 8;
+// The list: entry k of particle i. Blocks of 16 entries, the particles' side by side: a
+// pass of the step reads one block of each of its particles, and what is in use of the
+// list is compact whatever the longest row. Whole rows one after the other, at 3,700
+// entries each, spread 0.4 GB of entries over 5 GB and its pages: 390 us a step for 48
+// replicas against 360 so (the list build, which writes a row in several places, takes 565
+// against 490; there are 7 steps to a build).
+constexpr uint32_t B_LIST_BLOCK = 16;
+AZP_D size_t b_entry(uint32_t i, uint32_t k, uint32_t N)
+{
+    return ((size_t)(k / B_LIST_BLOCK) * N + i) * B_LIST_BLOCK + k % B_LIST_BLOCK;
+}
 constexpr int B_NL_WARPS = 4;
 constexpr uint32_t B_RANGES = 2 * 3 * 3;  // stencil rows and their wrapped parts
 template<bool WRAP>
 AZP_D uint32_t b_walk(const uint4* __restrict__ fixed, const double4_32a* __restrict__ pos, const SysInfo& si,
                       const uint2* range, uint32_t total, uint32_t first, uint32_t cnt, uint32_t* __restrict__ nbrs,
-                      uint32_t width, uint32_t max_nn)
+                      uint32_t N, uint32_t max_nn)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt = (1u << lane) - 1u;
@@ -257,7 +268,7 @@ AZP_D uint32_t b_walk(const uint4* __restrict__ fixed, const double4_32a* __rest
             }
             const uint32_t hits = __ballot_sync(0xffffffffu, hit);
             const uint32_t k = n[p] + __popc(hits & lt);
-            if (hit && k < max_nn) nbrs[(size_t)i * width + k] = jc;
+            if (hit && k < max_nn) nbrs[b_entry(i, k, N)] = jc;
             n[p] += __popc(hits);
         }
     }
@@ -272,7 +283,7 @@ __global__ void __launch_bounds__(B_NL_WARPS * 32)
     k_b_nlist(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed, uint32_t N,
               const SysInfo* __restrict__ info, const uint32_t* __restrict__ cell_start,
               const uint32_t* __restrict__ cell_of, uint32_t* __restrict__ counts, uint32_t* __restrict__ nbrs,
-              uint32_t width, uint32_t max_nn, uint32_t* __restrict__ maxcount, const uint32_t* __restrict__ gate)
+              uint32_t max_nn, uint32_t* __restrict__ maxcount, const uint32_t* __restrict__ gate)
 {
     if (gated_off(gate)) return;
     __shared__ uint2 s_range[B_NL_WARPS][B_RANGES + 1];
@@ -327,8 +338,8 @@ __global__ void __launch_bounds__(B_NL_WARPS * 32)
         }
         if (lane == 0u) range[nr] = make_uint2(0xffffffffu, 0u);
         __syncwarp();
-        const uint32_t n = si.far_cells ? b_walk<false>(fixed, pos, si, range, total, sa, cnt, nbrs, width, max_nn)
-                                        : b_walk<true>(fixed, pos, si, range, total, sa, cnt, nbrs, width, max_nn);
+        const uint32_t n = si.far_cells ? b_walk<false>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn)
+                                        : b_walk<true>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn);
         if (lane < cnt) {
             counts[sa + lane] = n;
             if (n > max_nn) atomicMax(maxcount, n);
@@ -366,7 +377,7 @@ struct BStep {
     uint32_t N;
     const uint32_t* counts;
     const uint32_t* nbrs;
-    uint32_t max_nn, width;
+    uint32_t max_nn;
     double dt, kT, gamma, noise;
     int noiseless;
     FlowD flow;
@@ -388,8 +399,9 @@ struct BStep {
 #endif
 constexpr int B_BATCH = AZP_B_BATCH;
 // blocks of BATCH_BLOCK_MAX threads an SM holds (64 registers a thread at 2): the FP32
-// step of the light evaluators is 1.3 times faster at 2 than at the 70 or so registers the
-// compiler takes at 1 (7.2 against 9.3 ms for 20 steps of 48 replicas); the others would spill
+// step of the light evaluators is faster at 2, a few spilled words and all, than at the 70 or
+// so registers the compiler takes at 1 (20 steps of 48 replicas: 9.3 and 11.2 ms); the others
+// would spill more
 template<class PE, typename R>
 constexpr int b_min_blocks()
 {
@@ -412,13 +424,14 @@ constexpr uint32_t B_TERM_ROW = B_TERMS * 4u + 4u;     // floats: (dx, dy, dz, f
 constexpr size_t b_step_smem(uint32_t block) { return (size_t)(block / 32u) * B_WARP_P * B_TERM_ROW * sizeof(float); }
 static_assert(3 * B_WARP_P <= 32, "a lane per particle and axis");
 static_assert(B_TERM_ROW % 4 == 0, "rows of 16-byte terms");
+static_assert(B_TERMS == B_LIST_BLOCK, "a pass takes a block of the list");
 
 // The fused step. A block takes particles of one replica; 2^lt lanes of a warp walk the
 // row of one particle, in passes over the block's particles, and its first threads
 // integrate them. Replicas differ by two orders of magnitude in the entries of a row; in
 // FP64 lt belongs to the replica (b_plan).
 // One thread per particle took 1,200 us a step for 48 replicas (94 M entries in FP32; its
-// last warps walked 2,800 entries each, one lane a row), this 390. Bound by issue
+// last warps walked 2,800 entries each, one lane a row), this 360. Bound by issue
 // (about 100 instructions an entry) and the latency of the gathers.
 template<class PE, typename R>
 __global__ void __launch_bounds__(BATCH_BLOCK_MAX, (b_min_blocks<PE, R>())) k_b_step(BStep a)
@@ -445,12 +458,11 @@ __global__ void __launch_bounds__(BATCH_BLOCK_MAX, (b_min_blocks<PE, R>())) k_b_
         const bool active = q < np;
         const uint32_t i = work.y + (active ? q : 0u);
         const uint32_t n = active && on ? min(a.counts[i], a.max_nn) : 0u;
-        const uint32_t* row = a.nbrs + (size_t)i * a.width;
         [[maybe_unused]] R fx = 0, fy = 0, fz = 0;
         if constexpr (std::is_same<R, double>::value) {
             const double4_32a pi = a.pos[i];
             for (uint32_t k = sub; k < n; k += tpp) {
-                const uint32_t j = row[k];
+                const uint32_t j = a.nbrs[b_entry(i, k, a.N)];
                 const double4_32a pj = a.pos[j];
                 const double dx = min_image1(pi.x - pj.x, si->L[0], si->Linv[0]);
                 const double dy = min_image1(pi.y - pj.y, si->L[1], si->Linv[1]);
@@ -478,11 +490,12 @@ __global__ void __launch_bounds__(BATCH_BLOCK_MAX, (b_min_blocks<PE, R>())) k_b_
             // the words of a pass gathered together, the list entries of the next loaded
             // meanwhile; the evaluator runs on every lane, at r_cut where a pair does not
             // count, so that the pairs of a lane overlap
+            const uint32_t* block = a.nbrs + (size_t)i * B_LIST_BLOCK + sub;
             uint32_t jn[B_BATCH];
 #pragma unroll
             for (int u = 0; u < B_BATCH; ++u) {
-                const uint32_t k = sub + ((uint32_t)u << B_LT);
-                jn[u] = k < n ? __ldg(row + k) : i;
+                const uint32_t k = (uint32_t)u << B_LT;
+                jn[u] = k + sub < n ? __ldg(block + k) : i;
             }
             for (uint32_t kb = 0; kb < nmax; kb += B_TERMS) {
                 uint32_t jj[B_BATCH];
@@ -491,10 +504,11 @@ __global__ void __launch_bounds__(BATCH_BLOCK_MAX, (b_min_blocks<PE, R>())) k_b_
                 for (int u = 0; u < B_BATCH; ++u) jj[u] = jn[u];
 #pragma unroll
                 for (int u = 0; u < B_BATCH; ++u) fj[u] = __ldg(a.fix + jj[u]);
+                block += (size_t)a.N * B_LIST_BLOCK;
 #pragma unroll
                 for (int u = 0; u < B_BATCH; ++u) {
-                    const uint32_t k = kb + B_TERMS + sub + ((uint32_t)u << B_LT);
-                    jn[u] = k < n ? __ldg(row + k) : i;
+                    const uint32_t k = (uint32_t)u << B_LT;
+                    jn[u] = kb + B_TERMS + sub + k < n ? __ldg(block + k) : i;
                 }
 #pragma unroll
                 for (int u = 0; u < B_BATCH; ++u) {
@@ -833,12 +847,12 @@ void b_free(azp_batch* b)
 
 uint32_t nblk(uint32_t n) { return (n + 255) / 256; }
 
-// words of a particle's list row: rows begin on 32-byte sectors
-uint32_t b_width(uint32_t max_nn) { return (max_nn + 7u) & ~7u; }
+// words of a particle's list row
+uint32_t b_width(uint32_t max_nn) { return (max_nn + B_LIST_BLOCK - 1u) / B_LIST_BLOCK * B_LIST_BLOCK; }
 
 // The blocks of the fused step, for the batch's block size and lanes per particle. FP32:
 // 2^B_LT lanes. FP64: a replica takes the smallest power of two at which a lane walks at
-// most per_lane entries of a row, 4 or more (narrower reads of a row waste its sectors),
+// most per_lane entries of a row, 4 or more (narrower reads waste the sectors of a block),
 // b->tpp or more; per_lane is 128, where fewer sums are combined and the rows of a warp are
 // read together, and less while the lanes would not fill a quarter of the chip. Replicas
 // with the longest rows go first, so that the last blocks are short.
@@ -912,8 +926,7 @@ int b_rebuild(azp_batch* b, cudaStream_t s, const uint32_t* gate)
     k_b_fixed<<<nblk(N), 256, 0, s>>>(b->pos[b->cur], b->sys, N, b->info, b->fix[b->cur], b->fix_build, gate);
     constexpr uint32_t per_block = B_NL_WARPS * B_CHUNK;
     k_b_nlist<<<(N + per_block - 1) / per_block, B_NL_WARPS * 32, 0, s>>>(
-        b->pos[b->cur], b->fix[b->cur], N, b->info, b->cell_start, b->cell_of, b->counts, b->nbrs, b_width(b->max_nn),
-        b->max_nn, b->flags + 3, gate);
+        b->pos[b->cur], b->fix[b->cur], N, b->info, b->cell_start, b->cell_of, b->counts, b->nbrs, b->max_nn, b->flags + 3, gate);
     k_b_finish<<<1, 1, 0, s>>>(b->flags, gate);
     AZP_CHECK_LAUNCH("b_rebuild");
     b->launches += 12;
@@ -949,7 +962,6 @@ BStep b_args(azp_batch* b)
     a.flags = b->flags;
     const double half = 0.5 * b->r_buff;
     a.disp_thresh2 = (float)(half * half * (1.0 - 1e-5));
-    a.width = b_width(b->max_nn);
     a.work = b->work;
     a.blocks = b->work_blocks;
     a.block = b->block;
