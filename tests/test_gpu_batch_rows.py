@@ -84,6 +84,28 @@ def test_accelerations_of_uneven_replicas(precision, tpp, block):
     b.close()
 
 
+def test_results_that_are_held_stay():
+    from azplugins_gb300.batch import ReplicaBatch
+
+    snaps = _snaps(8)[1:3]
+    b = ReplicaBatch(snaps, az.pair.ExpandedYukawa, [dict(epsilon=1.0, kappa=1.0, delta=0.0)] * 2, [1.6, 2.0], [1, 2],
+                     dt=0.001)
+    held, copies = [], []
+    for k in range(5):
+        b.run(2)
+        arrays = b.get_arrays()
+        # whole sets, and a slice of one array whose set is dropped
+        held.append(arrays if k % 2 else arrays[1][3:9, 1:])
+        copies.append([np.array(x) for x in held[-1]] if k % 2 else np.array(held[-1]))
+        del arrays
+    for h, c in zip(held, copies):
+        for x, y in zip(h, c):
+            assert np.array_equal(x, y)
+    first = b.get_arrays()
+    assert all(np.array_equal(x, y) for x, y in zip(first, b.get_arrays()))
+    b.close()
+
+
 SRC = r"""
 #include "fp32.cuh"
 using namespace azp;
