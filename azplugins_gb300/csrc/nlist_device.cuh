@@ -441,6 +441,7 @@ AZP_D void nlist_chunk(const ListArgs& L, const uint4* words, uint32_t chunk, ui
             }
         }
         band = __any_sync(0xffffffffu, band);
+        __syncwarp();  // the rows' entries, before other lanes read them (a vote orders no memory)
         // compaction, in order, of the rows that may hold what does not belong
         uint32_t kept[CH], kept_max = 0u;
 #pragma unroll
@@ -470,6 +471,7 @@ AZP_D void nlist_chunk(const ListArgs& L, const uint4* words, uint32_t chunk, ui
                         }
                         for (uint32_t x = 0; x < nex; ++x) keep = keep && ld_ro<NC>(ex_keys + (size_t)x * N + i) != e;
                     }
+                    __syncwarp();  // every lane has its entry before one is overwritten
                     const uint32_t mask = __ballot_sync(0xffffffffu, keep);
                     if (keep) {
                         const uint32_t d = m + __popc(mask & lt);
