@@ -80,8 +80,13 @@ AZP_D double d_sqrt(double x)
     return d_sqrt(x, rinv);
 }
 
-// a < b for a >= 0 or NaN, on the bit patterns (a NaN of positive sign, or b < 0: false)
-AZP_D bool less_nonneg(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+// a < b for a >= 0 or NaN of either sign (false) and b >= 0, on the bit patterns. The
+// comparison is unsigned: inf - inf gives a NaN whose sign bit is set, which a signed one
+// would take for less than everything.
+AZP_D bool less_nonneg(double a, double b)
+{
+    return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b);
+}
 
 // |a| > b for b >= 0 (NaN: true)
 AZP_D bool magnitude_above(double a, double b)
