@@ -184,7 +184,9 @@ __global__ void k_b_fixed(const double4_32a* __restrict__ pos, const uint16_t* _
 // floats relative to the chunk's first particle (an integer conversion per candidate, not
 // per test); where an axis has fewer than 2 reach + 3 cells the difference is wrapped once
 // more. |coordinate| <= L / 2 <= 2.5 r_list there, which the band around r_list
-// (make_list_cuts, 5e-6) covers: both coordinates' roundings come to 2.1e-6 of r^2.
+// (make_list_cuts, 5e-6) covers: both coordinates' roundings come to 2.1e-6 of r^2. Chunks
+// with a particle that was clamped into its cell (word_in_cell) form the differences pair by
+// pair.
 // Bound by issue (14 or 23 instructions a test). One thread per particle and a column of
 // the list each took 1,010 us for 48 replicas (337,467 particles, 94 M entries), with
 // 32 lanes on rows of 15 to 2,800 entries; this takes 565.
@@ -202,7 +204,8 @@ AZP_D size_t b_entry(uint32_t i, uint32_t k, uint32_t N)
 }
 constexpr int B_NL_WARPS = 4;
 constexpr uint32_t B_RANGES = 2 * 3 * 3;  // stencil rows and their wrapped parts
-template<bool WRAP>
+constexpr int B_NEAR = 0, B_WRAP = 1, B_PAIR = 2;  // as they are, wrapped once more, or pair by pair
+template<int FORM>
 AZP_D uint32_t b_walk(const uint4* __restrict__ fixed, const double4_32a* __restrict__ pos, const SysInfo& si,
                       const uint2* range, uint32_t total, uint32_t first, uint32_t cnt, uint32_t* __restrict__ nbrs,
                       uint32_t N, uint32_t max_nn)
@@ -249,7 +252,12 @@ AZP_D uint32_t b_walk(const uint4* __restrict__ fixed, const double4_32a* __rest
         for (int p = 0; p < B_CHUNK; ++p) {
             if (p >= (int)cnt) break;
             float dx = px[p] - qx, dy = py[p] - qy, dz = pz[p] - qz;
-            if constexpr (WRAP) {
+            if constexpr (FORM == B_PAIR) {
+                const uint4 f = fixed[first + (uint32_t)p];
+                dx = (float)(int32_t)(f.x - wc.x) * sx;
+                dy = (float)(int32_t)(f.y - wc.y) * sy;
+                dz = (float)(int32_t)(f.z - wc.z) * sz;
+            } else if constexpr (FORM == B_WRAP) {
                 dx = fmaf(-Lx, rintf(dx * ix), dx);
                 dy = fmaf(-Ly, rintf(dy * iy), dy);
                 dz = fmaf(-Lz, rintf(dz * iz), dz);
@@ -338,8 +346,13 @@ __global__ void __launch_bounds__(B_NL_WARPS * 32)
         }
         if (lane == 0u) range[nr] = make_uint2(0xffffffffu, 0u);
         __syncwarp();
-        const uint32_t n = si.far_cells ? b_walk<false>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn)
-                                        : b_walk<true>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn);
+        const uint4 mine = fixed[min(sa + lane, s_end - 1u)];
+        const bool in_cell = lane >= cnt || (word_in_cell(mine.x, cx, ncx) && word_in_cell(mine.y, cy, ncy) &&
+                                             word_in_cell(mine.z, cz, ncz));
+        const uint32_t n = !__all_sync(0xffffffffu, in_cell)
+                               ? b_walk<B_PAIR>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn)
+                           : si.far_cells ? b_walk<B_NEAR>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn)
+                                          : b_walk<B_WRAP>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn);
         if (lane < cnt) {
             counts[sa + lane] = n;
             if (n > max_nn) atomicMax(maxcount, n);

@@ -104,6 +104,19 @@ __device__ __forceinline__ uint32_t cell_of_fixed(const uint4& f, const CellGrid
     return (cz * (uint32_t)g.dim[1] + cy) * (uint32_t)g.dim[0] + cx;
 }
 
+// Whether fixed word w lies in cell c of dim along its axis, or within 2^-8 of a cell
+// beyond its faces: the cell of an FP64 position rounds there otherwise than its word. False
+// for the words of positions that cell_coord clamped into the cell (further out than 1.5 L,
+// or not a number), whose word lies anywhere.
+__device__ __forceinline__ bool word_in_cell(uint32_t w, int c, int dim)
+{
+    const long long one = 1ll << 32, all = (long long)dim << 32, slack = 1ll << 24;
+    long long d = (long long)((uint64_t)(w ^ 0x80000000u) * (uint32_t)dim) - ((long long)c << 32) + slack;
+    if (d < 0) d += all;
+    if (d >= all) d -= all;
+    return d < one + 2 * slack;
+}
+
 // Per type pair thresholds of the list decision (host-built, ntypes^2 entries).
 struct ListCut {
     double rlistsq;  // exact FP64 test: rsq < rlistsq

@@ -6,6 +6,8 @@
 #include "celllist.cuh"
 #include "fixed64.cuh"
 
+#include <type_traits>
+
 namespace azp
 {
 struct BoxArgs {
@@ -227,7 +229,9 @@ AZP_D void nlist_thread(const ListArgs& L, uint32_t i, const ListCut* s_cut, con
 // REF: coordinates as floats relative to the chunk's first particle, so that a test
 // costs no integer conversion (16 a clock and SM); grids with at least 2 reach + 3 cells on
 // every axis, where the minimum image relative to that particle is the pair's for all
-// pairs in range.
+// pairs in range. A position far outside the box or not finite is clamped into some cell:
+// the particles that share a chunk with it are tested pair by pair (word_in_cell); as a
+// candidate it needs nothing, for a word outside the stencil is out of range either way.
 constexpr int NLW_WARPS = 4;
 constexpr uint32_t NLW_ROW = 192;   // entries of a row held in shared memory; the rest go to the list at once
 constexpr uint32_t NLW_RANGES = 2 * 9 * 9;  // stencil rows (reach <= 4) and their wrapped parts
@@ -385,60 +389,72 @@ AZP_D void nlist_chunk(const ListArgs& L, const uint4* words, uint32_t chunk, ui
         if (lane == 0u) range[nr] = make_uint2(0xffffffffu, 0u);
         __syncwarp();
         bool band = false;
-        uint32_t q = 0u;
-        // slot of candidate c (rising by 32 a call)
-        const auto slot_of = [&](uint32_t c) -> uint32_t {
-            while (range[q + 1u].x <= c) ++q;
-            const uint2 r = range[q];
-            return r.y + (c - r.x);
-        };
-        uint32_t sl = lane < total ? slot_of(lane) : 0u;
-        uint4 w = ld_ro<NC>(words + sl);
-        uint32_t j = SORTED ? sl : ld_ro<NC>(members + sl);
-        for (uint32_t c0 = 0; c0 < total; c0 += 32u) {
-            const bool on = c0 + lane < total;
-            const uint4 wc = w;
-            const uint32_t jc = j;
-            if (c0 + 32u + lane < total) {
-                sl = slot_of(c0 + 32u + lane);
-                w = ld_ro<NC>(words + sl);
-                j = SORTED ? sl : ld_ro<NC>(members + sl);
-            }
-            // a lane without a candidate stands outside every radius
-            float qx = 0.0f, qy = 0.0f, qz = on ? 0.0f : INFINITY;
-            if (REF && on) {
-                qx = (float)(int32_t)(wc.x - ref.x) * bx.sfix[0];
-                qy = (float)(int32_t)(wc.y - ref.y) * bx.sfix[1];
-                qz = (float)(int32_t)(wc.z - ref.z) * bx.sfix[2];
-            }
-            const float* hi = s_hi + (ONE_TYPE ? 0u : wc.w);
-            const float* lo_ = s_lo + (ONE_TYPE ? 0u : wc.w);
+        const auto scan = [&](auto by_ref) {
+            uint32_t q = 0u;
+            // slot of candidate c (rising by 32 a call)
+            const auto slot_of = [&](uint32_t c) -> uint32_t {
+                while (range[q + 1u].x <= c) ++q;
+                const uint2 r = range[q];
+                return r.y + (c - r.x);
+            };
+            uint32_t sl = lane < total ? slot_of(lane) : 0u;
+            uint4 w = ld_ro<NC>(words + sl);
+            uint32_t j = SORTED ? sl : ld_ro<NC>(members + sl);
+            for (uint32_t c0 = 0; c0 < total; c0 += 32u) {
+                const bool on = c0 + lane < total;
+                const uint4 wc = w;
+                const uint32_t jc = j;
+                if (c0 + 32u + lane < total) {
+                    sl = slot_of(c0 + 32u + lane);
+                    w = ld_ro<NC>(words + sl);
+                    j = SORTED ? sl : ld_ro<NC>(members + sl);
+                }
+                // a lane without a candidate stands outside every radius
+                float qx = 0.0f, qy = 0.0f, qz = on ? 0.0f : INFINITY;
+                if (by_ref.value && on) {
+                    qx = (float)(int32_t)(wc.x - ref.x) * bx.sfix[0];
+                    qy = (float)(int32_t)(wc.y - ref.y) * bx.sfix[1];
+                    qz = (float)(int32_t)(wc.z - ref.z) * bx.sfix[2];
+                }
+                const float* hi = s_hi + (ONE_TYPE ? 0u : wc.w);
+                const float* lo_ = s_lo + (ONE_TYPE ? 0u : wc.w);
 #pragma unroll
-            for (int p = 0; p < CH; ++p) {
-                if (p >= (int)cnt) break;
-                float ddx, ddy, ddz;
-                if constexpr (REF) {
-                    ddx = px[p] - qx;
-                    ddy = py[p] - qy;
-                    ddz = pz[p] - qz;
-                } else {
-                    ddx = (float)(int32_t)(pw[p].x - wc.x) * bx.sfix[0];
-                    ddy = (float)(int32_t)(pw[p].y - wc.y) * bx.sfix[1];
-                    ddz = (float)(int32_t)(pw[p].z - wc.z) * bx.sfix[2] - qz;
+                for (int p = 0; p < CH; ++p) {
+                    if (p >= (int)cnt) break;
+                    float ddx, ddy, ddz;
+                    if constexpr (by_ref.value) {
+                        ddx = px[p] - qx;
+                        ddy = py[p] - qy;
+                        ddz = pz[p] - qz;
+                    } else {
+                        ddx = (float)(int32_t)(pw[p].x - wc.x) * bx.sfix[0];
+                        ddy = (float)(int32_t)(pw[p].y - wc.y) * bx.sfix[1];
+                        ddz = (float)(int32_t)(pw[p].z - wc.z) * bx.sfix[2] - qz;
+                    }
+                    const float rs = ddx * ddx + ddy * ddy + ddz * ddz;
+                    const bool hit = (rs < (ONE_TYPE ? cut0.hi : hi[pw[p].w])) & (jc != pi[p]);
+                    const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+                    if (hit) {
+                        const uint32_t k = n[p] + __popc(hits & lt);
+                        const bool sure = rs < (ONE_TYPE ? cut0.lo : lo_[pw[p].w]);
+                        const uint32_t e = sure ? jc : (jc | NL_BAND);
+                        band = band || !sure;
+                        if (k < NLW_ROW) rows[p][k] = e;
+                        else if (k < max_nn) nbrs[(size_t)k * N + pi[p]] = e;
+                    }
+                    n[p] += __popc(hits);
                 }
-                const float rs = ddx * ddx + ddy * ddy + ddz * ddz;
-                const bool hit = (rs < (ONE_TYPE ? cut0.hi : hi[pw[p].w])) & (jc != pi[p]);
-                const uint32_t hits = __ballot_sync(0xffffffffu, hit);
-                if (hit) {
-                    const uint32_t k = n[p] + __popc(hits & lt);
-                    const bool sure = rs < (ONE_TYPE ? cut0.lo : lo_[pw[p].w]);
-                    const uint32_t e = sure ? jc : (jc | NL_BAND);
-                    band = band || !sure;
-                    if (k < NLW_ROW) rows[p][k] = e;
-                    else if (k < max_nn) nbrs[(size_t)k * N + pi[p]] = e;
-                }
-                n[p] += __popc(hits);
             }
+        };
+        if constexpr (REF) {
+            // every particle of the chunk in its cell (with 64-bit fixed positions the cell
+            // is the word's), or the differences are formed pair by pair
+            const bool in_cell = lo || lane >= cnt || (word_in_cell(my_word.x, cx, dx) && word_in_cell(my_word.y, cy, dy) &&
+                                                       word_in_cell(my_word.z, cz, dz));
+            if (__all_sync(0xffffffffu, in_cell)) scan(std::true_type{});
+            else scan(std::false_type{});
+        } else {
+            scan(std::false_type{});
         }
         band = __any_sync(0xffffffffu, band);
         __syncwarp();  // the rows' entries, before other lanes read them (a vote orders no memory)
