@@ -815,6 +815,9 @@ struct azp_batch {
     uint32_t* t_tag = nullptr;
     uint16_t* t_sys = nullptr;
     uint32_t* t_cell = nullptr;
+    // packed state on its way to the host
+    double *o_pos = nullptr, *o_vel = nullptr, *o_accel = nullptr;
+    int* o_image = nullptr;
     // cells / list
     uint32_t ncell = 0;
     uint32_t *cell_of = nullptr, *slot = nullptr, *cell_count = nullptr, *cell_start = nullptr, *members = nullptr,
@@ -853,7 +856,7 @@ void b_free(azp_batch* b)
     void* ptrs[] = {b->info, b->sys_off, b->pos[0], b->pos[1], b->fix[0], b->fix[1], b->fix_build, b->vel, b->accel,
                     b->image, b->tag, b->sys, b->t_pos, b->t_vel, b->t_accel, b->t_image, b->t_tag, b->t_sys,
                     b->t_cell, b->cell_of, b->slot, b->cell_count, b->cell_start, b->members, b->scan_tmp,
-                    b->rindex, b->counts, b->nbrs, b->flags, b->d_ts, b->work};
+                    b->rindex, b->counts, b->nbrs, b->flags, b->d_ts, b->work, b->o_pos, b->o_vel, b->o_accel, b->o_image};
     for (void* p : ptrs) cudaFree(p);
     if (b->gstream) cudaStreamDestroy(b->gstream);
 }
@@ -1168,6 +1171,10 @@ azp_batch* azp_batch_create(const azp_batch_config* c, int* status)
     BALLOC(b->t_tag, N);
     BALLOC(b->t_sys, N);
     BALLOC(b->t_cell, N);
+    BALLOC(b->o_pos, (size_t)4 * N);
+    BALLOC(b->o_vel, (size_t)4 * N);
+    BALLOC(b->o_accel, (size_t)3 * N);
+    BALLOC(b->o_image, (size_t)3 * N);
     BALLOC(b->cell_of, N);
     BALLOC(b->slot, N);
     BALLOC(b->members, N);
@@ -1266,14 +1273,14 @@ int azp_batch_get_state(azp_batch* b, double* pos, double* vel, double* accel, i
     if (!b || !b->have_state || !pos || !vel || !accel || !image) return AZP_ERR_INVALID;
     cudaStream_t s = as_stream(stream);
     const uint32_t N = b->N;
-    // packed in the rebuild's temporaries, which hold nothing between rebuilds
-    double *dp = reinterpret_cast<double*>(b->t_pos), *dv = reinterpret_cast<double*>(b->t_vel);
-    k_b_store<<<nblk(N), 256, 0, s>>>(b->pos[b->cur], b->vel, b->accel, b->image, b->tag, b->sys, b->sys_off, N, dp, dv,
-                                      b->t_accel, b->t_image);
-    AZP_CUDA_TRY(cudaMemcpyAsync(pos, dp, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, s));
-    AZP_CUDA_TRY(cudaMemcpyAsync(vel, dv, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, s));
-    AZP_CUDA_TRY(cudaMemcpyAsync(accel, b->t_accel, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, s));
-    AZP_CUDA_TRY(cudaMemcpyAsync(image, b->t_image, sizeof(int) * 3 * N, cudaMemcpyDeviceToHost, s));
+    // packed in buffers that nothing else writes: a call on another stream than the run's
+    // may read a state that is changing, but changes none
+    k_b_store<<<nblk(N), 256, 0, s>>>(b->pos[b->cur], b->vel, b->accel, b->image, b->tag, b->sys, b->sys_off, N, b->o_pos,
+                                      b->o_vel, b->o_accel, b->o_image);
+    AZP_CUDA_TRY(cudaMemcpyAsync(pos, b->o_pos, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, s));
+    AZP_CUDA_TRY(cudaMemcpyAsync(vel, b->o_vel, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, s));
+    AZP_CUDA_TRY(cudaMemcpyAsync(accel, b->o_accel, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, s));
+    AZP_CUDA_TRY(cudaMemcpyAsync(image, b->o_image, sizeof(int) * 3 * N, cudaMemcpyDeviceToHost, s));
     AZP_CUDA_TRY(cudaStreamSynchronize(s));
     return AZP_OK;
 }

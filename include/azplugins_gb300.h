@@ -565,6 +565,9 @@ AZP_API void azp_batch_destroy(azp_batch* b);
  * image [sumN][3] or NULL; host pointers */
 AZP_API int azp_batch_set_state(azp_batch* b, const double* pos, const double* vel, const double* accel,
                                 const int32_t* image, uint64_t timestep, void* stream);
+/* the state as packed host arrays; returns when they are written. Called on another stream
+ * than a run that is under way, without waiting for it, it returns values of different
+ * moments (and leaves the run as it is) */
 AZP_API int azp_batch_get_state(azp_batch* b, double* pos, double* vel, double* accel, int32_t* image,
                                 void* stream);
 AZP_API int azp_batch_run(azp_batch* b, uint64_t steps, void* stream);
