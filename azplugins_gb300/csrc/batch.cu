@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "celllist.cuh"
@@ -786,13 +787,16 @@ int launch_b_step_kind(int kind, int precision, const BStep& a, cudaStream_t s)
 
 using namespace azp;
 
+constexpr int B_TPPS = 6, B_BLOCKS = 4;  // 1 to 32 lanes per particle, blocks of 64 to 512 threads
+
 struct azp_batch {
     uint32_t S = 0, N = 0;
     std::vector<uint32_t> n_of, off;
     int precision = AZP_FP64, kind = 0, tpp = 1, block = BATCH_BLOCK;
     std::vector<double> row_len;  // expected list entries per particle, by replica
-    uint2* work = nullptr;        // blocks of the fused step (b_plan), for block and tpp as they are
-    uint32_t work_blocks = 0;
+    uint2* work = nullptr;        // blocks of the fused step (b_plan)
+    // first entry and number of entries of work, by log2(tpp) and log2(block / 64)
+    std::pair<size_t, uint32_t> plan[B_TPPS][B_BLOCKS];
     double dt = 0.005, kT = 1.0, gamma = 1.0, r_buff = 0.4;
     int noiseless = 0;
     FlowD flow{};
@@ -866,10 +870,12 @@ uint32_t nblk(uint32_t n) { return (n + 255) / 256; }
 // words of a particle's list row
 uint32_t b_width(uint32_t max_nn) { return (max_nn + B_LIST_BLOCK - 1u) / B_LIST_BLOCK * B_LIST_BLOCK; }
 
-// The blocks of the fused step, for the batch's block size and lanes per particle. FP32:
-// 2^B_LT lanes. FP64: a replica takes the smallest power of two at which a lane walks at
-// most per_lane entries of a row, 4 or more (narrower reads waste the sectors of a block),
-// b->tpp or more; per_lane is 128, where fewer sums are combined and the rows of a warp are
+// The blocks of the fused step, for every block size and number of lanes per particle that
+// can be asked for, laid out once: azp_batch_set_tpp and azp_batch_set_block choose among
+// them on the host, beside runs in flight, allocations that are not to be made and captures.
+// FP32: 2^B_LT lanes. FP64: a replica takes the smallest power of two at which a lane walks
+// at most per_lane entries of a row, 4 or more (narrower reads waste the sectors of a block),
+// tpp or more; per_lane is 128, where fewer sums are combined and the rows of a warp are
 // read together, and less while the lanes would not fill a quarter of the chip. Replicas
 // with the longest rows go first, so that the last blocks are short.
 int b_plan(azp_batch* b)
@@ -877,32 +883,40 @@ int b_plan(azp_batch* b)
     int dev = 0, sms = 1;
     AZP_CUDA_TRY(cudaGetDevice(&dev));
     AZP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    double per_lane = 128.0;
-    const auto lanes_log2 = [&](uint32_t r) {
-        uint32_t lt = B_LT;
-        if (b->precision == AZP_FP32) return lt;
-        while (lt < 5 && (b->row_len[r] > per_lane * (1u << lt) || (1 << lt) < b->tpp)) ++lt;
-        return lt;
-    };
-    for (; per_lane > 8.0; per_lane *= 0.5) {
-        size_t lanes = 0;
-        for (uint32_t r = 0; r < b->S; ++r) lanes += (size_t)b->n_of[r] << lanes_log2(r);
-        if (lanes >= (size_t)sms * 512) break;
-    }
     std::vector<uint32_t> order(b->S);
     for (uint32_t r = 0; r < b->S; ++r) order[r] = r;
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return b->row_len[x] > b->row_len[y]; });
     std::vector<uint2> work;
-    for (uint32_t r : order) {
-        const uint32_t lt = lanes_log2(r);
-        const uint32_t per = b_block_particles((uint32_t)b->block, lt);
-        for (uint32_t k = 0; k < b->n_of[r]; k += per) work.push_back(make_uint2(r | lt << 16, b->off[r] + k));
+    for (int kt = 0; kt < B_TPPS; ++kt) {
+        double per_lane = 128.0;
+        const auto lanes_log2 = [&](uint32_t r) {
+            uint32_t lt = B_LT;
+            if (b->precision == AZP_FP32) return lt;
+            while (lt < 5 && (b->row_len[r] > per_lane * (1u << lt) || (int)lt < kt)) ++lt;
+            return lt;
+        };
+        for (; per_lane > 8.0; per_lane *= 0.5) {
+            size_t lanes = 0;
+            for (uint32_t r = 0; r < b->S; ++r) lanes += (size_t)b->n_of[r] << lanes_log2(r);
+            if (lanes >= (size_t)sms * 512) break;
+        }
+        for (int kb = 0; kb < B_BLOCKS; ++kb) {
+            if (kt > 0 && b->precision == AZP_FP32) {
+                b->plan[kt][kb] = b->plan[0][kb];
+                continue;
+            }
+            b->plan[kt][kb].first = work.size();
+            for (uint32_t r : order) {
+                const uint32_t lt = lanes_log2(r);
+                const uint32_t per = b_block_particles(64u << kb, lt);
+                for (uint32_t k = 0; k < b->n_of[r]; k += per) work.push_back(make_uint2(r | lt << 16, b->off[r] + k));
+            }
+            b->plan[kt][kb].second = (uint32_t)(work.size() - b->plan[kt][kb].first);
+        }
     }
-    cudaFree(b->work);
     const int st = balloc(&b->work, work.size());
     if (st) return st;
     AZP_CUDA_TRY(cudaMemcpy(b->work, work.data(), sizeof(uint2) * work.size(), cudaMemcpyHostToDevice));
-    b->work_blocks = (uint32_t)work.size();
     return AZP_OK;
 }
 
@@ -978,8 +992,11 @@ BStep b_args(azp_batch* b)
     a.flags = b->flags;
     const double half = 0.5 * b->r_buff;
     a.disp_thresh2 = (float)(half * half * (1.0 - 1e-5));
-    a.work = b->work;
-    a.blocks = b->work_blocks;
+    int kt = 0, kb = 0;
+    while ((1 << kt) < b->tpp) ++kt;
+    while ((64 << kb) < b->block) ++kb;
+    a.work = b->work + b->plan[kt][kb].first;
+    a.blocks = b->plan[kt][kb].second;
     a.block = b->block;
     return a;
 }
@@ -1341,19 +1358,17 @@ int azp_batch_error(azp_batch* b, uint32_t* err_word, uint32_t* n_builds, void* 
 int azp_batch_set_block(azp_batch* b, int block)
 {
     if (!b || !(block == 64 || block == 128 || block == 256 || block == 512)) return AZP_ERR_INVALID;
-    if (b->block == block) return AZP_OK;
-    b_free_graphs(b);
+    if (b->block != block) b_free_graphs(b);
     b->block = block;
-    return b_plan(b);
+    return AZP_OK;
 }
 
 int azp_batch_set_tpp(azp_batch* b, int tpp)
 {
     if (!b || !(tpp == 1 || tpp == 2 || tpp == 4 || tpp == 8 || tpp == 16 || tpp == 32)) return AZP_ERR_INVALID;
-    if (b->tpp == tpp) return AZP_OK;
-    b_free_graphs(b);
+    if (b->tpp != tpp) b_free_graphs(b);
     b->tpp = tpp;
-    return b_plan(b);
+    return AZP_OK;
 }
 
 uint64_t azp_batch_last_launches(const azp_batch* b) { return b ? b->launches : 0; }

@@ -1,5 +1,5 @@
 """A batch used from more than one place: its state read on another stream while a run is
-under way."""
+under way, and its block size and lanes chosen beside a run and inside a capture."""
 
 import ctypes
 
@@ -48,3 +48,36 @@ def test_reads_on_another_stream_leave_the_state_alone(precision):
         b.close()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+def test_choices_allocate_nothing_and_wait_for_nothing():
+    """Inside a capture of this thread, where allocations, copies and waits are errors."""
+    import torch
+
+    b, ref = _batch(), _batch()
+    b.run(1)  # (too short for graphs, whose destruction a capture does not allow either)
+    ref.run(1)
+    torch.cuda.synchronize()
+    x = torch.zeros(1000, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x.add_(1.0)
+        b.set_block(128)
+        b.set_tpp(8)
+        b.set_block(64)
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 1000.0
+    # and beside a run that is under way
+    b.run(200, check=False)
+    b.set_block(512)
+    b.run(50, check=False)
+    b.set_block(128)
+    b.run(50)
+    for n in (200, 50, 50):
+        ref.run(n)
+    # the block size changes no particle's arithmetic
+    for a, c in zip(b.get_arrays(), ref.get_arrays()):
+        assert np.array_equal(a, c)
+    b.close()
+    ref.close()
