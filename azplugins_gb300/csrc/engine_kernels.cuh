@@ -1597,6 +1597,9 @@ __global__ void __launch_bounds__(RUN_BLOCK, FX ? 3 : 2) k_md_run(const __grid_c
         }
         uint32_t* word = r.request + s % 3u;
         if (__any_sync(0xffffffffu, want) && (threadIdx.x & 31u) == 0u) atomicOr(word, 1u);
+        // (every warp of the block has raised its errors: a step that fails is followed by no
+        // rebuild, as where the steps are launches)
+        __syncthreads();
         if (threadIdx.x == 0u && *(volatile uint32_t*)(flags + 1) != 0u) atomicOr(word, 2u);
         if (!grid_barrier(r, gen, &s_word)) return;
         const uint32_t got = *(volatile uint32_t*)word;
