@@ -693,6 +693,15 @@ __global__ void __launch_bounds__(STATE_BLOCK)
 using namespace azp;
 
 constexpr uint32_t RUN_SYNC = 32, FLAG_WORDS = 64;
+constexpr uint32_t FLAG_BEFORE = 7;  // the error word that the last set_state found
+
+// all words zero but FLAG_BEFORE (one block of FLAG_WORDS threads)
+__global__ void k_open_flags(uint32_t* flags)
+{
+    const uint32_t before = flags[1];
+    __syncthreads();
+    flags[threadIdx.x] = threadIdx.x == FLAG_BEFORE ? before : 0u;
+}
 
 struct azp_md {
     uint32_t N = 0, ntypes = 0, nbt = 0;
@@ -824,6 +833,7 @@ struct azp_md {
     double* snap_diam = nullptr;
     // whether this engine's steps go as persistent launches (k_md_run)
     bool run_kernel = false;
+    uint32_t run_polls = RUN_MAX_POLLS;
     // graphs
     bool use_graphs = true;
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // pair of mid steps starting at cur = 0 / 1
@@ -1196,6 +1206,7 @@ int enqueue_run(azp_md* m, int integ, uint64_t steps, cudaStream_t s)
     r.blocks = (uint32_t)(((size_t)m->N * m->tpp + RUN_BLOCK - 1) / RUN_BLOCK);
     r.sync = m->flags + RUN_SYNC;
     r.request = r.sync + 4;
+    r.max_polls = m->run_polls;
     while (steps > 0) {
         r.steps = (uint32_t)std::min(steps, RUN_STEPS);
         r.cur = m->cur;
@@ -1601,6 +1612,13 @@ azp_md* azp_md_create(const azp_md_config* c, int* status)
         ALLOC(m->mass, N);
         ALLOC(m->t_mass, N);
     }
+    // A run that gives up at a barrier leaves the buffers of its later steps as they were,
+    // and the launches enqueued behind it read them: types of 0 there, not what was in the
+    // memory before.
+    CTRY(cudaMemset(m->pos[1], 0, sizeof(double4_32a) * N));
+    CTRY(cudaMemset(m->fix[1], 0, sizeof(uint4) * N));
+    if (m->lo[1]) CTRY(cudaMemset(m->lo[1], 0, sizeof(uint4) * N));
+    CTRY(cudaStreamSynchronize(cudaStreamLegacy));
     ALLOC(m->vel, N);
     ALLOC(m->accel, (size_t)3 * N);
     ALLOC(m->image, (size_t)3 * N);
@@ -1816,6 +1834,8 @@ azp_md* azp_md_create(const azp_md_config* c, int* status)
     const char* env_run = std::getenv("AZP_RUN_KERNEL");
     m->run_kernel = m->use_graphs && !m->d_dvel && !m->d_img0 && !m->d_wall_f && !m->tile_tab &&
                     m->grid.ncell <= RUN_MAX_CELLS && !(env_run && env_run[0] == '0');
+    const char* env_polls = std::getenv("AZP_RUN_POLLS");
+    if (env_polls && std::atoi(env_polls) > 0) m->run_polls = (uint32_t)std::atoi(env_polls);
 #undef ALLOC
 #undef CTRY
     if (status) *status = AZP_OK;
@@ -1870,7 +1890,8 @@ int azp_md_set_state(azp_md* m, const double* pos, const double* vel, const doub
     m->timestep = timestep;
     const unsigned long long ts = timestep;
     AZP_CUDA_TRY(cudaMemcpyAsync(m->d_ts, &ts, sizeof(ts), cudaMemcpyHostToDevice, s));
-    AZP_CUDA_TRY(cudaMemsetAsync(m->flags, 0, sizeof(uint32_t) * FLAG_WORDS, s));
+    k_open_flags<<<1, FLAG_WORDS, 0, s>>>(m->flags);
+    AZP_CHECK_LAUNCH("k_open_flags");
     int st = AZP_OK;
     bool placed = false;
     uint32_t flags_seen[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -1879,7 +1900,8 @@ int azp_md_set_state(azp_md* m, const double* pos, const double* vel, const doub
         // order and rebuild only if some particle lies more than r_buff / 2 from
         // its position at the last build (a state read back from this engine and
         // set again moves nothing). A denser new state that overflows the list
-        // takes the full path below.
+        // takes the full path below, and so does a state after a run that gave up,
+        // whose order may be half of one sort and half of another.
         const MDArgs a = base_args(m);
         if (m->precision == AZP_FP32) {
             k_load_state_ordered_fx<<<blocks_for(N, STATE_BLOCK), STATE_BLOCK, 0, s>>>(
@@ -1900,7 +1922,7 @@ int azp_md_set_state(azp_md* m, const double* pos, const double* vel, const doub
         if (st) return st;
         AZP_CUDA_TRY(cudaMemcpyAsync(flags_seen, m->flags, sizeof(flags_seen), cudaMemcpyDeviceToHost, s));
         AZP_CUDA_TRY(cudaStreamSynchronize(s));
-        placed = flags_seen[3] <= m->max_nn;
+        placed = flags_seen[3] <= m->max_nn && !(flags_seen[FLAG_BEFORE] & AZP_EBIT_TIMEOUT);
         if (!placed) AZP_CUDA_TRY(cudaMemsetAsync(m->flags, 0, sizeof(uint32_t) * 8, s));
     }
     if (!placed) {
@@ -2190,6 +2212,7 @@ int azp_md_thermo(azp_md* m, double* out, void* stream)
     if (f[3] > m->max_nn) return AZP_ERR_NLIST_OVERFLOW;
     if (f[1] & AZP_EBIT_BOND) return AZP_ERR_BOND;
     if (f[1] & AZP_EBIT_NONFINITE) return AZP_ERR_NONFINITE;
+    if (f[1] & AZP_EBIT_TIMEOUT) return AZP_ERR_TIMEOUT;
     return AZP_OK;
 }
 

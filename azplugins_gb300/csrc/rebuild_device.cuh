@@ -142,6 +142,7 @@ struct RunArgs {
     RebuildArgs rebuild[2];
     uint32_t steps, blocks;     // timesteps, and thread blocks one step takes
     int cur;                    // parity of the first step
+    uint32_t max_polls;         // of one wait at a barrier
     uint32_t* sync;             // grid barrier: arrivals, generation
     uint32_t* request;          // three rotating words: 1 a particle asked for a rebuild, 2 an error is set;
                                 // then three rotating counters of the blocks taken beyond the launch's own
@@ -150,8 +151,10 @@ struct RunArgs {
 // All blocks of the (cooperative) launch. Thread 0 releases the block's writes with its
 // arrival (an acquire-release add, which with the block barrier before it covers the
 // whole block) and polls the generation with relaxed loads until the last arrival has
-// raised it, then acquires. The wait is bounded: about ten seconds of polls, after which
-// the launch's error word gets AZP_EBIT_TIMEOUT and the block leaves.
+// raised it, then acquires. The wait is bounded: r.max_polls polls, after which the
+// launch's error word gets AZP_EBIT_TIMEOUT and the block leaves. It has arrived, so the
+// others pass this barrier at most, with all of the phase before it done, and give up at
+// the next. AZP_RUN_POLLS sets another limit than about ten seconds.
 // gen: the generation before the launch's first barrier, counted on by every thread.
 constexpr uint32_t RUN_MAX_POLLS = 1u << 24;
 AZP_D uint32_t load_relaxed(const uint32_t* p)
@@ -173,7 +176,7 @@ AZP_D bool grid_barrier(const RunArgs& r, uint32_t& gen, uint32_t* s_word)
         } else {
             uint32_t polls = 0;
             while (load_relaxed(r.sync + 1) == gen)
-                if (++polls == RUN_MAX_POLLS) {
+                if (++polls >= r.max_polls) {
                     atomicOr(r.step[0].flags + 1, AZP_EBIT_TIMEOUT);
                     ok = 0u;
                     break;
