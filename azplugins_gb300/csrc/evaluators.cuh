@@ -27,7 +27,8 @@ constexpr int CUT_REC = 4;    // rcutsq, ronsq, 1/(rcutsq-ronsq)^3, xplor flag
 // reciprocal maps to the hardware-assisted rounded reciprocal instead of a full
 // division (an approximate reciprocal's extra ulp, raised to the 12th power by
 // the LJ core, costs too much of the FP32 force budget at overlapped pairs). FP64
-// on the device: the refined forms of fp64.cuh, within an ulp.
+// on the device: the refined forms of fp64.cuh, rounded as the operators round but in
+// rare cases near a boundary.
 AZP_HD double rcp(double x)
 {
 #ifdef __CUDA_ARCH__
@@ -77,7 +78,7 @@ template<typename R> AZP_HD R over(R a, R b) { return a / b; }
 template<> AZP_HD double over<double>(double a, double b)
 {
 #ifdef __CUDA_ARCH__
-    return a * d_rcp(b);
+    return d_div(a, b);
 #else
     return a / b;
 #endif
