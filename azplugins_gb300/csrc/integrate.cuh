@@ -8,6 +8,8 @@
 // (the reference writes the type as a number, src/TwoStepBrownianFlow.h:177).
 #pragma once
 
+#include <cmath>
+
 #include "common.cuh"
 #include "fp64.cuh"
 #include "philox.cuh"
@@ -20,7 +22,7 @@ constexpr uint32_t MAX_GAMMA_TYPES = 64;
 struct FlowD {
     int kind;
     double a, b, c;  // CONSTANT: U; PARABOLIC: a = Umax = 1.5 mean_velocity, b = L = separation / 2
-    double binv;     // 1 / b
+    double binv;     // 1 / b; 0 where b or 1 / b is 0, infinite or not a number
 };
 
 inline FlowD make_flow(const azp_flow& f)
@@ -32,7 +34,8 @@ inline FlowD make_flow(const azp_flow& f)
         r.a = 1.5 * f.p[0];
         r.b = 0.5 * f.p[1];
         r.c = 0.0;
-        r.binv = 1.0 / r.b;
+        const double binv = 1.0 / r.b;
+        if (std::isnormal(r.b) && std::isnormal(binv)) r.binv = binv;
     } else {
         r.a = f.p[0];
         r.b = f.p[1];
@@ -46,7 +49,7 @@ AZP_D void flow_at(const FlowD& f, double y, double& ux, double& uy, double& uz)
     if (f.kind == AZP_FLOW_PARABOLIC) {
         // y / b: the product with 1 / b corrected by its residual
         double yr = y * f.binv;
-        yr = fma(fma(-yr, f.b, y), f.binv, yr);
+        yr = f.binv != 0.0 ? fma(fma(-yr, f.b, y), f.binv, yr) : y / f.b;
         ux = f.a * (1.0 - yr * yr);
         uy = 0.0;
         uz = 0.0;
@@ -61,7 +64,7 @@ AZP_D void flow_at(const FlowD& f, double y, double& ux, double& uy, double& uz)
 AZP_D void flow_at_f(const FlowD& f, float y, float& ux, float& uy, float& uz)
 {
     if (f.kind == AZP_FLOW_PARABOLIC) {
-        const float yr = y * (float)f.binv;
+        const float yr = y * (float)(f.binv != 0.0 ? f.binv : 1.0 / f.b);
         ux = (float)f.a * (1.0f - yr * yr);
         uy = 0.0f;
         uz = 0.0f;
