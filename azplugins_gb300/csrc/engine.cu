@@ -1481,11 +1481,19 @@ int size_list(azp_md* m, cudaStream_t s)
 // only while the launch has fewer threads than half of what the chip holds. Cutoffs
 // far apart make rows uneven (a colloid lists many times what a solvent bead does,
 // and its warp waits for it): those are split from 28 entries a thread on.
+// The row is an estimate, far above the rows of a mixture (453 against 25 for solvent and
+// 134 for colloids in the one below), so in either precision uneven rows are split to more
+// than four threads only while the launch stays at two million threads.
 //   LJ fluid              N = 4,096: 85 / 64 / 51 / 47 / 47
 //                         N = 54,872: 108 / 90 / 92 / 102 / 121
 //                         N = 110,592: 127 / 130 / 132 / 151 / 196
 //   melt                  N = 40,000: 35 / 34 / 36 / 43 / 55
-//   colloid mixture       N = 65,537: 441 / 311 / 240 / 220 / 207
+//   colloid mixture       N = 65,537: 406 / 256 / 183 / 168 / 151 (FP64 1,755 / 951 / 747 / 604 / 544)
+//   the same with 0.4 % colloids    N = 20,000: 461 / 261 / 145 / 98 / 81
+//                                   N = 200,000: 728 / 529 / 441 / 403 / 451 (FP64 2,819 / 2,044 / 1,644 / 1,519 / 1,669)
+//                                   N = 1,000,000: 2,197 / 1,845 / 1,734 / 1,749 / 2,093 (FP64 10.5 / 8.3 / 7.19 / 7.11 / 8.2 ms)
+//   0.04 % colloids                 N = 200,000: 651 / 417 / 302 / 269 / 290
+//                                   N = 1,000,000: 1,202 / 1,013 / 946 / 1,008 / 1,239
 int threads_per_particle(const azp_md_config& c)
 {
     if (c.pair_kind < 0 || !c.r_cut || c.N == 0) return 1;
@@ -1497,11 +1505,13 @@ int threads_per_particle(const azp_md_config& c)
         }
     const double row = c.N / (c.box.L[0] * c.box.L[1] * c.box.L[2]) * 4.18879 * rmax * rmax * rmax;
     int tpp = 1;
+    const bool uneven = rmax > 1.5 * rmin;
+    const auto room = [&] { return !uneven || tpp < 4 || 2.0 * c.N * tpp <= 2e6; };
     if (c.precision == AZP_FP64) {
-        while (tpp < 16 && 2 * tpp <= row / 13.0) tpp *= 2;
+        while (tpp < 16 && 2 * tpp <= row / 13.0 && room()) tpp *= 2;
         while (tpp < 32 && 2 * tpp <= row / 3.0 && (double)c.N * tpp < 60000.0) tpp *= 2;
     } else {
-        while (rmax > 1.5 * rmin && tpp < 16 && 2 * tpp <= row / 28.0) tpp *= 2;
+        while (uneven && tpp < 16 && 2 * tpp <= row / 28.0 && room()) tpp *= 2;
         while (tpp < 16 && 2 * tpp <= row / 3.0 && (double)c.N * tpp < 80000.0) tpp *= 2;
     }
     return tpp;
