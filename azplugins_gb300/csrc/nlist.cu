@@ -399,18 +399,21 @@ void launch_nlist_build(const double4_32a* pos, const uint4* fixed, uint32_t N, 
     const ListArgs L{pos, fixed, lo, N, ntypes, bx, g, cell_start, members, cell_of, cuts, ex_n, ex_keys, keys,
                      counts, nbrs, max_nn, flags};
     if (!keys && !tile && (!members || words) && warp_list_build(N, g, !members)) {
-        // small systems: four particles a warp, for more warps
-        const bool few = N < 40000u;
-        const auto go = [&](auto kernel, size_t smem) {
-            const uint32_t per = NLW_WARPS * (few ? 4u : 8u);
+        // Four particles a warp: eight share the candidates' loads between more tests, but
+        // hold twice the rows in shared memory and leave half the warps. Microseconds a
+        // build at 4 and at 8, caller's order: LJ fluid N = 4,096 98 / 105, 20,000 124 / 124,
+        // 40,000 160 / 175, 103,823 271 / 308, 250,000 758 / 821; engine steps with their
+        // builds, N = 250,000 FP32 233 / 241, 103,823 FP64 552 / 556.
+        constexpr int CH = 4;
+        const auto go = [&](auto kernel) {
+            const uint32_t per = NLW_WARPS * CH;
+            const size_t smem = nlw_shared_bytes<CH>(ntypes, NLW_WARPS);
             if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             kernel<<<(N + per - 1) / per, NLW_WARPS * 32, smem, s>>>(L, members ? words : fixed, gate);
         };
-        const size_t s4 = nlw_shared_bytes<4>(ntypes, NLW_WARPS), s8 = nlw_shared_bytes<8>(ntypes, NLW_WARPS);
-#define AZP_NLW(ONE, SORTED)                                                               \
-    (list_by_reference(g)                                                                  \
-         ? (few ? go(k_nlist_build_warps<ONE, SORTED, true, 4>, s4) : go(k_nlist_build_warps<ONE, SORTED, true, 8>, s8)) \
-         : (few ? go(k_nlist_build_warps<ONE, SORTED, false, 4>, s4) : go(k_nlist_build_warps<ONE, SORTED, false, 8>, s8)))
+#define AZP_NLW(ONE, SORTED)                                                    \
+    (list_by_reference(g) ? go(k_nlist_build_warps<ONE, SORTED, true, CH>)      \
+                          : go(k_nlist_build_warps<ONE, SORTED, false, CH>))
         if (ntypes == 1) members ? AZP_NLW(true, false) : AZP_NLW(true, true);
         else members ? AZP_NLW(false, false) : AZP_NLW(false, true);
 #undef AZP_NLW
