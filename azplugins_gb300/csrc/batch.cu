@@ -288,6 +288,14 @@ AZP_D uint32_t b_walk(const uint4* __restrict__ fixed, const double4_32a* __rest
     return mine;
 }
 
+// out of line: its registers do not count against the others
+static __device__ __noinline__ uint32_t b_walk_pairs(const uint4* fixed, const double4_32a* pos, const SysInfo& si,
+                                                     const uint2* range, uint32_t total, uint32_t first, uint32_t cnt,
+                                                     uint32_t* nbrs, uint32_t N, uint32_t max_nn)
+{
+    return b_walk<B_PAIR>(fixed, pos, si, range, total, first, cnt, nbrs, N, max_nn);
+}
+
 __global__ void __launch_bounds__(B_NL_WARPS * 32)
     k_b_nlist(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed, uint32_t N,
               const SysInfo* __restrict__ info, const uint32_t* __restrict__ cell_start,
@@ -351,7 +359,7 @@ __global__ void __launch_bounds__(B_NL_WARPS * 32)
         const bool in_cell = lane >= cnt || (word_in_cell(mine.x, cx, ncx) && word_in_cell(mine.y, cy, ncy) &&
                                              word_in_cell(mine.z, cz, ncz));
         const uint32_t n = !__all_sync(0xffffffffu, in_cell)
-                               ? b_walk<B_PAIR>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn)
+                               ? b_walk_pairs(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn)
                            : si.far_cells ? b_walk<B_NEAR>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn)
                                           : b_walk<B_WRAP>(fixed, pos, si, range, total, sa, cnt, nbrs, N, max_nn);
         if (lane < cnt) {
@@ -361,6 +369,70 @@ __global__ void __launch_bounds__(B_NL_WARPS * 32)
         __syncwarp();
         sa += cnt;
     }
+}
+
+// The list with a thread per particle: the same entries in the same order. For batches of
+// many particles with rows of about one length (b_plan), where no lane waits for another
+// and a warp's chunk of a few particles only leaves lanes without a candidate. Microseconds
+// a step with its list builds, a warp per chunk and a thread per particle:
+//   N = 400,000, rows of 7 (1,000,000) / 17 / 32 / 59 / 110: 226 and 155 / 111 and 93 /
+//   125 and 112 / 190 and 166 / 313 and 268; N = 160,000, 7 / 32 / 59: 54 and 44 / 65 and 60 /
+//   91 and 86; N = 40,000: 30 and 28 / 35 and 37 / 44 and 49; N = 4,000, 32: 22 and 26.
+__global__ void __launch_bounds__(128)
+    k_b_nlist_threads(const double4_32a* __restrict__ pos, const uint4* __restrict__ fixed, uint32_t N,
+                      const SysInfo* __restrict__ info, const uint32_t* __restrict__ cell_start,
+                      const uint32_t* __restrict__ cell_of, uint32_t* __restrict__ counts, uint32_t* __restrict__ nbrs,
+                      uint32_t max_nn, uint32_t* __restrict__ maxcount, const uint32_t* __restrict__ gate)
+{
+    if (gated_off(gate)) return;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const uint4 fi = fixed[i];
+    const SysInfo& si = info[fi.w];
+    const float sx = si.sfix[0], sy = si.sfix[1], sz = si.sfix[2], hi = si.list_hi, lo = si.list_lo;
+    const int ncx = si.dim[0], ncy = si.dim[1], ncz = si.dim[2];
+    const int r0 = si.reach[0], r1 = si.reach[1], r2 = si.reach[2];
+    const uint32_t c = cell_of[i] - si.cell_off;
+    const int cx = (int)(c % (uint32_t)ncx);
+    const int cy = (int)((c / (uint32_t)ncx) % (uint32_t)ncy);
+    const int cz = (int)(c / ((uint32_t)ncx * (uint32_t)ncy));
+    // the x-cells of a stencil row in their order: one slot range, or two at a face
+    const int x0 = cx - r0, x1 = cx + r0;
+    const bool two = x0 < 0 || x1 >= ncx;
+    const int b0 = x0 < 0 ? ncx + x0 : x0, e0 = two ? ncx - 1 : x1;
+    const int e1 = x1 >= ncx ? x1 - ncx : x1;
+    uint32_t n = 0u;
+    for (int oz = cz - r2; oz <= cz + r2; ++oz) {
+        const int nz = oz < 0 ? oz + ncz : (oz >= ncz ? oz - ncz : oz);
+        for (int oy = cy - r1; oy <= cy + r1; ++oy) {
+            const int ny = oy < 0 ? oy + ncy : (oy >= ncy ? oy - ncy : oy);
+            const uint32_t rb = si.cell_off + ((uint32_t)nz * ncy + ny) * ncx;
+            for (int part = 0; part < (two ? 2 : 1); ++part) {
+                const uint32_t sb = cell_start[rb + (part ? 0 : b0)], se = cell_start[rb + (part ? e1 : e0) + 1];
+                for (uint32_t j = sb; j < se; ++j) {
+                    const uint4 fj = fixed[j];
+                    const float dx = (float)(int32_t)(fi.x - fj.x) * sx;
+                    const float dy = (float)(int32_t)(fi.y - fj.y) * sy;
+                    const float dz = (float)(int32_t)(fi.z - fj.z) * sz;
+                    const float rs = dx * dx + dy * dy + dz * dz;
+                    if (!(rs < hi) || j == i) continue;
+                    if (!(rs < lo)) {
+                        // inside the band: the exact FP64 decision
+                        const double4_32a pi = pos[i];
+                        const double4_32a pj = pos[j];
+                        const double vx = min_image1(pi.x - pj.x, si.L[0], si.Linv[0]);
+                        const double vy = min_image1(pi.y - pj.y, si.L[1], si.Linv[1]);
+                        const double vz = min_image1(pi.z - pj.z, si.L[2], si.Linv[2]);
+                        if (!(rsq_exact(vx, vy, vz) < si.rlistsq)) continue;
+                    }
+                    if (n < max_nn) nbrs[b_entry(i, n, N)] = j;
+                    ++n;
+                }
+            }
+        }
+    }
+    counts[i] = n;
+    if (n > max_nn) atomicMax(maxcount, n);
 }
 
 __global__ void k_b_finish(uint32_t* __restrict__ flags, const uint32_t* __restrict__ gate)
@@ -401,7 +473,7 @@ struct BStep {
     float disp_thresh2;
     int next;
     const uint2* work;  // per block: (replica | log2 of the lanes per particle << 16, first particle)
-    uint32_t blocks;
+    uint32_t blocks;    // 0: a thread per particle instead
     int block;  // threads per block of the launch
     cudaGraphConditionalHandle next_cond;
     int set_cond;
@@ -426,6 +498,124 @@ constexpr int b_min_blocks()
 // but at least a warp's worth, so that the integration runs on full warps
 AZP_HD uint32_t b_block_particles(uint32_t block, uint32_t lt) { return block >> lt > 32u ? block >> lt : 32u; }
 
+// force / r of a pair in the FP32 step
+template<class PE> AZP_D float b_force(const float* rec, float rsq)
+{
+    float fdr, e;
+    PE::eval(rec, rsq, fdr, e);
+    return fdr;
+}
+
+// Langevin step two of particle i with the force f, and step one of the next timestep; whether
+// the particle asks for a list build
+template<typename R>
+AZP_D bool b_integrate(const BStep& a, const SysInfo* si, uint32_t i, R fx, R fy, R fz)
+{
+    const unsigned long long ts = *a.d_ts;
+    double4_32a p = a.pos[i];
+    double4_32a v = a.vel[i];
+    const uint32_t tg = a.tag[i];
+    bool want = false, moved = false;
+    if constexpr (std::is_same<R, double>::value) {
+        double ux, uy, uz;
+        flow_at(a.flow, p.y, ux, uy, uz);
+        const double c = a.noiseless ? 0.0 : a.noise;
+        double r0, r1, r2;
+        uniform3(AZP_RNG_LANGEVIN_FLOW, ts, si->seed, tg, -c, c - (-c), r0, r1, r2);
+        const double minv = 1.0 / v.w;
+        const double ax = (fx + (r0 - a.gamma * (v.x - ux))) * minv;
+        const double ay = (fy + (r1 - a.gamma * (v.y - uy))) * minv;
+        const double az = (fz + (r2 - a.gamma * (v.z - uz))) * minv;
+        const double h = 0.5 * a.dt;
+        v.x += h * ax;
+        v.y += h * ay;
+        v.z += h * az;
+        if (a.next) {
+            p.x += (v.x + h * ax) * a.dt;
+            p.y += (v.y + h * ay) * a.dt;
+            p.z += (v.z + h * az) * a.dt;
+            v.x += h * ax;
+            v.y += h * ay;
+            v.z += h * az;
+            moved = true;
+        } else {
+            a.accel[3 * i] = ax;
+            a.accel[3 * i + 1] = ay;
+            a.accel[3 * i + 2] = az;
+        }
+    } else {
+        float ux, uy, uz;
+        flow_at_f(a.flow, (float)p.y, ux, uy, uz);
+        const float c = a.noiseless ? 0.0f : (float)a.noise;
+        const float g = (float)a.gamma, dt = (float)a.dt;
+        float r0, r1, r2;
+        uniform3f(AZP_RNG_LANGEVIN_FLOW, ts, si->seed, tg, -c, 2.0f * c, r0, r1, r2);
+        const float minv = __frcp_rn((float)v.w);
+        const float ax = (fx + (r0 - g * ((float)v.x - ux))) * minv;
+        const float ay = (fy + (r1 - g * ((float)v.y - uy))) * minv;
+        const float az = (fz + (r2 - g * ((float)v.z - uz))) * minv;
+        if (a.next) {
+            const float kx = dt * ax, ky = dt * ay, kz = dt * az;
+            p.x += (double)(((float)v.x + kx) * dt);
+            p.y += (double)(((float)v.y + ky) * dt);
+            p.z += (double)(((float)v.z + kz) * dt);
+            v.x += (double)kx;
+            v.y += (double)ky;
+            v.z += (double)kz;
+            moved = true;
+        } else {
+            const float h = 0.5f * dt;
+            v.x += (double)(h * ax);
+            v.y += (double)(h * ay);
+            v.z += (double)(h * az);
+            a.accel[3 * i] = ax;
+            a.accel[3 * i + 1] = ay;
+            a.accel[3 * i + 2] = az;
+        }
+    }
+    a.vel[i] = v;
+    if (moved) {
+        int w[3] = {0, 0, 0};
+        wrap1(p.x, w[0], si->L[0], si->lo[0], si->hi[0]);
+        wrap1(p.y, w[1], si->L[1], si->lo[1], si->hi[1]);
+        wrap1(p.z, w[2], si->L[2], si->lo[2], si->hi[2]);
+        if (w[0] | w[1] | w[2])
+            for (int d = 0; d < 3; ++d) a.image[3 * i + d] += w[d];
+        a.pos_next[i] = p;
+        uint4 f;
+        f.x = to_fixed(p.x, si->Linv[0]);
+        f.y = to_fixed(p.y, si->Linv[1]);
+        f.z = to_fixed(p.z, si->Linv[2]);
+        f.w = a.sys[i];
+        a.fix_next[i] = f;
+        const uint4 fb = a.fix_build[i];
+        const float ddx = (float)(int32_t)(f.x - fb.x) * si->sfix[0];
+        const float ddy = (float)(int32_t)(f.y - fb.y) * si->sfix[1];
+        const float ddz = (float)(int32_t)(f.z - fb.z) * si->sfix[2];
+        want = ddx * ddx + ddy * ddy + ddz * ddz > a.disp_thresh2;
+        if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicOr(&a.flags[1], AZP_EBIT_NONFINITE);
+    }
+    return want;
+}
+
+// the last block to finish advances the timestep and arms the next build
+AZP_D void b_finish_step(const BStep& a, bool want)
+{
+    if (__any_sync(0xffffffffu, want) && (threadIdx.x & 31) == 0) atomicOr(&a.flags[0], 1u);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const uint32_t t = atomicAdd(&a.flags[4], 1u);
+        if (t == gridDim.x - 1) {
+            __threadfence();
+            const uint32_t req = atomicAdd(&a.flags[0], 0u) && !atomicAdd(&a.flags[1], 0u);
+            if (a.set_cond) cudaGraphSetConditional(a.next_cond, req ? 1u : 0u);
+            a.flags[4] = 0u;
+            *a.d_ts_rw = *a.d_ts_rw + 1ull;
+        }
+    }
+}
+
 // FP32 step: 2^B_LT lanes evaluate the pairs of a particle, B_TERMS entries of its row a
 // pass, and leave their terms in shared memory; one lane per particle and axis then adds
 // them in list order. The compensated addition is not free of its order (its product is
@@ -438,6 +628,7 @@ constexpr uint32_t B_TERM_ROW = B_TERMS * 4u + 4u;     // floats: (dx, dy, dz, f
 constexpr size_t b_step_smem(uint32_t block) { return (size_t)(block / 32u) * B_WARP_P * B_TERM_ROW * sizeof(float); }
 static_assert(3 * B_WARP_P <= 32, "a lane per particle and axis");
 static_assert(B_TERM_ROW % 4 == 0, "rows of 16-byte terms");
+static_assert(B_BATCH == 4 && B_LIST_BLOCK % 4 == 0, "a batch is a 16-byte word of the list");
 static_assert(B_TERMS == B_LIST_BLOCK, "a pass takes a block of the list");
 
 // The fused step. A block takes particles of one replica; 2^lt lanes of a warp walk the
@@ -539,8 +730,7 @@ __global__ void __launch_bounds__(BATCH_BLOCK_MAX, (b_min_blocks<PE, R>())) k_b_
                         const double vz = min_image1(pi.z - pj.z, si->L[2], si->Linv[2]);
                         in = rsq_exact(vx, vy, vz) < si->rcutsq;
                     }
-                    float fdr, e;
-                    PE::eval(rec, in ? rsq : rc2, fdr, e);
+                    const float fdr = b_force<PE>(rec, in ? rsq : rc2);
                     put[u << B_LT] = make_float4(dx, dy, dz, in ? fdr : 0.0f);
                 }
                 __syncwarp();
@@ -571,104 +761,87 @@ __global__ void __launch_bounds__(BATCH_BLOCK_MAX, (b_min_blocks<PE, R>())) k_b_
     if (threadIdx.x < np) {
         const uint32_t i = work.y + threadIdx.x;
         const R fx = s_force[0][threadIdx.x], fy = s_force[1][threadIdx.x], fz = s_force[2][threadIdx.x];
-        const unsigned long long ts = *a.d_ts;
-        double4_32a p = a.pos[i];
-        double4_32a v = a.vel[i];
-        const uint32_t tg = a.tag[i];
-        bool moved = false;
+        want = b_integrate(a, si, i, fx, fy, fz);
+    }
+    b_finish_step(a, want);
+}
+
+// The same with a thread per particle, which walks its row in words of four entries, adds the
+// terms in list order and integrates: full warps however small the replicas are, and no
+// lanes without an entry. For batches of many particles with rows of about one length
+// (b_plan); the states are those of k_b_step (FP32: bitwise).
+template<class PE, typename R>
+__global__ void __launch_bounds__(BATCH_BLOCK_MAX) k_b_step_threads(BStep a)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool want = false;
+    if (i < a.N) {
+        const SysInfo* si = a.info + a.sys[i];
+        R rec[PAIR_TBL];
+#pragma unroll
+        for (int k = 0; k < PAIR_TBL; ++k) {
+            if constexpr (std::is_same<R, double>::value)
+                rec[k] = si->rec[k];
+            else
+                rec[k] = si->recf[k];
+        }
+        const uint32_t n = PE::enabled(rec) ? min(a.counts[i], a.max_nn) : 0u;
         if constexpr (std::is_same<R, double>::value) {
-            double ux, uy, uz;
-            flow_at(a.flow, p.y, ux, uy, uz);
-            const double c = a.noiseless ? 0.0 : a.noise;
-            double r0, r1, r2;
-            uniform3(AZP_RNG_LANGEVIN_FLOW, ts, si->seed, tg, -c, c - (-c), r0, r1, r2);
-            const double minv = 1.0 / v.w;
-            const double ax = (fx + (r0 - a.gamma * (v.x - ux))) * minv;
-            const double ay = (fy + (r1 - a.gamma * (v.y - uy))) * minv;
-            const double az = (fz + (r2 - a.gamma * (v.z - uz))) * minv;
-            const double h = 0.5 * a.dt;
-            v.x += h * ax;
-            v.y += h * ay;
-            v.z += h * az;
-            if (a.next) {
-                p.x += (v.x + h * ax) * a.dt;
-                p.y += (v.y + h * ay) * a.dt;
-                p.z += (v.z + h * az) * a.dt;
-                v.x += h * ax;
-                v.y += h * ay;
-                v.z += h * az;
-                moved = true;
-            } else {
-                a.accel[3 * i] = ax;
-                a.accel[3 * i + 1] = ay;
-                a.accel[3 * i + 2] = az;
+            double fx = 0, fy = 0, fz = 0;
+            const double4_32a pi = a.pos[i];
+            for (uint32_t k = 0; k < n; ++k) {
+                const uint32_t j = a.nbrs[b_entry(i, k, a.N)];
+                const double4_32a pj = a.pos[j];
+                const double dx = min_image1(pi.x - pj.x, si->L[0], si->Linv[0]);
+                const double dy = min_image1(pi.y - pj.y, si->L[1], si->Linv[1]);
+                const double dz = min_image1(pi.z - pj.z, si->L[2], si->Linv[2]);
+                const double rsq = rsq_exact(dx, dy, dz);
+                if (!(rsq < si->rcutsq)) continue;
+                double fdr, e;
+                PE::eval(rec, rsq, fdr, e);
+                fx += dx * fdr;
+                fy += dy * fdr;
+                fz += dz * fdr;
             }
+            want = b_integrate(a, si, i, fx, fy, fz);
         } else {
-            float ux, uy, uz;
-            flow_at_f(a.flow, (float)p.y, ux, uy, uz);
-            const float c = a.noiseless ? 0.0f : (float)a.noise;
-            const float g = (float)a.gamma, dt = (float)a.dt;
-            float r0, r1, r2;
-            uniform3f(AZP_RNG_LANGEVIN_FLOW, ts, si->seed, tg, -c, 2.0f * c, r0, r1, r2);
-            const float minv = __frcp_rn((float)v.w);
-            const float ax = (fx + (r0 - g * ((float)v.x - ux))) * minv;
-            const float ay = (fy + (r1 - g * ((float)v.y - uy))) * minv;
-            const float az = (fz + (r2 - g * ((float)v.z - uz))) * minv;
-            if (a.next) {
-                const float kx = dt * ax, ky = dt * ay, kz = dt * az;
-                p.x += (double)(((float)v.x + kx) * dt);
-                p.y += (double)(((float)v.y + ky) * dt);
-                p.z += (double)(((float)v.z + kz) * dt);
-                v.x += (double)kx;
-                v.y += (double)ky;
-                v.z += (double)kz;
-                moved = true;
-            } else {
-                const float h = 0.5f * dt;
-                v.x += (double)(h * ax);
-                v.y += (double)(h * ay);
-                v.z += (double)(h * az);
-                a.accel[3 * i] = ax;
-                a.accel[3 * i + 1] = ay;
-                a.accel[3 * i + 2] = az;
+            Comp cx{0.f, 0.f}, cy{0.f, 0.f}, cz{0.f, 0.f};
+            const uint4 fi = a.fix[i];
+            const float rc2 = si->rcutf;
+            const float rc_lo = rc2 * 0.999996f, rc_hi = rc2 * 1.000004f;
+            const float sx = si->sfix[0], sy = si->sfix[1], sz = si->sfix[2];
+            for (uint32_t kb = 0; kb < n; kb += B_BATCH) {
+                const uint4 q = __ldg(reinterpret_cast<const uint4*>(a.nbrs + b_entry(i, kb, a.N)));
+                const uint32_t jj[4] = {q.x, kb + 1u < n ? q.y : i, kb + 2u < n ? q.z : i, kb + 3u < n ? q.w : i};
+                uint4 fj[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) fj[u] = __ldg(a.fix + jj[u]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float dx = (float)(int32_t)(fi.x - fj[u].x) * sx;
+                    const float dy = (float)(int32_t)(fi.y - fj[u].y) * sy;
+                    const float dz = (float)(int32_t)(fi.z - fj[u].z) * sz;
+                    const float rsq = dx * dx + dy * dy + dz * dz;
+                    bool in = rsq < rc_hi && jj[u] != i;
+                    if (in && rsq >= rc_lo) {
+                        const double4_32a pi = a.pos[i];
+                        const double4_32a pj = a.pos[jj[u]];
+                        const double vx = min_image1(pi.x - pj.x, si->L[0], si->Linv[0]);
+                        const double vy = min_image1(pi.y - pj.y, si->L[1], si->Linv[1]);
+                        const double vz = min_image1(pi.z - pj.z, si->L[2], si->Linv[2]);
+                        in = rsq_exact(vx, vy, vz) < si->rcutsq;
+                    }
+                    if (!in) continue;
+                    const float fdr = b_force<PE>(rec, rsq);
+                    cx.add(dx * fdr);
+                    cy.add(dy * fdr);
+                    cz.add(dz * fdr);
+                }
             }
-        }
-        a.vel[i] = v;
-        if (moved) {
-            int w[3] = {0, 0, 0};
-            wrap1(p.x, w[0], si->L[0], si->lo[0], si->hi[0]);
-            wrap1(p.y, w[1], si->L[1], si->lo[1], si->hi[1]);
-            wrap1(p.z, w[2], si->L[2], si->lo[2], si->hi[2]);
-            if (w[0] | w[1] | w[2])
-                for (int d = 0; d < 3; ++d) a.image[3 * i + d] += w[d];
-            a.pos_next[i] = p;
-            uint4 f;
-            f.x = to_fixed(p.x, si->Linv[0]);
-            f.y = to_fixed(p.y, si->Linv[1]);
-            f.z = to_fixed(p.z, si->Linv[2]);
-            f.w = a.sys[i];
-            a.fix_next[i] = f;
-            const uint4 fb = a.fix_build[i];
-            const float ddx = (float)(int32_t)(f.x - fb.x) * si->sfix[0];
-            const float ddy = (float)(int32_t)(f.y - fb.y) * si->sfix[1];
-            const float ddz = (float)(int32_t)(f.z - fb.z) * si->sfix[2];
-            want = ddx * ddx + ddy * ddy + ddz * ddz > a.disp_thresh2;
-            if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicOr(&a.flags[1], AZP_EBIT_NONFINITE);
+            want = b_integrate(a, si, i, cx.value(), cy.value(), cz.value());
         }
     }
-    if (__any_sync(0xffffffffu, want) && (threadIdx.x & 31) == 0) atomicOr(&a.flags[0], 1u);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const uint32_t t = atomicAdd(&a.flags[4], 1u);
-        if (t == gridDim.x - 1) {
-            __threadfence();
-            const uint32_t req = atomicAdd(&a.flags[0], 0u) && !atomicAdd(&a.flags[1], 0u);
-            if (a.set_cond) cudaGraphSetConditional(a.next_cond, req ? 1u : 0u);
-            a.flags[4] = 0u;
-            *a.d_ts_rw = *a.d_ts_rw + 1ull;
-        }
-    }
+    b_finish_step(a, want);
 }
 
 // Langevin step one in place at the start of a run
@@ -763,7 +936,16 @@ __global__ void k_b_store(const double4_32a* __restrict__ pos, const double4_32a
 template<class PE>
 int launch_b_step(int precision, const BStep& a, cudaStream_t s)
 {
-    if (a.blocks == 0) return AZP_OK;
+    if (a.blocks == 0) {  // a thread per particle
+        const uint32_t blocks = (a.N + (uint32_t)a.block - 1u) / (uint32_t)a.block;
+        if (blocks == 0) return AZP_OK;
+        if (precision == AZP_FP32)
+            k_b_step_threads<PE, float><<<blocks, a.block, 0, s>>>(a);
+        else
+            k_b_step_threads<PE, double><<<blocks, a.block, 0, s>>>(a);
+        AZP_CHECK_LAUNCH("k_b_step_threads");
+        return AZP_OK;
+    }
     if (precision == AZP_FP32)
         k_b_step<PE, float><<<a.blocks, a.block, b_step_smem((uint32_t)a.block), s>>>(a);
     else
@@ -794,6 +976,7 @@ struct azp_batch {
     std::vector<uint32_t> n_of, off;
     int precision = AZP_FP64, kind = 0, tpp = 1, block = BATCH_BLOCK;
     std::vector<double> row_len;  // expected list entries per particle, by replica
+    bool alike = false;           // rows of about one length (b_plan)
     uint2* work = nullptr;        // blocks of the fused step (b_plan)
     // first entry and number of entries of work, by log2(tpp) and log2(block / 64)
     std::pair<size_t, uint32_t> plan[B_TPPS][B_BLOCKS];
@@ -878,6 +1061,22 @@ uint32_t b_width(uint32_t max_nn) { return (max_nn + B_LIST_BLOCK - 1u) / B_LIST
 // tpp or more; per_lane is 128, where fewer sums are combined and the rows of a warp are
 // read together, and less while the lanes would not fill a quarter of the chip. Replicas
 // with the longest rows go first, so that the last blocks are short.
+// Rows of about one length (alike): the longest is not longer, against the mean, than the
+// particles are many against a quarter of the chip's threads, so that a thread per particle
+// keeps them busy to the end; or all are short and the replicas too small to fill the blocks
+// that they would have to themselves. Then the list and the FP32 step go a thread per
+// particle (k_b_nlist_threads, k_b_step_threads; no entries here), and the FP64 step, which
+// the pipe bounds whatever the split, where rows are short besides and no lanes are asked
+// for. Microseconds a step without list builds, lanes and thread per particle, replicas of
+// 1,000 particles with rows of 5 / 20 / 61 / 132 / 500:
+//   FP32 N =   4,000: 18 and 20 / 20 and 24 / 22 and 36 / 26 and 51 / 46 and 137
+//        N =  40,000: 25 and 24 / 28 and 28 / 35 and 41 / 47 and 59 / 106 and 157
+//        N = 400,000: 96 and 56 / 122 and 72 / 175 and 124 / 254 and 205 / 720 and 641
+//   FP64 N =  40,000: 61 and 70 / 154 and 219 / 398 and 620 / 758 and 1,204
+//        N = 400,000: 349 and 297 / 1,154 and 1,133 / 3,192 and 3,335
+//   4,000 replicas of 50: FP32 57 and 38 / 66 and 46; FP64 229 and 193 / 645 and 629
+//   4,096 replicas of 10: FP32 48 and 23; FP64 89 and 57
+// 48 replicas of 337,467 particles with rows of 15 to 2,800: 360 and 1,200.
 int b_plan(azp_batch* b)
 {
     int dev = 0, sms = 1;
@@ -886,6 +1085,13 @@ int b_plan(azp_batch* b)
     std::vector<uint32_t> order(b->S);
     for (uint32_t r = 0; r < b->S; ++r) order[r] = r;
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return b->row_len[x] > b->row_len[y]; });
+    double longest = 0.0, entries = 0.0;
+    for (uint32_t r = 0; r < b->S; ++r) {
+        longest = std::max(longest, b->row_len[r]);
+        entries += b->row_len[r] * b->n_of[r];
+    }
+    b->alike = longest * 512.0 * sms <= entries || (longest <= 64.0 && b->N < 32u * b->S);
+    const bool threads = b->alike && (b->precision == AZP_FP32 || longest <= 24.0);
     std::vector<uint2> work;
     for (int kt = 0; kt < B_TPPS; ++kt) {
         double per_lane = 128.0;
@@ -900,12 +1106,15 @@ int b_plan(azp_batch* b)
             for (uint32_t r = 0; r < b->S; ++r) lanes += (size_t)b->n_of[r] << lanes_log2(r);
             if (lanes >= (size_t)sms * 512) break;
         }
+        const bool one = threads && (b->precision == AZP_FP32 || kt == 0);
         for (int kb = 0; kb < B_BLOCKS; ++kb) {
             if (kt > 0 && b->precision == AZP_FP32) {
                 b->plan[kt][kb] = b->plan[0][kb];
                 continue;
             }
             b->plan[kt][kb].first = work.size();
+            b->plan[kt][kb].second = 0u;
+            if (one) continue;
             for (uint32_t r : order) {
                 const uint32_t lt = lanes_log2(r);
                 const uint32_t per = b_block_particles(64u << kb, lt);
@@ -955,8 +1164,12 @@ int b_rebuild(azp_batch* b, cudaStream_t s, const uint32_t* gate)
     k_b_back<<<nblk(N), 256, 0, s>>>(p, gate);
     k_b_fixed<<<nblk(N), 256, 0, s>>>(b->pos[b->cur], b->sys, N, b->info, b->fix[b->cur], b->fix_build, gate);
     constexpr uint32_t per_block = B_NL_WARPS * B_CHUNK;
-    k_b_nlist<<<(N + per_block - 1) / per_block, B_NL_WARPS * 32, 0, s>>>(
-        b->pos[b->cur], b->fix[b->cur], N, b->info, b->cell_start, b->cell_of, b->counts, b->nbrs, b->max_nn, b->flags + 3, gate);
+    if (b->alike)
+        k_b_nlist_threads<<<(N + 127u) / 128u, 128, 0, s>>>(b->pos[b->cur], b->fix[b->cur], N, b->info, b->cell_start, b->cell_of,
+                                                           b->counts, b->nbrs, b->max_nn, b->flags + 3, gate);
+    else
+        k_b_nlist<<<(N + per_block - 1) / per_block, B_NL_WARPS * 32, 0, s>>>(
+            b->pos[b->cur], b->fix[b->cur], N, b->info, b->cell_start, b->cell_of, b->counts, b->nbrs, b->max_nn, b->flags + 3, gate);
     k_b_finish<<<1, 1, 0, s>>>(b->flags, gate);
     AZP_CHECK_LAUNCH("b_rebuild");
     b->launches += 12;
