@@ -502,7 +502,8 @@ AZP_HD uint32_t b_block_particles(uint32_t block, uint32_t lt) { return block >>
 template<class PE> AZP_D float b_force(const float* rec, float rsq)
 {
     float fdr, e;
-    PE::eval(rec, rsq, fdr, e);
+    if constexpr (std::is_same<PE, ExpandedYukawa>::value) PE::force_f(rec, rsq, fdr);
+    else PE::eval(rec, rsq, fdr, e);
     return fdr;
 }
 

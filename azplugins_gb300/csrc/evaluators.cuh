@@ -135,20 +135,22 @@ struct ExpandedYukawa {
         for (int k = 3; k < PAIR_REC; ++k) rec[k] = R(0);
     }
     template<typename R> AZP_HD static bool enabled(const R* rec) { return rec[0] != R(0); }
+#ifdef __CUDACC__
+    // force / r in FP32 without branches (fp32.cuh), for the batched step, where it is wanted
+    // for 16 pairs at once: as eval but for the last bit in rare cases, and not a number
+    // where r or r - delta is 0
+    AZP_D static void force_f(const float* rec, float rsq, float& fdr)
+    {
+        float r, rinv;
+        f_root(rsq, r, rinv);
+        const float s = r - rec[2];
+        const float sinv = f_rcp(s);
+        const float u = rec[0] * expf(-rec[1] * s) * sinv;
+        fdr = f_over(u * (rec[1] + sinv), r, rinv);
+    }
+#endif
     template<typename R> AZP_HD static void eval(const R* rec, R rsq, R& fdr, R& e)
     {
-#ifdef __CUDA_ARCH__
-        if constexpr (std::is_same<R, float>::value) {
-            float r, rinv;
-            f_root(rsq, r, rinv);
-            const float s = r - rec[2];
-            const float sinv = f_rcp(s);
-            const float u = rec[0] * expf(-rec[1] * s) * sinv;
-            fdr = f_over(u * (rec[1] + sinv), r, rinv);
-            e = u;
-            return;
-        }
-#endif
         const R r = root(rsq);
         const R s = r - rec[2];
         const R sinv = rcp(s);
