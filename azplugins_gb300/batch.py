@@ -91,6 +91,7 @@ class ReplicaBatch:
         self._b = L.azp_batch_create(ctypes.byref(c), ctypes.byref(st))
         _lib.check(st.value, "azp_batch_create")
         self.timestep = timestep
+        self.precision = precision
         self._free = collections.deque(maxlen=2)  # memory of result arrays not in use (appends and pops are atomic)
         self.set_state(snapshots)
         self.tpp = 1
@@ -168,18 +169,24 @@ class ReplicaBatch:
 
     def autotune(self, candidates=(1, 2, 4, 8), steps=20, repeats=2, blocks=(256,)):
         """Pick the threads-per-particle and the block size of the fused step by
-        timing every pair (CUDA events on the launching stream).
+        timing every pair (CUDA events on the launching stream). With FP32 forces the
+        step splits the rows its own way, so one timing of a block size stands for all
+        candidates.
 
         The state is restored afterwards; returns {tpp: ms per step} when one
         block size is tried, else {(tpp, block): ms per step}."""
         import torch
 
+        candidates = list(candidates)
         saved = self.get_arrays()
         t0 = self.timestep
         res = {}
         for block in blocks:
             self.set_block(block)
             for tpp in candidates:
+                if self.precision == "fp32" and tpp != candidates[0]:
+                    res[(tpp, block)] = res[(candidates[0], block)]
+                    continue
                 self.set_tpp(tpp)
                 self.run(2, check=False)  # graph capture + warm-up
                 best = float("inf")

@@ -1580,7 +1580,7 @@ int azp_batch_set_block(azp_batch* b, int block)
 int azp_batch_set_tpp(azp_batch* b, int tpp)
 {
     if (!b || !(tpp == 1 || tpp == 2 || tpp == 4 || tpp == 8 || tpp == 16 || tpp == 32)) return AZP_ERR_INVALID;
-    if (b->tpp != tpp) b_free_graphs(b);
+    if (b->tpp != tpp && b->precision == AZP_FP64) b_free_graphs(b);  // (the FP32 step does not change)
     b->tpp = tpp;
     return AZP_OK;
 }

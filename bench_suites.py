@@ -120,7 +120,7 @@ def suite_batched(args):
     yk = [dict(epsilon=p["epsilon"], kappa=p["kappa"], delta=p["delta"]) for p in params]
     rc = [p["r_cut"] for p in params]
     b = ReplicaBatch(snaps, az.pair.ExpandedYukawa, yk, rc, seeds, dt=0.002, precision="fp32")
-    tune = b.autotune(candidates=(1, 2, 4, 8), steps=20, blocks=(128, 256, 512))
+    tune = b.autotune(candidates=(1,), steps=20, blocks=(128, 256, 512))  # (FP32 forces: lanes are the step's choice)
     b.run(50)  # warm-up
     steps = args.steps if args.steps != 2000 else 500
     ms = _cuda_ms(lambda: b.run(steps, check=False))

@@ -101,3 +101,15 @@ def test_both_forms_of_the_fp32_step_agree_bitwise():
     assert builds[0] == builds[1]
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+def test_autotune_in_fp32_times_a_block_size_once():
+    b = _batch(_snaps([50, 60, 70], 5), "fp32")
+    ran = []
+    run = b.run
+    b.run = lambda steps, check=True: (ran.append((b.block, b.tpp)), run(steps, check))
+    res = b.autotune(candidates=(1, 2, 4), steps=3, repeats=1, blocks=(128, 256))
+    assert set(res) == {(t, k) for t in (1, 2, 4) for k in (128, 256)}
+    assert len(set(ran)) == 2 and len(ran) == 4
+    del b.run
+    b.close()
