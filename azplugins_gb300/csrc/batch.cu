@@ -188,16 +188,17 @@ __global__ void k_b_fixed(const double4_32a* __restrict__ pos, const uint16_t* _
 // (make_list_cuts, 5e-6) covers: both coordinates' roundings come to 2.1e-6 of r^2. Chunks
 // with a particle that was clamped into its cell (word_in_cell) form the differences pair by
 // pair.
-// Bound by issue (14 or 23 instructions a test). One thread per particle and a column of
-// the list each took 1,010 us for 48 replicas (337,467 particles, 94 M entries), with
-// 32 lanes on rows of 15 to 2,800 entries; this takes 565.
+// Bound by issue (14 or 23 instructions a test) at 22 % of the warps (114 registers). A
+// build of 48 replicas (337,467 particles, 94 M entries), all kernels, takes 1,760 us so and
+// took 3,115 with one thread per particle and a column of the list each, with 32 lanes on
+// rows of 15 to 2,800 entries.
 constexpr int B_CHUNK = 8;
 // The list: entry k of particle i. Blocks of 16 entries, the particles' side by side: a
 // pass of the step reads one block of each of its particles, and what is in use of the
 // list is compact whatever the longest row. Whole rows one after the other, at 3,700
 // entries each, spread 0.4 GB of entries over 5 GB and its pages: 390 us a step for 48
-// replicas against 360 so (the list build, which writes a row in several places, takes 565
-// against 490; there are 7 steps to a build).
+// replicas against 360 so (the list build, which writes a row in several places, takes 15 %
+// longer; there are about 18 steps to a build).
 constexpr uint32_t B_LIST_BLOCK = 16;
 AZP_D size_t b_entry(uint32_t i, uint32_t k, uint32_t N)
 {

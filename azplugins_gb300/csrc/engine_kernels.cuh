@@ -394,8 +394,8 @@ static __device__ __noinline__ double2 adjusted_fp64(const MDArgs& a, const doub
 // r_cut decision. The particles' sums then move to the block's first threads, so
 // that bonds and integration run on full warps too.
 // Measured (ncu, LJ fluid of N = 54,872, 131 listed and 90 in range a particle):
-// 950 us with one thread per particle evaluating as it walked, 347 us so, the FP64
-// pipe 80 % busy; melt of N = 131,300: 274 -> 118 us.
+// 950 us with one thread per particle evaluating as it walked, 250 us so; melt of
+// N = 131,300: 274 -> 118 us.
 constexpr uint32_t MD_QUEUE = 16;  // queued candidates per lane of a particle
 constexpr int MD_SCAN = 4;         // list entries a lane scans per pass
 
@@ -1345,8 +1345,9 @@ AZP_D bool md_step_fx_body(const MDArgs& a, uint32_t block, unsigned long long t
                 jn[u] = k < n ? ld_ro<NC>(col + (size_t)k * a.N) : (TILE ? (TILE_GLOBAL | i) : i);
             }
 #endif
-            // a lane's batch is FX_BATCH consecutive entries, so that the batch sums (and
-            // with them the force) do not depend on the threads per particle
+            // a lane's batch is FX_BATCH consecutive entries, so that the batch sums do not
+            // depend on the threads per particle (the total does in its last bits: each
+            // lane compensates its own batches, and reduce() joins the lanes)
             for (uint32_t kb = sub * FX_BATCH; kb < kend; kb += FX_BATCH * tpp) {
                 uint32_t jj[FX_BATCH];
                 uint4 fj[FX_BATCH];
@@ -1636,6 +1637,8 @@ int launch_run_k(const RunArgs& r, cudaStream_t s)
     // body has 80 registers and the rebuild's phases share the residency: graph and this
     // kernel 113.9 and 111.7 us per step at 432 blocks (fluid 110,592), but 54.5 and 63.4
     // at 500 (colloid 8,000), 42.9 and 46.6 at 513 (melt 131,300), 173 and 271 at 4,097.
+    // Colloid mixtures below the line: 38.9 and 32.2 at 63 blocks (1,000 particles), 45.7 and
+    // 38.7 at 313, 48.1 and 39.5 at 456.
     // FP64, whose longer steps refill the SMs block by block: a thread per particle must
     // fit, for the rebuild; 73.9 and 61.9 (melt 40,000), 580 and 573 (colloid 65,537),
     // but 122.6 and 122.1 at 131,300 and 319 and 348 at 400,000.

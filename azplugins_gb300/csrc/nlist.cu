@@ -91,9 +91,11 @@ void make_list_cuts(const double* r_cut, uint32_t ntypes, double r_buff, const a
     const double Lmax = std::max(box.L[0], std::max(box.L[1], box.L[2]));
     // worst-case relative error of the FP32 fixed-point rsq: float rounding of
     // three components and their squares (< 1e-6), of the two coordinates relative
-    // to a particle of the cell where the warp build forms them so (each below 1.6
-    // r_list_max, so < 1e-6 r_max / r_min together), plus the fixed-point rounding of
-    // both positions (L 2^-33 each) against the smallest list radius.
+    // to a particle of the cell where the warp build forms them so (cells are up to 1.2
+    // r_list_max wide, so a particle of the cell lies within 1.2 of it and a candidate in
+    // the band within 2.2; two roundings of 2^-24 each, so 4e-7 r_max per axis and
+    // < 1.5e-6 r_max / r_min of r^2), plus the fixed-point rounding of both positions
+    // (L 2^-33 each) against the smallest list radius.
     double delta = 4e-6;
     if (rmax > 0.0) delta = 3e-6 + 2e-6 * rmax / rmin;
     if (rmax > 0.0) delta = std::max(delta, 16.0 * Lmax * 2.3283064365386963e-10 / rmin);
