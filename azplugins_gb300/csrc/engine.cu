@@ -1170,9 +1170,10 @@ bool is_capturing(cudaStream_t s)
     return true;
 }
 
-// `steps` mid steps as one persistent launch (k_md_run); it leaves no rebuild pending
+// `steps` mid steps as persistent launches (k_md_run), counted down; they leave no rebuild
+// pending
 constexpr uint64_t RUN_STEPS = 256;  // per launch, so that other streams get their turn
-int enqueue_run(azp_md* m, int integ, uint64_t steps, cudaStream_t s)
+int enqueue_run(azp_md* m, int integ, uint64_t& steps, cudaStream_t s)
 {
     RunArgs r{};
     const int cur = m->cur;
@@ -2125,9 +2126,8 @@ int azp_md_run(azp_md* m, uint64_t steps, void* stream)
         st = enqueue_run(m, integ, mid, s);
         if (st == AZP_ERR_UNSUPPORTED) {  // refused before the first launch
             m->run_kernel = false;
-        } else {
+        } else if (st != AZP_ERR_TOO_LARGE) {  // (refused on this stream)
             if (st) return st;
-            mid = 0;
             settled = true;
         }
     }

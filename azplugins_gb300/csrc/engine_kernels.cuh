@@ -1647,7 +1647,13 @@ int launch_run_k(const RunArgs& r, cudaStream_t s)
     const uint32_t grid = std::min(std::max(r.blocks, 16u), most);
     RunArgs args = r;
     void* params[] = {&args};
-    AZP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k, dim3(grid), dim3(RUN_BLOCK), params, smem, s));
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k, dim3(grid), dim3(RUN_BLOCK), params, smem, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        // a stream with part of the device's SMs (a green context): step by step there
+        cudaGetLastError();
+        return AZP_ERR_TOO_LARGE;
+    }
+    AZP_CUDA_TRY(e);
     return AZP_OK;
 }
 
