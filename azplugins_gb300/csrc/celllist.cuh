@@ -181,7 +181,7 @@ void launch_cell_scatter(const uint32_t* cell_of, const uint32_t* slot, const ui
 // Full neighbour list. members == NULL means the particles are already stored in
 // cell order (members[s] = s). keys: exclusion keys of particles (NULL: index);
 // ex_n[i] / ex_keys[k * N + i]: excluded keys of particle i. Rows are written
-// column-major nbrs[k * N + i]; counts[i] = the true count even past max_nn;
+// column-major nbrs[k * N + i]; counts[i] = the entries written (at most max_nn);
 // flags[0] = max count over particles (atomicMax), used to detect overflow.
 void launch_nlist_build(const double4_32a* pos, const uint4* fixed, uint32_t N, const azp_box& box, const CellGrid& g,
                         const uint32_t* cell_start, const uint32_t* members, const uint32_t* cell_of,

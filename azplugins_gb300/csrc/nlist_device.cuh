@@ -212,7 +212,7 @@ AZP_D void nlist_thread(const ListArgs& L, uint32_t i, const ListCut* s_cut, con
             ++m;
         }
     }
-    counts[i] = n > max_nn ? n : m;
+    counts[i] = m;  // what is written, also past the capacity
     if (n > max_nn) atomicMax(&flags[0], n);
 }
 
@@ -501,7 +501,7 @@ AZP_D void nlist_chunk(const ListArgs& L, const uint4* words, uint32_t chunk, ui
             kept[p] = min(m, NLW_ROW);
             kept_max = max(kept_max, kept[p]);
             if (lane == 0u) {
-                counts[i] = raw > max_nn ? raw : m;
+                counts[i] = m;  // what is written, also past the capacity
                 if (raw > max_nn) atomicMax(&flags[0], raw);
             }
         }
