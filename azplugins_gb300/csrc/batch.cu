@@ -1065,10 +1065,11 @@ uint32_t b_width(uint32_t max_nn) { return (max_nn + B_LIST_BLOCK - 1u) / B_LIST
 // with the longest rows go first, so that the last blocks are short.
 // Rows of about one length (alike): the longest is not longer, against the mean, than the
 // particles are many against a quarter of the chip's threads, so that a thread per particle
-// keeps them busy to the end; or all are short and the replicas too small to fill the blocks
-// that they would have to themselves. Then the list and the FP32 step go a thread per
-// particle (k_b_nlist_threads, k_b_step_threads; no entries here), and the FP64 step, which
-// the pipe bounds whatever the split, where rows are short besides and no lanes are asked
+// keeps them busy to the end, and no row has more than 1,000 entries; or all are short and
+// the replicas too small to fill the blocks that they would have to themselves. Then the
+// list and the FP32 step go a thread per particle (k_b_nlist_threads, k_b_step_threads; no
+// entries here), and the FP64 step, which the pipe bounds whatever the split, where rows
+// are short besides and no lanes are asked
 // for. Microseconds a step without list builds, lanes and thread per particle, replicas of
 // 1,000 particles with rows of 5 / 20 / 61 / 132 / 500:
 //   FP32 N =   4,000: 18 and 20 / 20 and 24 / 22 and 36 / 26 and 51 / 46 and 137
@@ -1078,6 +1079,10 @@ uint32_t b_width(uint32_t max_nn) { return (max_nn + B_LIST_BLOCK - 1u) / B_LIST
 //        N = 400,000: 349 and 297 / 1,154 and 1,133 / 3,192 and 3,335
 //   4,000 replicas of 50: FP32 57 and 38 / 66 and 46; FP64 229 and 193 / 645 and 629
 //   4,096 replicas of 10: FP32 48 and 23; FP64 89 and 57
+//   with list builds, FP32, longest row / mean: N = 120,000 64 / 48: 63 and 55; 115 / 73: 73 and
+//   70; 345 / 94: 99 and 159; N = 400,000 115 / 40: 162 and 109; 345 / 63: 212 and 193;
+//   N = 1,200,000 345 / 63: 572 and 366; N = 680,095 2,232 / 223: 735 and 907;
+//   N = 1,320,729 2,898 / 291: 1,753 and 1,836
 // 48 replicas of 337,467 particles with rows of 15 to 2,800: 360 and 1,200.
 int b_plan(azp_batch* b)
 {
@@ -1092,7 +1097,7 @@ int b_plan(azp_batch* b)
         longest = std::max(longest, b->row_len[r]);
         entries += b->row_len[r] * b->n_of[r];
     }
-    b->alike = longest * 512.0 * sms <= entries || (longest <= 64.0 && b->N < 32u * b->S);
+    b->alike = (longest <= 1000.0 && longest * 512.0 * sms <= entries) || (longest <= 64.0 && b->N < 32u * b->S);
     const bool threads = b->alike && (b->precision == AZP_FP32 || longest <= 24.0);
     std::vector<uint2> work;
     for (int kt = 0; kt < B_TPPS; ++kt) {
