@@ -20,6 +20,8 @@
 namespace azp
 {
 #ifdef __CUDACC__
+AZP_D bool finite_bits(double a) { return (__double2hiint(a) & 0x7ff00000) != 0x7ff00000; }
+
 // |x| in [2^-100, 2^100], by its exponent field
 AZP_D bool seed_range(int hi) { return (uint32_t)((hi & 0x7fffffff) - 0x39b00000) < 0x0c800000u; }
 
@@ -54,18 +56,17 @@ AZP_D double d_rcp(double x)
 }
 
 // a / b: the product with 1 / b corrected once by its residual, which rounds it as the
-// division does but for quotients within 2^-8 ulp or so of a rounding boundary (the bare
-// product is an ulp off in 27 % of the cases). |a| in [2^-900, 2^900]; others divide, out of
-// line.
-static __device__ __noinline__ double divide(double a, double b) { return a / b; }
+// division does but for quotients within 2^-8 ulp or so of a rounding boundary and for |a|
+// below 2^-900 (the bare product is an ulp off in 27 % of the cases). Where there is no
+// residual (a infinite or not a number) the product stands.
 AZP_D double d_div(double a, double b)
 {
     const int hb = __double2hiint(b);
-    const uint32_t ha = (uint32_t)__double2hiint(a) & 0x7fffffffu;
-    if (!seed_range(hb) || ha - 0x07b00000u >= 0x70800000u) return divide(a, b);
+    if (!seed_range(hb)) return a / b;
     const double y = rcp_in_range(b, hb);
     const double q = a * y;
-    return fma(fma(-q, b, a), y, q);
+    const double r = fma(-q, b, a);
+    return finite_bits(r) ? fma(r, y, q) : q;
 }
 
 // 1 / sqrt(x), x > 0: y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2
@@ -112,8 +113,6 @@ AZP_D bool magnitude_above(double a, double b)
 {
     return (__double_as_longlong(a) & 0x7fffffffffffffffll) > __double_as_longlong(b);
 }
-
-AZP_D bool finite_bits(double a) { return (__double2hiint(a) & 0x7ff00000) != 0x7ff00000; }
 
 // min_image1 that runs only where it changes v: |v| > L / 2. The body is out of
 // line: as a predicated or speculated body its FP64 instructions would occupy the
